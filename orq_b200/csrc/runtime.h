@@ -240,7 +240,7 @@ void op_sub_b(Ctx& c, int w, size_t n, CSh3 x, CSh3 y, Sh3 z);
 void op_zero_share(Ctx& c, bool arith, int w, size_t n, Sh3 r);
 void op_reshare(Ctx& c, bool arith, int w, size_t n, int group, Sh3 s);
 
-// ---- permutations (perm.cu) ----
+// ---- permutations (fy.cu, perm.cu) ----
 void release_fy(Ctx& c);
 void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>& out);
 void reserve_perms(Ctx& c, size_t n, size_t count);
