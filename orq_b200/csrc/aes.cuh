@@ -76,15 +76,12 @@ struct AesSmem {
     }
 };
 
-// Encrypt one block (4 little-endian column words) in place.
-__device__ __forceinline__ void aes256_encrypt(const AesSmem& S, const AesRK& rk, uint32_t& s0,
-                                               uint32_t& s1, uint32_t& s2, uint32_t& s3) {
-    s0 ^= rk.k[0];
-    s1 ^= rk.k[1];
-    s2 ^= rk.k[2];
-    s3 ^= rk.k[3];
+// Rounds R0..14 of one block, in place, from the state after round R0 - 1.
+template <int R0>
+__device__ __forceinline__ void aes256_rounds_from(const AesSmem& S, const AesRK& rk, uint32_t& s0,
+                                                   uint32_t& s1, uint32_t& s2, uint32_t& s3) {
 #pragma unroll
-    for (int r = 1; r < 14; r++) {
+    for (int r = R0; r < 14; r++) {
         const uint32_t n0 = S.lk<0, 0>(s0) ^ S.lk<1, 1>(s1) ^ S.lk<2, 2>(s2) ^ S.lk<3, 3>(s3) ^ rk.k[4 * r + 0];
         const uint32_t n1 = S.lk<0, 0>(s1) ^ S.lk<1, 1>(s2) ^ S.lk<2, 2>(s3) ^ S.lk<3, 3>(s0) ^ rk.k[4 * r + 1];
         const uint32_t n2 = S.lk<0, 0>(s2) ^ S.lk<1, 1>(s3) ^ S.lk<2, 2>(s0) ^ S.lk<3, 3>(s1) ^ rk.k[4 * r + 2];
@@ -108,6 +105,16 @@ __device__ __forceinline__ void aes256_encrypt(const AesSmem& S, const AesRK& rk
     s1 = n1 ^ rk.k[57];
     s2 = n2 ^ rk.k[58];
     s3 = n3 ^ rk.k[59];
+}
+
+// Encrypt one block (4 little-endian column words) in place.
+__device__ __forceinline__ void aes256_encrypt(const AesSmem& S, const AesRK& rk, uint32_t& s0,
+                                               uint32_t& s1, uint32_t& s2, uint32_t& s3) {
+    s0 ^= rk.k[0];
+    s1 ^= rk.k[1];
+    s2 ^= rk.k[2];
+    s3 ^= rk.k[3];
+    aes256_rounds_from<1>(S, rk, s0, s1, s2, s3);
 }
 
 // Keystream block `blk` of a draw that starts at nonce `nonce0` of the stream

@@ -10,23 +10,23 @@
 // nonces depend on how many draws the previous one used.
 //
 // GPU design:
-//  * fy_gen  (all SMs but three): AES keystream of a window of buffers; per
-//    32768-draw tile, nested lists (in draw order) of the draws below n/4^L,
-//    and the tile's last draw.
-//  * fy_scan (one 1024-thread CTA per group): replays the sequential
-//    acceptance exactly over the sparsest level that holds every candidate; an
-//    entry is certainly accepted if v + (its index in the step) <= n-1-i,
-//    certainly rejected if v > n-1-i, and the few in between are decided in
-//    order by one warp. Windows are generated up to five ahead of the scans.
-//  * fy_small (M <= 2^17, a predictable number of buffers per permutation):
+//  * the draws of a group's buffers do not depend on where permutations start,
+//    so k_fy_gen computes them ahead, as pure keystream, into a ring;
+//  * a permutation's threshold T = n-1-i falls along a predictable curve
+//    (x' = -x/M), so k_fy_classify decides almost every draw in parallel from a
+//    window around the curve: accepted, rejected, or uncertain;
+//  * k_fy_resolve (one CTA per group) walks only the uncertain draws in order,
+//    and k_fy_emit writes the accepted offsets at their exact ranks and checks
+//    the windows against the exact thresholds;
+//    A one-CTA scanner that replayed every draw bounded the chain before: the
+//    radix step of 2^22 rows took 418 ms and takes 280 ms, of 2^20 rows 127.6
+//    and 62.8 ms, of 100003 rows 19.0 and 12.5 ms.
+//  * fy_small (M <= 2^15, one buffer per permutation almost always):
 //    every (permutation, group) in its own CTA at once from predicted start
-//    buffers, re-run from the first wrong prediction until all are verified.
+//    buffers, re-run from the first wrong prediction until all are verified;
 //  * fy_finalize: turns the accepted offsets into the final permutation in
 //    parallel and writes its inverse.
 #include <algorithm>
-#include <array>
-#include <chrono>
-#include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <memory>
@@ -37,158 +37,504 @@ namespace orqcu {
 
 namespace {
 
-constexpr uint32_t kTileDraws = 32768;        // draws per tile
-constexpr uint32_t kTileBlocks = kTileDraws / 4;
-constexpr uint32_t kTilesPerRefill = (1u << 20) / kTileDraws;  // 32
+// ---------------------------------------------------------------------------
+// The chain of permutations of one group (M = 2^bit_width(n) >= kChainMinM).
+constexpr uint32_t kBufDraws = 1u << 20;   // draws per getNext buffer
+constexpr uint32_t kListDraws = 2048;      // draws behind one sparse list
+constexpr uint32_t kListCap = 256;
+constexpr uint32_t kListsPerBuf = kBufDraws / kListDraws;
+constexpr uint32_t kRuns = 8;              // runs (warps) per tile; a CTA classifies a tile
+constexpr uint32_t kMaxRunLists = 4;       // a run is 1..4 lists' draws (FyScanArgs::rl)
+constexpr uint32_t kRunUnc = 512;          // uncertain draws kept per run
+constexpr uint32_t kTileUnc = kRuns * kRunUnc;
+constexpr uint32_t kPieceUnc = 8192;       // uncertain draws k_fy_resolve holds at once
 constexpr int kGenThreads = 512;
-constexpr int kBlocksPerThread = kTileBlocks / kGenThreads;     // 16 blocks = 64 draws
-constexpr int kMaxLevels = 16;
-constexpr int kScanThreads = 1024;
-constexpr uint32_t kMaxWindowTiles = 1024;
+constexpr int kTabEntries = 520;           // U[256], V[257] of one chunk, padded
 
-// Level L of a tile keeps, in draw order, the draws with v < n >> 2L (level 0:
-// every draw that can ever be accepted). Entries are (position << 32) | v.
-__host__ __device__ inline uint32_t level_threshold(uint32_t n, int L) { return n >> (2 * L); }
-__host__ inline uint32_t level_capacity(int L) {
-    // twice the largest expected count (mask >= n) plus slack; overflow is
-    // reported as an error, never truncated silently
-    return L == 0 ? kTileDraws : ((kTileDraws >> (2 * L)) * 2 + 256);
+// Scan state of one group's chain. `pos` counts tiles and `start` buffers from
+// the chain's first buffer.
+struct FyState {
+    unsigned long long pos;    // first tile not yet scanned
+    unsigned long long start;  // buffer where the current permutation starts
+    uint32_t m;                // index of the current permutation
+    uint32_t i;                // accepted so far
+    uint32_t done;             // every permutation is complete
+    uint32_t bad;              // a window missed its threshold or a list overflowed
+};
+
+// GCM's counter block is (nonce, 0, BE32(j + 2)): inside a chunk of 65536
+// blocks only the counter's low bytes change, and after two AES rounds the
+// state is U[ctr & 255] ^ V[ctr >> 8] with tables that depend on the key and
+// the chunk's nonce alone (byte 15 reaches column 0 of round 1, the other
+// counter bytes columns 1 and 2; round 2 is the XOR of one table word per
+// column). Two loads replace 32 of a block's 224 lookups: alone in a loop, the
+// keystream goes from 4.17e10 to 4.70e10 blocks/s.
+__global__ void __launch_bounds__(544) k_fy_tab(StreamArg st, uint4* tab) {
+    const auto T = [](int t, uint32_t w, int byte) { return __ldg(&g_aes_T[t * 256 + ((w >> (8 * byte)) & 255u)]); };
+    const AesRK& rk = st.rk;
+    const unsigned long long nonce = st.nonce + blockIdx.x;
+    uint4* out = tab + (size_t)blockIdx.x * kTabEntries;
+    const uint32_t w0 = (uint32_t)nonce ^ rk.k[0], w1 = (uint32_t)(nonce >> 32) ^ rk.k[1], w2 = rk.k[2];
+    const uint32_t t = threadIdx.x;
+    if (t < 256) {
+        const uint32_t w3 = (t << 24) ^ rk.k[3];
+        const uint32_t n0 = T(0, w0, 0) ^ T(1, w1, 1) ^ T(2, w2, 2) ^ T(3, w3, 3) ^ rk.k[4];
+        out[t] = make_uint4(T(0, n0, 0), T(3, n0, 3), T(2, n0, 2), T(1, n0, 1));
+    } else if (t < 513) {
+        const uint32_t w3 = __byte_perm((t - 256) << 8, 0, 0x0123) ^ rk.k[3];
+        const uint32_t n1 = T(0, w1, 0) ^ T(1, w2, 1) ^ T(2, w3, 2) ^ T(3, w0, 3) ^ rk.k[5];
+        const uint32_t n2 = T(0, w2, 0) ^ T(1, w3, 1) ^ T(2, w0, 2) ^ T(3, w1, 3) ^ rk.k[6];
+        const uint32_t n3 = T(0, w3, 0) ^ T(1, w0, 1) ^ T(2, w1, 2) ^ T(3, w2, 3) ^ rk.k[7];
+        out[t] = make_uint4(T(1, n1, 1) ^ T(2, n2, 2) ^ T(3, n3, 3) ^ rk.k[8],
+                            T(0, n1, 0) ^ T(1, n2, 1) ^ T(2, n3, 2) ^ rk.k[9],
+                            T(0, n2, 0) ^ T(1, n3, 1) ^ T(3, n1, 3) ^ rk.k[10],
+                            T(0, n3, 0) ^ T(2, n1, 2) ^ T(3, n2, 3) ^ rk.k[11]);
+    }
 }
 
-struct FyState {
-    unsigned long long start_tile;  // absolute tile where the current permutation starts
-    uint32_t m;                     // index of the permutation being scanned
-    uint32_t i;                     // accepted so far
-    uint32_t done;
-    uint32_t pad;
-};
-
-struct FyLayout {
-    uint32_t nl;               // levels in use
-    uint32_t off[kMaxLevels];  // entry offset of each level list inside a tile slot
-    uint32_t cap[kMaxLevels];
-    uint32_t slot;             // entries per tile slot
-};
-
 struct FyGenArgs {
-    StreamArg st[3];  // nonce = chain start nonce + 4 * (window start buffer)
-    uint32_t n, mask, tiles;
-    FyLayout lay;
-    uint32_t* ev;    // [3][tiles][slot] entry values v
-    uint32_t* last;  // [3][tiles] masked value of each tile's last draw
-    uint32_t* cnt;  // [3][tiles][kMaxLevels]
+    StreamArg st;
+    const uint4* tab;  // k_fy_tab of the same buffers
+    uint32_t mask, th; // th: draws below it go to the sparse lists
+    uint32_t lists;    // sparse lists (kListDraws draws each) to produce
+    uint32_t* raw;     // masked draws
+    uint32_t* lst;     // [lists][kListCap]
+    uint32_t* lcnt;    // [lists] entries; above kListCap: the list overflowed
     const FyState* state;
-    int* err;
 };
 
-constexpr int kHalfBlocks = kBlocksPerThread / 2;  // blocks per thread per half tile
-
+// Masked draws of a range of buffers, and per kListDraws of them the list of
+// those below n/16 in draw order (what the scan of a permutation's last 7/8 of
+// draws reads). A warp owns a list, so nothing but the table staging is
+// block-wide. Bound by the T-table lookups (shared-memory pipe): 192 lookups,
+// two table loads and one 16-byte store a block; 64 buffers take 414 us
+// (4.06e10 blocks/s; with nested lists built by block scans it was 2.0e10).
 __global__ void __launch_bounds__(kGenThreads, 1) k_fy_gen(FyGenArgs a) {
     extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ uint32_t sdone;
-    __shared__ uint32_t sbase[kMaxLevels];
-    __shared__ uint32_t wsum[kGenThreads / 32][kMaxLevels / 2];  // per-warp packed level counts
-    __shared__ uint32_t htot[kMaxLevels / 2];                    // half-tile totals
     aes_stage_tables(sm);
     const AesSmem S(sm);
-    const uint32_t total = 3 * a.tiles;
-    for (uint32_t item = blockIdx.x; item < total; item += gridDim.x) {
-        const uint32_t g = item / a.tiles, tile = item % a.tiles;
-        // the scanner may be updating the flag concurrently: read it once per CTA
-        if (threadIdx.x == 0) sdone = *(volatile const uint32_t*)&a.state[g].done;
-        if (threadIdx.x < kMaxLevels) sbase[threadIdx.x] = 0;
-        __syncthreads();
-        if (sdone) continue;
-        const size_t slot = (size_t)g * a.tiles + tile;
-        uint32_t* ov = a.ev + slot * a.lay.slot;
-        for (int half = 0; half < 2; half++) {
-            // this thread's 32 consecutive draws of the half tile
-            uint32_t v[4 * kHalfBlocks];
-            const uint32_t blk0 = half * (kTileBlocks / 2) + threadIdx.x * kHalfBlocks;
-#pragma unroll
-            for (int b = 0; b < kHalfBlocks; b++) {
-                const uint4 ks = keystream_block(S, a.st[g], (unsigned long long)tile * kTileBlocks + blk0 + b);
-                v[4 * b + 0] = ks.x & a.mask;
-                v[4 * b + 1] = ks.y & a.mask;
-                v[4 * b + 2] = ks.z & a.mask;
-                v[4 * b + 3] = ks.w & a.mask;
+    if (*(volatile const uint32_t*)&a.state->done) return;  // no barrier follows
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t nw = gridDim.x * (kGenThreads / 32);
+    constexpr uint32_t kPerChunk = 65536 / (kListDraws / 4);  // lists per chunk
+    for (uint32_t l = blockIdx.x * (kGenThreads / 32) + (threadIdx.x >> 5); l < a.lists; l += nw) {
+        const uint4* U = a.tab + (size_t)(l / kPerChunk) * kTabEntries;
+        const uint4* V = U + 256;
+        uint32_t ctr = (l % kPerChunk) * (kListDraws / 4) + lane + 2;
+        uint4* out = reinterpret_cast<uint4*>(a.raw + (size_t)l * kListDraws) + lane;
+        uint32_t* li = a.lst + (size_t)l * kListCap;
+        uint32_t lc = 0;
+        uint4 u = __ldg(U + (ctr & 255u)), v = __ldg(V + (ctr >> 8));
+#pragma unroll 1
+        for (int it = 0; it < (int)(kListDraws / 128); it++) {
+            uint32_t s0 = u.x ^ v.x, s1 = u.y ^ v.y, s2 = u.z ^ v.z, s3 = u.w ^ v.w;
+            ctr += 32;
+            if (it + 1 < (int)(kListDraws / 128)) {
+                u = __ldg(U + (ctr & 255u));
+                v = __ldg(V + (ctr >> 8));
             }
-            if (half == 1 && threadIdx.x == kGenThreads - 1) a.last[slot] = v[4 * kHalfBlocks - 1];
-            // every level at once (nested lists: level L keeps v < n >> 2L):
-            // per-thread counts two levels per word (16-bit fields; half-tile
-            // totals <= 16384), one block-wide scan for all of them
-            constexpr int kPk = kMaxLevels / 2;
-            uint32_t pc[kPk], ex[kPk];
-#pragma unroll
-            for (int j = 0; j < kPk; j++) pc[j] = 0;
-#pragma unroll
-            for (int L = 0; L < kMaxLevels; L++) {
-                if (L < (int)a.lay.nl) {
-                    const uint32_t th = level_threshold(a.n, L);
-                    uint32_t c = 0;
-#pragma unroll
-                    for (int k = 0; k < 4 * kHalfBlocks; k++) c += v[k] < th;
-                    pc[L >> 1] |= c << (16 * (L & 1));
-                }
+            aes256_rounds_from<3>(S, a.st.rk, s0, s1, s2, s3);
+            s0 &= a.mask;
+            s1 &= a.mask;
+            s2 &= a.mask;
+            s3 &= a.mask;
+            out[32 * it] = make_uint4(s0, s1, s2, s3);
+            const bool c0 = s0 < a.th, c1 = s1 < a.th, c2 = s2 < a.th, c3 = s3 < a.th;
+            const uint32_t b0 = __ballot_sync(0xffffffffu, c0), b1 = __ballot_sync(0xffffffffu, c1);
+            const uint32_t b2 = __ballot_sync(0xffffffffu, c2), b3 = __ballot_sync(0xffffffffu, c3);
+            uint32_t o = lc + __popc(b0 & lt) + __popc(b1 & lt) + __popc(b2 & lt) + __popc(b3 & lt);
+            lc += __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
+            if (lc <= kListCap) {
+                if (c0) li[o++] = s0;
+                if (c1) li[o++] = s1;
+                if (c2) li[o++] = s2;
+                if (c3) li[o] = s3;
             }
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-            for (int j = 0; j < kPk; j++) {
-                uint32_t inc = pc[j];
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += y;
-                }
-                ex[j] = inc - pc[j];
-                if (lane == 31) wsum[warp][j] = inc;
-            }
-            __syncthreads();
-            if (threadIdx.x < kPk) {  // exclusive offsets of the warps, and the totals
-                uint32_t run = 0;
-                for (int w = 0; w < kGenThreads / 32; w++) {
-                    const uint32_t t = wsum[w][threadIdx.x];
-                    wsum[w][threadIdx.x] = run;
-                    run += t;
-                }
-                htot[threadIdx.x] = run;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int L = 0; L < kMaxLevels; L++) {
-                if (L >= (int)a.lay.nl) break;
-                const int sh = 16 * (L & 1);
-                const uint32_t mine = (pc[L >> 1] >> sh) & 0xffffu;
-                const uint32_t pre = ((ex[L >> 1] + wsum[warp][L >> 1]) >> sh) & 0xffffu;
-                const uint32_t tt = (htot[L >> 1] >> sh) & 0xffffu;
-                const uint32_t base = sbase[L];
-                if (base + tt > a.lay.cap[L]) {
-                    if (threadIdx.x == 0) atomicOr(a.err, 16);
-                    continue;
-                }
-                if (mine) {
-                    const uint32_t th = level_threshold(a.n, L);
-                    uint32_t* olv = ov + a.lay.off[L] + base + pre;
-                    uint32_t o = 0;
-#pragma unroll
-                    for (int k = 0; k < 4 * kHalfBlocks; k++)
-                        if (v[k] < th) olv[o++] = v[k];
-                }
-            }
-            __syncthreads();  // every thread has read sbase
-            if (threadIdx.x < a.lay.nl) sbase[threadIdx.x] += (htot[threadIdx.x >> 1] >> (16 * (threadIdx.x & 1))) & 0xffffu;
-            __syncthreads();
         }
-        // an overflowing level was flagged above; its count is clamped so the
-        // scanner never reads past the level's list
-        if (threadIdx.x < a.lay.nl)
-            a.cnt[slot * kMaxLevels + threadIdx.x] = min(sbase[threadIdx.x], a.lay.cap[threadIdx.x]);
+        if (lane == 0) a.lcnt[l] = lc;
+    }
+}
+
+// One run's classification (k_fy_classify -> k_fy_emit).
+struct FyRun {
+    uint32_t cpre, upre;  // certain / uncertain draws of the tile before the run
+    uint32_t cnt, unc;    // candidates (certain + uncertain) and uncertain draws
+    long long lo, hi;     // the window that T at the run's start was assumed in
+};
+struct FySeg {  // what k_fy_resolve settled of a step, for k_fy_emit
+    uint32_t ntiles, m;
+};
+
+struct FyScanArgs {
+    uint32_t n, count, g;
+    uint32_t mbits;                // M = 2^mbits
+    uint32_t th;                   // list threshold of k_fy_gen
+    uint32_t rl;                   // lists per run: 1, 2 or 4
+    uint32_t tpb;                  // tiles per buffer: kListsPerBuf / (kRuns * rl)
+    uint32_t ring_tiles;           // tiles the ring holds
+    uint32_t seg_cap;              // tiles a step may scan
+    unsigned long long limit;      // tiles generated so far
+    double rate;                   // log(1 - 1/M)
+    double width;                  // window half-width in standard deviations
+    const uint32_t *raw, *lst, *lcnt;
+    FyState* state;
+    uint32_t* cand;                // [seg_cap][kRuns][rl * kListDraws] candidates
+    uint2* unc;                    // [seg_cap][kTileUnc] (v + certain draws before it in the tile, place in its run's candidates)
+    FyRun* run;                    // [seg_cap][kRuns]
+    uint32_t *tc, *tu;             // [seg_cap] certain / uncertain draws
+    uint32_t* base;                // [seg_cap] rank of the tile's first acceptance
+    uint32_t* uoff;                // [seg_cap] index of the tile's first uncertain draw in `ok`
+    uint32_t* ok;                  // one bit per uncertain draw of the step: accepted
+    FySeg* seg;
+    uint32_t* acc;                 // [count][3][n] accepted offsets
+};
+
+// Tiles of the next step: what is generated, at most seg_cap, and not much
+// past the place where the permutation ends (x = n - i values remain; they
+// take about M (ln x + 4) draws or fewer with probability 0.98; a step that
+// stops short is continued by the next). Integer arithmetic, so that every
+// kernel of the step finds the same number.
+__device__ __forceinline__ uint32_t fy_step_tiles(const FyScanArgs& a, const FyState& s) {
+    if (s.done || s.bad || s.pos >= a.limit) return 0;
+    const uint32_t lg = 32 - __clz(a.n - s.i);                                // log2(x) rounded up
+    // M in tiles (kRuns * rl * 2048 draws each), times ln x + 4 in 16 fractional bits
+    const unsigned long long span =
+        ((((1ull << a.mbits) / (kRuns * a.rl * kListDraws)) * (lg * 45427ull + 4 * 65536ull)) >> 16) + 2;
+    unsigned long long t = a.limit - s.pos;
+    t = t < a.seg_cap ? t : a.seg_cap;
+    return (uint32_t)(t < span ? t : span);
+}
+
+// Classification of one step's draws. `x` values remain when the step begins,
+// so after d draws x e^(d log(1-1/M)) remain on average, with variance below
+// x p (1 - p): T at a run's start lies in [lo, hi] = mean -+ (width sigma + 3
+// width) except about once in 1e7 permutations (checked afterwards). With k
+// candidates and c certain draws of the run before draw q: accepted for
+// certain if v + k <= lo (at most k acceptances so far), rejected if v > hi - c
+// (at least c), uncertain otherwise. Sizes: 2^22 rows have ~1e3 deviations at
+// worst, so ~1.5 in 1000 draws are uncertain. Small register count: the CTAs
+// run beside the generator's, in its idle issue slots.
+__global__ void __launch_bounds__(kRuns * 32, 4) k_fy_classify(FyScanArgs a) {
+    __shared__ uint2 su[kRuns][kRunUnc];
+    __shared__ uint32_t scert[kRuns], sunc[kRuns];
+    const FyState s = *a.state;
+    const uint32_t nt = fy_step_tiles(a, s);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const double x = (double)(a.n - s.i);
+    const uint32_t rd = a.rl * kListDraws;  // draws per run
+    for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
+        const uint32_t rt = (uint32_t)((s.pos + t) % a.ring_tiles);
+        const double p = exp(a.rate * ((double)t * kRuns + (double)w) * rd);
+        const double half = a.width * sqrt(x * p * (1.0 - p)) + 3.0 * a.width;
+        const long long lo = (long long)floor(x * p - 1.0 - half);
+        const long long hi = min((long long)ceil(x * p - 1.0 + half), (long long)(a.n - s.i) - 1);
+        const bool some = lo >= 0;
+        const uint32_t lou = some ? (uint32_t)lo : 0u, hiu = (uint32_t)hi;
+        const size_t l0 = ((size_t)rt * kRuns + w) * a.rl;
+        const uint32_t* raw = a.raw + l0 * kListDraws;
+        uint32_t* cand = a.cand + ((size_t)t * kRuns + w) * rd;
+        uint32_t k = 0, nu = 0;
+        const uint32_t mycnt = lane < (int)a.rl ? a.lcnt[l0 + lane] : 0u;
+        // (q, e): list q of the run, first of the next 128 entries in it
+        const auto source = [&](uint32_t q, const uint32_t*& src, uint32_t& cnt) {
+            const uint32_t c = __shfl_sync(0xffffffffu, mycnt, q & (kMaxRunLists - 1));
+            const bool use = hiu < a.th && c <= kListCap;
+            src = use ? a.lst + (l0 + q) * kListCap : raw + q * kListDraws;
+            cnt = use ? c : kListDraws;
+        };
+        const uint32_t* src;
+        uint32_t cnt;
+        source(0, src, cnt);
+        uint32_t q = 0, e = 0;
+        uint4 nx = make_uint4(0, 0, 0, 0);
+        if (4 * (uint32_t)lane < cnt) nx = *reinterpret_cast<const uint4*>(src + 4 * lane);
+        while (q < a.rl) {
+            const uint32_t left = cnt - min(cnt, e);
+            const uint4 v4 = nx;
+            // the next 128 entries are loaded before these are decided
+            e += 128;
+            if (e >= cnt) {
+                e = 0;
+                if (++q < a.rl) source(q, src, cnt);
+            }
+            if (q < a.rl && e + 4 * lane < cnt) nx = *reinterpret_cast<const uint4*>(src + e + 4 * lane);
+            const uint32_t v[4] = {v4.x, v4.y, v4.z, v4.w};
+            const uint32_t c = k - nu;
+            bool cd[4], un[4];
+            uint32_t m[4];
+            bool any = false;
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const uint32_t j = 4u * lane + r;
+                cd[r] = j < left && v[r] + c <= hiu;
+                un[r] = cd[r] && !(some && v[r] + k + j <= lou);
+                any = any || un[r];
+                m[r] = __ballot_sync(0xffffffffu, cd[r]);
+            }
+            uint32_t o = k + __popc(m[0] & lt) + __popc(m[1] & lt) + __popc(m[2] & lt) + __popc(m[3] & lt);
+            uint32_t po[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                po[r] = o;
+                if (cd[r]) cand[o++] = v[r];
+            }
+            if (__any_sync(0xffffffffu, any)) {
+                uint32_t um[4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) um[r] = __ballot_sync(0xffffffffu, un[r]);
+                uint32_t uo = nu + __popc(um[0] & lt) + __popc(um[1] & lt) + __popc(um[2] & lt) + __popc(um[3] & lt);
+#pragma unroll
+                for (int r = 0; r < 4; r++)
+                    if (un[r]) {
+                        if (uo < kRunUnc) su[w][uo] = make_uint2(v[r] + (po[r] - uo), po[r]);
+                        uo++;
+                    }
+                nu += __popc(um[0]) + __popc(um[1]) + __popc(um[2]) + __popc(um[3]);
+            }
+            k += __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
+        }
+        if (nu > kRunUnc) {
+            if (lane == 0) atomicOr(&a.state->bad, 2u);
+            nu = kRunUnc;
+        }
+        if (lane == 0) {
+            scert[w] = k - nu;
+            sunc[w] = nu;
+        }
+        __syncthreads();
+        uint32_t cp = 0, up = 0, ct = 0, ut = 0;
+        for (uint32_t r = 0; r < kRuns; r++) {
+            if ((int)r < w) {
+                cp += scert[r];
+                up += sunc[r];
+            }
+            ct += scert[r];
+            ut += sunc[r];
+        }
+        uint2* ou = a.unc + (size_t)t * kTileUnc + up;
+        for (uint32_t j = lane; j < nu; j += 32) {
+            const uint2 z = su[w][j];
+            ou[j] = make_uint2(z.x + cp, z.y);
+        }
+        if (lane == 0) a.run[(size_t)t * kRuns + w] = FyRun{cp, up, k, nu, lo, hi};
+        if (threadIdx.x == 0) {
+            a.tc[t] = ct;
+            a.tu[t] = ut;
+        }
         __syncthreads();
     }
 }
 
+// Decides a step's uncertain draws (one CTA), gives every tile the rank of its
+// first acceptance, and moves the state to the next step. An uncertain draw
+// with v + (certain draws before it) = u is accepted iff u <= X - a, a the
+// uncertain acceptances before it. A thread holds kResEach consecutive ones and
+// decides them from an assumed a at its first; the block's prefix sums give the
+// next assumption, until nothing changes: thread 0 starts from the true count,
+// so the fixed point is the sequential result, and each pass shrinks the error
+// about tenfold (a piece's threshold moves by much less than the window).
+// Between launches of a group's stream nothing else writes the state but the
+// flag `bad`.
+constexpr int kResThreads = 512;
+constexpr int kResEach = kPieceUnc / kResThreads;  // 16
+__global__ void __launch_bounds__(kResThreads, 1) k_fy_resolve(FyScanArgs a) {
+    __shared__ __align__(16) uint32_t su[kPieceUnc];
+    __shared__ uint32_t smask[kResThreads], sbef[kResThreads + 1];
+    __shared__ uint32_t sc[kResThreads], so[kResThreads + 1];
+    __shared__ uint32_t red[33];
+    __shared__ uint32_t s_take, s_end, s_call;
+    const FyState s = *a.state;
+    const uint32_t nt = fy_step_tiles(a, s);
+    const uint32_t tid = threadIdx.x;
+    const int lane = tid & 31, w = tid >> 5;
+    if (!nt) {
+        if (tid == 0) *a.seg = FySeg{0, s.m};
+        return;
+    }
+    const int top = (int)(a.n - s.i - 1);  // T when the step begins
+    uint32_t cbase = 0, abase = 0;         // certain / uncertain acceptances of earlier pieces
+    uint32_t t_end = 0xffffffffu, words = 0;
+    for (uint32_t t0 = 0; t0 < nt && t_end == 0xffffffffu;) {
+        // the next tiles whose uncertain draws fit the piece
+        const uint32_t t = t0 + tid;
+        const uint32_t c = t < nt ? a.tc[t] : 0u, u = t < nt ? min(a.tu[t], kTileUnc) : 0u;
+        uint32_t ctot, utot;
+        const uint32_t cpre = block_excl_sum(c, red, ctot);
+        const uint32_t upre = block_excl_sum(u, red, utot);
+        sc[tid] = cpre;
+        so[tid] = upre;
+        if (tid == 0) {
+            s_take = 0;
+            s_end = 0xffffffffu;
+        }
+        __syncthreads();
+        if (t < nt && upre + u <= kPieceUnc) atomicMax(&s_take, tid + 1);
+        __syncthreads();
+        const uint32_t take = s_take;
+        if (tid == take - 1) {
+            so[take] = upre + u;
+            s_call = cpre + c;
+        }
+        __syncthreads();
+        const uint32_t tot = so[take], call = s_call;
+        for (uint32_t q = w; q < take; q += kResThreads / 32) {
+            const uint2* src = a.unc + (size_t)(t0 + q) * kTileUnc;
+            const uint32_t o = so[q], cnt = so[q + 1] - o, add = cbase + sc[q];
+#pragma unroll 4
+            for (uint32_t j = lane; j < cnt; j += 32) su[o + j] = src[j].x + add;
+        }
+        __syncthreads();
+        int d[kResEach];  // accepted iff d >= a
+#pragma unroll
+        for (int e = 0; e < kResEach; e++) {
+            const uint32_t k = tid * kResEach + e;
+            d[e] = k < tot ? top - (int)su[k] : INT32_MIN;
+        }
+        uint32_t start = abase + tid * kResEach / 2, mask = 0;
+        for (int pass = 0; pass <= kResThreads; pass++) {  // thread k is settled after pass k at the latest
+            int acc = (int)start;
+            mask = 0;
+#pragma unroll
+            for (int e = 0; e < kResEach; e++)
+                if (d[e] >= acc) {
+                    mask |= 1u << e;
+                    acc++;
+                }
+            uint32_t all;
+            const uint32_t next = abase + block_excl_sum((uint32_t)(acc - (int)start), red, all);
+            const bool moved = next != start;
+            start = next;
+            if (tid == kResThreads - 1) sbef[kResThreads] = abase + all;
+            if (!__syncthreads_or(moved)) break;
+        }
+        smask[tid] = mask;
+        sbef[tid] = start;
+        {
+            const uint32_t hi = __shfl_down_sync(0xffffffffu, mask, 1);
+            if (!(tid & 1)) a.ok[words + tid / 2] = mask | (hi << 16);
+        }
+        __syncthreads();
+        // uncertain acceptances before entry k of the piece
+        const auto before = [&](uint32_t k) {
+            const uint32_t r = k % kResEach;
+            return sbef[k / kResEach] + (r ? (uint32_t)__popc(smask[k / kResEach] & ((1u << r) - 1u)) : 0u);
+        };
+        if (tid < take) {
+            const uint32_t b = before(so[tid]);
+            const uint32_t rank = s.i + cbase + sc[tid] + b;
+            a.base[t] = rank;
+            a.uoff[t] = words * 32 + so[tid];
+            if (rank + c + (before(so[tid + 1]) - b) >= a.n) atomicMin(&s_end, t);
+        }
+        __syncthreads();
+        t_end = s_end;
+        cbase += call;
+        abase = sbef[kResThreads];
+        t0 += take;
+        words += kPieceUnc / 32;
+        __syncthreads();
+    }
+    if (tid) return;
+    FyState z = s;
+    if (t_end == 0xffffffffu) {
+        z.pos += nt;
+        z.i += cbase + abase;
+        *a.seg = FySeg{nt, s.m};
+    } else {
+        // The permutation ends in tile t_end. gen_perm refills when its index
+        // reaches the end of a buffer, the last accepted draw included: when
+        // that draw is the buffer's last one, one more buffer is used. The
+        // last acceptance has v = 0 (T = 0), so it is the buffer's last draw
+        // iff that draw is 0 and was accepted (a 0 is always a candidate, so
+        // it is the last candidate of the tile's last run).
+        const unsigned long long te = s.pos + t_end;
+        unsigned long long next = te / a.tpb + 1;
+        if (te % a.tpb == a.tpb - 1 &&
+            a.raw[((size_t)(te % a.ring_tiles) + 1) * (kRuns * a.rl * kListDraws) - 1] == 0) {
+            const FyRun r = a.run[(size_t)t_end * kRuns + kRuns - 1];
+            bool ok = true;
+            if (r.unc && a.unc[(size_t)t_end * kTileUnc + r.upre + r.unc - 1].y == r.cnt - 1) {
+                const uint32_t k = a.uoff[t_end] + r.upre + r.unc - 1;
+                ok = (a.ok[k >> 5] >> (k & 31u)) & 1u;
+            }
+            if (ok) next++;
+        }
+        z.start = next;
+        z.pos = next * a.tpb;
+        z.i = 0;
+        z.m++;
+        z.done = z.m >= a.count;
+        *a.seg = FySeg{t_end + 1, s.m};
+    }
+    // `bad` is only ever set, by this step's classification before this
+    // launch or the emission after it
+    a.state->pos = z.pos;
+    a.state->start = z.start;
+    a.state->m = z.m;
+    a.state->i = z.i;
+    a.state->done = z.done;
+}
+
+// Writes a step's accepted offsets at their ranks: a run's candidates without
+// its rejected uncertain draws, which are marked in a bitmap so that ranks are
+// popcounts. Checks that T at the start of every run lay in the window its
+// classification assumed, which makes the whole step exact.
+__global__ void __launch_bounds__(kRuns * 32, 4) k_fy_emit(FyScanArgs a) {
+    constexpr uint32_t kWords = kMaxRunLists * kListDraws / 32;
+    __shared__ uint32_t sacc[kRuns], bm[kRuns][kWords];
+    const FySeg seg = *a.seg;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t* acc = a.acc + ((size_t)seg.m * 3 + a.g) * a.n;
+    for (uint32_t t = blockIdx.x; t < seg.ntiles; t += gridDim.x) {
+        const FyRun r = a.run[(size_t)t * kRuns + w];
+        const uint2* un = a.unc + (size_t)t * kTileUnc + r.upre;
+        const uint32_t k0 = a.uoff[t] + r.upre;
+        for (uint32_t j = lane; j * 32 < r.cnt; j += 32) bm[w][j] = 0;
+        __syncwarp();
+        uint32_t mine = 0;
+        for (uint32_t j = lane; j < r.unc; j += 32) {
+            const uint32_t p = un[j].y;
+            const bool ok = (a.ok[(k0 + j) >> 5] >> ((k0 + j) & 31u)) & 1u;
+            mine += ok;
+            if (!ok && p < r.cnt) atomicOr(&bm[w][p >> 5], 1u << (p & 31u));
+        }
+        mine = __reduce_add_sync(0xffffffffu, mine);
+        if (lane == 0) sacc[w] = mine;
+        __syncthreads();
+        uint32_t out = a.base[t] + r.cpre;
+        for (int k = 0; k < w; k++) out += sacc[k];
+        __syncthreads();
+        const long long T = (long long)a.n - 1 - out;
+        // past the permutation's end (T < 0) nothing may be certain
+        const bool good = T >= 0 ? (T >= r.lo && T <= r.hi) : r.cnt == r.unc;
+        if (!good && lane == 0) atomicOr(&a.state->bad, 1u);
+        const uint32_t* cand = a.cand + ((size_t)t * kRuns + w) * (a.rl * kListDraws);
+        for (uint32_t b = 0; b < r.cnt; b += 256) {
+            uint32_t v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const uint32_t p = b + 32 * k + lane;
+                v[k] = p < r.cnt ? cand[p] : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const uint32_t p = b + 32 * k + lane;
+                if (b + 32 * k >= r.cnt) break;
+                const uint32_t rej = bm[w][(b >> 5) + k];
+                const uint32_t o = out + (lane - __popc(rej & lt));
+                if (p < r.cnt && !((rej >> lane) & 1u) && o < a.n) acc[o] = v[k];
+                out += 32 - __popc(rej);
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // ---------------------------------------------------------------------------
-// Small permutations (M = 2^bit_width(n) <= 2^17). A permutation then takes
+// Small permutations (M = 2^bit_width(n) <= 2^15). A permutation then takes
 // d ≈ M·H_n draws (std ≈ 1.3·M) and 1 + floor(d / 2^20) getNext buffers, a
 // count that is predictable: permutation m of a group is assumed to start at
 // buffer m·b̂ of the chain, and every (permutation, group) pair runs at once,
@@ -203,7 +549,10 @@ __global__ void __launch_bounds__(kGenThreads, 1) k_fy_gen(FyGenArgs a) {
 // chunks sets `overflow`, and the general chain redoes everything.
 constexpr uint32_t kSmallChunk = 8192;  // draws per chunk
 constexpr int kSmallThreads = 512;
-constexpr uint32_t kSmallMaxM = 1u << 17;
+// above it predictions fail too often (at 2^16 one in 75 permutations) and a
+// repeated pass costs a whole permutation on one SM: the group-by of 60000
+// rows took 20.2 ms with this path and takes 19.5 with the chain
+constexpr uint32_t kSmallMaxM = 1u << 15;
 constexpr uint32_t kChunksPerBuffer = (1u << 20) / kSmallChunk;  // 128
 constexpr size_t kSmallSmem = (size_t)kAesSmemBytes + 2 * kSmallChunk * 4;
 
@@ -322,448 +671,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_fy_small(FySmallArgs a) {
         // the last accepted draw included: 1 + floor(draws / 2^20) buffers
         if (i >= n) a.used[g * a.count + m] = 1u + (s_dlast + 1u) / (1u << 20);
         else atomicOr(a.overflow, 1u);
-    }
-}
-
-struct FyScanArgs {
-    uint32_t n, count, tiles;
-    uint32_t g0;                   // group of block 0 (one launch per group)
-    unsigned long long win_tile0;  // absolute index of the window's first tile
-    FyLayout lay;
-    const uint32_t* ev;
-    const uint32_t* last;  // [3][tiles] masked value of each tile's last draw
-    const uint32_t* cnt;
-    FyState* state;     // [3]
-    uint32_t* acc;      // [count][3][n] accepted offsets v_i (swap with i + v_i)
-    uint32_t* refills;  // [3][count] getNext buffers used
-    unsigned long long* stats;  // optional [3][kFyStats] diagnostic counters (ORQ_FY_STATS)
-};
-
-
-// ---------------------------------------------------------------------------
-// The scanner. One 1024-thread CTA per group replays the acceptance of its
-// chain exactly. A step takes the next cs entries (<= 32768) of the current
-// level; warp w owns entries [1024w, 1024w + 1024) and at iteration u its lane
-// l holds entry q = 1024w + 32u + l, so loads, ranks and the stores of
-// accepted values are all lane-parallel (ballots and popcounts, no per-thread
-// serial loops) and coalesced. Level 1: entry q is certainly accepted if
-// v + q <= T (at most q acceptances precede it), certainly rejected if v > T,
-// otherwise uncertain. Level 2 (warp 0, 32 uncertain entries at a time):
-// with c = certain accepts before an uncertain entry and a = uncertain accepts
-// before it, it is accepted iff a <= T - c - v ("slack"); lane j of a chunk is
-// certain if slack >= a_chunk + j, rejected if slack < a_chunk, and only the
-// rest is decided lane by lane. A step with more uncertain entries than the
-// list holds is halved until they fit (a step of at most kUncCap entries
-// always does).
-constexpr uint32_t kMaxStepEntries = 32768;
-constexpr int kPerThread = kMaxStepEntries / kScanThreads;  // 32
-constexpr int kScanWarps = kScanThreads / 32;
-constexpr int kFyStats = 10;  // diagnostic counters per group
-constexpr int kQuads = kPerThread / 4;  // lane-quads per thread and step
-constexpr uint32_t kUncCap = 2048;
-// dynamic shared memory: the step's entries, then the lane-quad classes and
-// prefixes (cq below)
-constexpr size_t kScanSmem = (size_t)kMaxStepEntries * 4 + (size_t)kScanWarps * kQuads * 32 * 4;
-
-// entries per step at level L: uncertain entries of a step are about
-// cs^2 / (2 n/4^L); keep that near 512
-__device__ __forceinline__ uint32_t step_entries(uint32_t n, uint32_t L) {
-    const unsigned long long t = level_threshold(n, L);
-    uint32_t s = kMaxStepEntries;
-    while (s > 1024 && (unsigned long long)s * s > 1024ull * t) s >>= 1;
-    return s;
-}
-
-// 4-byte global -> shared copy that completes asynchronously (cp.async);
-// dst is a shared-window address
-__device__ __forceinline__ void cp_async4(uint32_t dst, const uint32_t* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-// bulk prefetch of [addr, addr + bytes) into L2; addr and bytes multiples of 16
-// (the range may round a list out to 16 bytes: list buffers carry slack)
-__device__ __forceinline__ void prefetch_l2(uintptr_t addr, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(addr), "r"(bytes) : "memory");
-}
-
-// class of entry q with value v in a step of cs entries at bound T: bit 0
-// certainly accepted (v + q <= T: at most q acceptances precede it), bit 4
-// uncertain (v <= T but not certain); rejected otherwise
-// (v < n < 2^31 and q < 2^15 for real entries, so v + q fits 32 bits; the
-// padding entries beyond cs are excluded first)
-__device__ __forceinline__ uint32_t fy_class(uint32_t q, uint32_t v, uint32_t cs, uint32_t T) {
-    const bool in = q < cs;
-    const bool cert = in && v + q <= T;
-    const bool unc = in && !cert && v <= T;
-    return (uint32_t)cert | ((uint32_t)unc << 4);
-}
-
-// exclusive warp prefix and warp total of a lane-quad's (certain | uncertain << 16)
-__device__ __forceinline__ void quad_prefix(uint32_t code, int lane, uint32_t& excl, uint32_t& total) {
-    const uint32_t x = __popc(code & 0xfu) | (__popc(code >> 4) << 16);
-    uint32_t inc = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    total = __shfl_sync(0xffffffffu, inc, 31);
-    excl = inc - x;
-}
-
-// tile holding entry e, searching P[lo..hi] (P[lo] <= e < P[hi+1])
-__device__ __forceinline__ uint32_t tile_in(const uint32_t* P, uint32_t lo, uint32_t hi, uint32_t e) {
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (P[mid] <= e) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// quads (128 entries) of warp w's range [1024w, 1024w + 1024) below cs
-__device__ __forceinline__ int wquads(int w, uint32_t cs) {
-    const uint32_t b = (uint32_t)w * 1024u;
-    return b >= cs ? 0 : (int)min((uint32_t)kQuads, (cs - b + 127u) / 128u);
-}
-
-__global__ void __launch_bounds__(kScanThreads, 1) k_fy_scan(FyScanArgs a) {
-    extern __shared__ __align__(16) uint32_t sv[];  // step entries, sv[q]
-    __shared__ uint32_t red[33];
-    __shared__ uint32_t P[kMaxWindowTiles + 1];  // prefix of level-L counts over the window
-    __shared__ uint32_t unc_v[kUncCap], unc_cp[kUncCap], unc_pre[kUncCap + 1];
-    __shared__ uint32_t wtot[kScanWarps], wpre[kScanWarps];
-    // per warp, quad iteration and lane: bits 0-7 the four entries' classes,
-    // bits 8-18 the certain and bits 19-29 the uncertain entries of the warp
-    // before this lane-quad (at most 1024 each); in the dynamic allocation
-    // after the entries (static shared memory is limited to 48 KB)
-    auto cq = reinterpret_cast<uint32_t (*)[kQuads][32]>(sv + kMaxStepEntries);
-    __shared__ uint32_t s_last_q, s_uacc, s_tot;
-    const uint32_t g = a.g0 + blockIdx.x;
-    const uint32_t n = a.n;
-    const uint32_t tiles = a.tiles;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t lt = (1u << lane) - 1u;
-    // scan state, identical in every thread
-    uint32_t i = a.state[g].i, m = a.state[g].m, done = a.state[g].done;
-    unsigned long long start = a.state[g].start_tile;
-    uint32_t tau = 0, ix = 0, L = 0, Lp = 0xffffffffu;
-    const uint32_t* EV = a.ev + (size_t)g * tiles * a.lay.slot;
-    const uint32_t* LAST = a.last + (size_t)g * tiles;
-    const uint32_t* C = a.cnt + (size_t)g * tiles * kMaxLevels;
-    unsigned long long st_steps = 0, st_unc_steps = 0, st_ent = 0, st_unc = 0,
-                       st_cyc_load = 0, st_cyc_unc = 0, st_cyc_all = 0, st_cyc_list = 0, st_cyc_acc = 0;
-    const unsigned long long t_begin = clock64();
-    for (int guard = 0; guard < (1 << 24) && !done; guard++) {
-        // never look before the current permutation's first tile
-        if (a.win_tile0 + tau < start) {
-            const unsigned long long d = start - a.win_tile0;
-            tau = d > tiles ? tiles : (uint32_t)d;
-            ix = 0;
-        }
-        if (tau >= tiles) break;
-        const uint32_t T = n - 1 - i;
-        // sparsest level still holding every candidate v <= T
-        uint32_t want = 0;
-        while (want + 1 < a.lay.nl && T < level_threshold(n, want + 1)) want++;
-        if (ix == 0) L = want;  // levels change only at tile starts
-        if (L != Lp) {
-            uint32_t tot;
-            const uint32_t c = threadIdx.x < tiles ? C[threadIdx.x * kMaxLevels + L] : 0u;
-            const uint32_t pre = block_excl_sum(c, red, tot);
-            if (threadIdx.x < tiles) P[threadIdx.x] = pre;
-            if (threadIdx.x == 0) P[tiles] = tot;
-            __syncthreads();
-            Lp = L;
-        }
-        const uint32_t e0 = P[tau] + ix;
-        const uint32_t eend = (ix != 0 && want != L) ? P[tau + 1] : P[tiles];
-        if (e0 >= eend) {
-            if (eend == P[tiles]) tau = tiles;
-            else {
-                tau++;
-                ix = 0;
-            }
-            continue;
-        }
-        uint32_t cs = min(step_entries(n, L), eend - e0);
-        const unsigned long long t_l0 = clock64();
-        if (warp == 0) {
-            // warm L2 with the entries of the next two steps (a hint: the
-            // staging of a later step then reads L2 instead of DRAM); lane j
-            // covers the j-th tile of that range
-            const uint32_t pf0 = e0 + cs, pf1 = min(P[tiles], e0 + cs + 2 * step_entries(n, L));
-            if (pf0 < pf1) {
-                const uint32_t t = tile_in(P, tau, tiles - 1, pf0) + lane;
-                if (t < tiles && P[t] < pf1) {
-                    const uint32_t s0 = max(P[t], pf0), s1 = min(P[t + 1], pf1);
-                    if (s0 < s1) {
-                        const uint32_t* src = EV + (size_t)t * a.lay.slot + a.lay.off[L] + (s0 - P[t]);
-                        const uintptr_t lo = (uintptr_t)src & ~(uintptr_t)15;
-                        const uintptr_t hi = ((uintptr_t)(src + (s1 - s0)) + 15) & ~(uintptr_t)15;
-                        prefetch_l2(lo, (uint32_t)(hi - lo));
-                    }
-                }
-            }
-        }
-        const uint32_t qw = (uint32_t)warp * 1024u + lane;  // staging: this thread's entry at u = 0
-        // ---- stage the step's entries into shared memory at sv[q] with
-        // asynchronous copies: no registers hold them, so all of a thread's
-        // loads are in flight at once (coalesced per iteration; each lane walks
-        // its tile cursor forward). Warp w stages and then processes entries
-        // [1024w, 1024w + 1024), so a warp-level sync publishes them.
-        {
-            // the lane's current tile: entry e lives at EV[boff + e] while
-            // e < tend; the tile advances only when a lane crosses into the next
-            const size_t off = a.lay.off[L];
-            uint32_t t = tau;
-            uint32_t tend = P[t + 1];
-            size_t boff = (size_t)t * a.lay.slot + off - (size_t)P[t];  // wraps; boff + e does not
-            const uint32_t sv_sh = (uint32_t)__cvta_generic_to_shared(sv);
-            // entries past cs are never read as entries (their class is
-            // forced to rejected), so they are not staged
-#pragma unroll
-            for (int u = 0; u < kPerThread; u++) {
-                if ((uint32_t)warp * 1024u + 32u * u >= cs) break;  // warp-uniform
-                const uint32_t q = qw + 32u * u;
-                if (q < cs) {
-                    const uint32_t e = e0 + q;
-                    if (e >= tend) {
-                        do {
-                            t++;
-                        } while (P[t + 1] <= e);
-                        tend = P[t + 1];
-                        boff = (size_t)t * a.lay.slot + off - (size_t)P[t];
-                    }
-                    cp_async4(sv_sh + 4u * q, EV + (boff + e));
-                }
-            }
-            cp_async_wait_all();
-        }
-        __syncwarp();
-        // In the passes below lane l of warp w holds, at iteration u, the four
-        // consecutive entries q = 1024w + 128u + 4l + r (r = 0..3); cq[w][u][l]
-        // keeps their classification (bit r: certainly accepted, bit 4 + r:
-        // uncertain): a lane-quad is one 16-byte shared load, and ranks come
-        // from one packed warp scan per 128 entries.
-        const uint32_t q0 = (uint32_t)warp * 1024u + 4u * (uint32_t)lane;
-        // ---- level 1 counts per warp, block prefix over warps; halve the step
-        // while the uncertain entries do not fit the list
-        uint32_t tot_c, tot_u;
-        for (;;) {
-            uint32_t x = 0;  // the warp's (certain | uncertain << 16) so far
-            // the warp's quads holding entries (warp-uniform; the passes below
-            // skip the rest, whose classes would all be zero)
-            const int nq = wquads(warp, cs);
-#pragma unroll
-            for (int u = 0; u < kQuads; u++) {
-                if (u >= nq) break;
-                const uint32_t q = q0 + 128u * u;
-                const uint4 v4 = *reinterpret_cast<const uint4*>(sv + q);
-                const uint32_t code = fy_class(q, v4.x, cs, T) | (fy_class(q + 1, v4.y, cs, T) << 1) |
-                                      (fy_class(q + 2, v4.z, cs, T) << 2) | (fy_class(q + 3, v4.w, cs, T) << 3);
-                uint32_t ex, tot;
-                quad_prefix(code, lane, ex, tot);
-                const uint32_t pre = x + ex;
-                cq[warp][u][lane] = code | ((pre & 0xffffu) << 8) | ((pre >> 16) << 19);
-                x += tot;
-            }
-            if (lane == 0) wtot[warp] = x;
-            __syncthreads();
-            if (warp == 0) {
-                const uint32_t y = wtot[lane];
-                uint32_t inc = y;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t z = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += z;
-                }
-                wpre[lane] = inc - y;
-                if (lane == 31) s_tot = inc;
-            }
-            __syncthreads();
-            tot_c = s_tot & 0xffffu;
-            tot_u = s_tot >> 16;
-            if (tot_u <= kUncCap) break;
-            cs >>= 1;  // uniform: every thread read the same total
-            __syncthreads();
-        }
-        const uint32_t cbase = wpre[warp] & 0xffffu, ubase = wpre[warp] >> 16;
-        st_steps++;
-        st_ent += cs;
-        st_cyc_load += clock64() - t_l0;
-        const unsigned long long t_li0 = clock64();
-        // ---- list the uncertain entries in order, with the certain accepts
-        // before each
-        const int nq = wquads(warp, cs);
-        if (tot_u) {
-#pragma unroll
-            for (int u = 0; u < kQuads; u++) {
-                if (u >= nq) break;
-                const uint32_t cw = cq[warp][u][lane];
-                const uint32_t code = cw & 0xffu;
-                if (code >> 4) {
-                    const uint32_t q = q0 + 128u * u;
-                    uint32_t c = cbase + ((cw >> 8) & 0x7ffu), k = ubase + (cw >> 19);
-#pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        if ((code >> (4 + r)) & 1u) {
-                            unc_v[k] = sv[q + r];
-                            unc_cp[k] = c;
-                            k++;
-                        }
-                        c += (code >> r) & 1u;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        const unsigned long long t_u0 = clock64();
-        st_cyc_list += t_u0 - t_li0;
-        if (warp == 0) {
-            // level 2 over the listed uncertain entries
-            uint32_t acc_so_far = 0;
-            for (uint32_t base = 0; base < tot_u; base += 32) {
-                const uint32_t k = base + lane;
-                const bool valid = k < tot_u;
-                long long slack = -1;
-                if (valid) slack = (long long)T - unc_cp[k] - unc_v[k];
-                const bool cert = valid && slack >= (long long)acc_so_far + lane;
-                const bool und = valid && !cert && slack >= (long long)acc_so_far;
-                uint32_t okmask = __ballot_sync(0xffffffffu, cert);
-                const uint32_t undmask = __ballot_sync(0xffffffffu, und);
-                if (undmask) {
-                    // decide the undetermined lanes in order; the certain ones
-                    // (already in okmask) and the rejected ones do not depend
-                    // on the lanes before them
-                    uint32_t pend = undmask;
-                    while (pend) {
-                        const int j = __ffs(pend) - 1;
-                        pend &= pend - 1;
-                        const long long sj = __shfl_sync(0xffffffffu, slack, j);
-                        const uint32_t before = acc_so_far + __popc(okmask & ((1u << j) - 1u));
-                        if (sj >= (long long)before) okmask |= 1u << j;
-                    }
-                }
-                if (valid) {
-                    unc_pre[k] = acc_so_far + __popc(okmask & lt);
-                    unc_cp[k] = (okmask >> lane) & 1u;  // reuse as the decision
-                }
-                acc_so_far += __popc(okmask);
-            }
-            if (lane == 0) {
-                unc_pre[tot_u] = acc_so_far;
-                s_uacc = acc_so_far;
-            }
-        }
-        __syncthreads();
-        if (tot_u) {
-            st_unc_steps++;
-            st_unc += tot_u;
-            st_cyc_unc += clock64() - t_u0;
-        }
-        // ---- accept, rank, store (a lane's accepted entries go to consecutive
-        // ranks, consecutive lanes to consecutive runs)
-        const unsigned long long t_a0 = clock64();
-        const uint32_t tot_a = tot_c + s_uacc;
-        const uint32_t need = n - i;
-        uint32_t* acc = a.acc + ((size_t)m * 3 + g) * (size_t)n;
-        {
-            uint32_t* acci = acc + i;
-#pragma unroll
-            for (int u = 0; u < kQuads; u++) {
-                if (u >= nq) break;
-                const uint32_t cw = cq[warp][u][lane];
-                const uint32_t code = cw & 0xffu;
-                if (code) {
-                    const uint32_t q = q0 + 128u * u;
-                    const uint4 v4 = *reinterpret_cast<const uint4*>(sv + q);
-                    const uint32_t vv[4] = {v4.x, v4.y, v4.z, v4.w};
-                    // certain / uncertain entries before q + r
-                    uint32_t c = cbase + ((cw >> 8) & 0x7ffu), k = ubase + (cw >> 19);
-                    if ((code >> 4) == 0) {
-                        // no uncertain entry in the quad: one lookup of the
-                        // uncertain acceptances before it serves all four
-                        const uint32_t up = unc_pre[k];
-#pragma unroll
-                        for (int r = 0; r < 4; r++) {
-                            if ((code >> r) & 1u) {
-                                const uint32_t rank = c + up;
-                                if (rank < need) {
-                                    acci[rank] = vv[r];
-                                    if (rank == need - 1) s_last_q = q + r;
-                                }
-                                c++;
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int r = 0; r < 4; r++) {
-                            const bool cert = (code >> r) & 1u, unc = (code >> (4 + r)) & 1u;
-                            if (cert || (unc && unc_cp[k])) {
-                                const uint32_t rank = c + unc_pre[k];
-                                if (rank < need) {
-                                    acci[rank] = vv[r];
-                                    if (rank == need - 1) s_last_q = q + r;
-                                }
-                            }
-                            c += cert;
-                            k += unc;
-                        }
-                    }
-                }
-            }
-        }
-        if (tot_a >= need) {
-            __syncthreads();
-            // permutation complete: locate its last draw, count the getNext buffers
-            const uint32_t e = e0 + s_last_q;
-            const uint32_t t = tile_in(P, tau, tiles - 1, e);
-            // only a last draw at the very end of a getNext buffer changes the
-            // count below: that is the tile's last draw, and then it is the
-            // last entry of the tile's list
-            const bool tile_end = e + 1 == P[t + 1] && LAST[t] < level_threshold(n, L);
-            const unsigned long long kend =
-                (a.win_tile0 + t - start) * (unsigned long long)kTileDraws + (tile_end ? kTileDraws - 1 : 0);
-            const unsigned long long R = 1 + ((kend + 1) >> 20);
-            if (threadIdx.x == 0) a.refills[(size_t)g * a.count + m] = (uint32_t)R;
-            start = (start / kTilesPerRefill + R) * kTilesPerRefill;
-            m++;
-            i = 0;
-            ix = 0;
-            if (m >= a.count) done = 1;
-        } else {
-            i += tot_a;
-            const uint32_t enew = e0 + cs;
-            if (enew >= P[tiles]) {
-                tau = tiles;
-                ix = 0;
-            } else {
-                tau = tile_in(P, tau, tiles - 1, enew);
-                ix = enew - P[tau];
-            }
-        }
-        __syncthreads();  // the lists and counters are reused by the next step
-        st_cyc_acc += clock64() - t_a0;
-    }
-    if (threadIdx.x == 0) {
-        a.state[g].i = i;
-        a.state[g].m = m;
-        a.state[g].done = done;
-        a.state[g].start_tile = start;
-        if (a.stats) {
-            st_cyc_all = clock64() - t_begin;
-            unsigned long long* st = a.stats + g * kFyStats;
-            st[0] += st_steps;
-            st[1] += st_unc_steps;
-            st[3] += st_ent;
-            st[4] += st_unc;
-            st[5] += st_cyc_load;
-            st[6] += st_cyc_unc;
-            st[7] += st_cyc_all;
-            st[8] += st_cyc_list;
-            st[9] += st_cyc_acc;
-        }
     }
 }
 
@@ -965,9 +872,8 @@ namespace {
 FyRes& fy_res(Ctx& c) {
     FyRes& R = c.fy;
     if (R.ready) return R;
-    // the scanners' streams have the highest priority: when generator CTAs
-    // (which fill an SM's registers and shared memory) retire, pending scans
-    // are dispatched before the next generator window
+    // the scans' streams have the highest priority: their small CTAs are
+    // dispatched before the next generator launch's
     int prio_lo = 0, prio_hi = 0;
     ORQ_CUDA_CHECK(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
     ORQ_CUDA_CHECK(cudaStreamCreateWithPriority(&R.gs, cudaStreamNonBlocking, prio_lo));
@@ -975,14 +881,12 @@ FyRes& fy_res(Ctx& c) {
     ORQ_CUDA_CHECK(cudaStreamCreateWithPriority(&R.fs, cudaStreamNonBlocking, prio_lo));
     ORQ_CUDA_CHECK(cudaEventCreateWithFlags(&R.ev_start, cudaEventDisableTiming));
     ORQ_CUDA_CHECK(cudaEventCreateWithFlags(&R.fin_done, cudaEventDisableTiming));
-    for (int k = 0; k < kFyRingMax; k++) {
-        ORQ_CUDA_CHECK(cudaEventCreateWithFlags(&R.gen_done[k], cudaEventDisableTiming));
+    for (int k = 0; k < kFyInFlight; k++)
         for (int g = 0; g < 3; g++) {
-            ORQ_CUDA_CHECK(cudaEventCreateWithFlags(&R.scan_done[g][k], cudaEventDisableTiming));
+            ORQ_CUDA_CHECK(cudaEventCreateWithFlags(&R.gen_done[g][k], cudaEventDisableTiming));
             ORQ_CUDA_CHECK(cudaEventCreateWithFlags(&R.st_ev[g][k], cudaEventDisableTiming));
         }
-    }
-    ORQ_CUDA_CHECK(cudaMallocHost(&R.hst, (size_t)kFyRingMax * 3 * sizeof(FyState)));
+    ORQ_CUDA_CHECK(cudaMallocHost(&R.hst, (size_t)kFyInFlight * 3 * sizeof(FyState)));
     R.ready = true;
     return R;
 }
@@ -996,13 +900,11 @@ void release_fy(Ctx& c) {
     cudaStreamSynchronize(R.fs);
     cudaEventDestroy(R.ev_start);
     cudaEventDestroy(R.fin_done);
-    for (int k = 0; k < kFyRingMax; k++) {
-        cudaEventDestroy(R.gen_done[k]);
+    for (int k = 0; k < kFyInFlight; k++)
         for (int g = 0; g < 3; g++) {
-            cudaEventDestroy(R.scan_done[g][k]);
+            cudaEventDestroy(R.gen_done[g][k]);
             cudaEventDestroy(R.st_ev[g][k]);
         }
-    }
     cudaStreamDestroy(R.gs);
     for (int g = 0; g < 3; g++) cudaStreamDestroy(R.ss[g]);
     cudaStreamDestroy(R.fs);
@@ -1037,53 +939,13 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     for (size_t k = 1; k <= std::min<size_t>(n, 1 << 16); k++) H += 1.0 / k;
     if (n > (1u << 16)) H += std::log((double)n / (1 << 16));
     const double per_perm = M * H / (double)(1 << 20) + 1.0;  // expected buffers
-    uint32_t W = (uint32_t)std::clamp(per_perm * count / 8.0, 2.0, (double)(kMaxWindowTiles / kTilesPerRefill));
-    const uint32_t tiles = W * kTilesPerRefill;
-
-    FyLayout lay{};
-    {
-        // levels down to a threshold of 256: sparser ones would hold almost
-        // nothing, and the scan of a permutation's last steps reads at most a
-        // few thousand entries of the last level instead
-        uint32_t nl = 1;
-        while (nl < (uint32_t)kMaxLevels && level_threshold((uint32_t)n, nl) >= 256) nl++;
-        lay.nl = nl;
-        uint32_t o = 0;
-        for (uint32_t L = 0; L < nl; L++) {
-            lay.off[L] = o;
-            lay.cap[L] = level_capacity(L);
-            o += lay.cap[L];
-        }
-        lay.slot = o;
-    }
-    const size_t ents_b = (size_t)3 * tiles * lay.slot * 4;
-    const size_t cnt_b = (size_t)3 * tiles * kMaxLevels * 4;
-    // Ring of window buffers: the draws of a window do not depend on the scan
-    // (windows are consecutive buffers of the group streams), so the generator
-    // runs up to kRing-1 windows ahead. It stays ahead through the dense start
-    // of a permutation (scan-bound) and the scanner catches up through the
-    // sparse tail (generation-bound). The three groups are scanned on three
-    // streams: their dense phases fall in different windows, and a shared
-    // launch per window would cost the slowest group every time.
-    // (allocated below, after the small-permutation path, which needs none)
-    constexpr int kRing = 6;
     Scratch acc(c, (size_t)3 * count * n * 4);
-    const bool want_stats = std::getenv("ORQ_FY_STATS") != nullptr;
-    const auto t_start = std::chrono::steady_clock::now();
-
-    // generator and scanner run on private non-blocking streams so they overlap
+    // generator and scans run on private non-blocking streams so they overlap
     // whatever the caller's stream is (the legacy default stream included)
-    // the scanner's stream has the highest priority: when generator CTAs
-    // (which fill an SM's registers and shared memory) retire, a pending scan
-    // is dispatched before the next generator window
     FyRes& R = fy_res(c);
     cudaStream_t gs = R.gs;
     cudaStream_t* ss = R.ss;
     cudaEvent_t ev_start = R.ev_start;
-    auto& gen_done = R.gen_done;
-    auto& scan_done = R.scan_done;
-    auto& st_ev = R.st_ev;
-    static_assert(kRing <= kFyRingMax, "ring deeper than the cached events");
     // On every exit path (an exception included) the generator and scanner
     // streams are drained before the ring, state and output scratch above go
     // back to the pool: a later call on the runtime's stream could otherwise
@@ -1236,180 +1098,209 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         // the general chain below redoes all of them (no nonce was consumed)
     }
 
-    std::vector<std::unique_ptr<Scratch>> ring_ev, ring_last, ring_cnt;
-    for (int k = 0; k < kRing; k++) {
-        ring_ev.emplace_back(new Scratch(c, ents_b + 256));  // slack for 16-byte rounded prefetches
-        ring_last.emplace_back(new Scratch(c, (size_t)3 * tiles * 4));
-        ring_cnt.emplace_back(new Scratch(c, cnt_b));
+    // Buffers are generated `W` at a time per group into a ring of kRing * W
+    // (up to kRing - 1 chunks ahead of the scan: the draws do not depend on
+    // it). W buffers of 2^20 draws keep every SM busy for ~6 us each.
+    constexpr uint32_t kRing = 4;
+    // Three SMs are left to k_fy_resolve, whose registers do not fit beside a
+    // generator CTA's; W is rounded so that the last wave of lists is full.
+    const uint32_t gen_sms = (uint32_t)std::max(1, c.num_sms - 3), gen_warps = gen_sms * (kGenThreads / 32);
+    const double want = std::clamp(per_perm * count / 8.0, 2.0, 64.0);
+    const uint32_t waves = std::max(1u, (uint32_t)(want * kListsPerBuf / gen_warps));
+    const uint32_t W = std::max(2u, waves * gen_warps / kListsPerBuf);
+    // Runs of 8192 draws, or shorter ones where a permutation has few of them:
+    // a step's latency is then what counts, and more warps share its draws.
+    const uint32_t rl = M >= (double)(1u << 22) ? 4 : (M >= (double)(1u << 20) ? 2 : 1);
+    const uint32_t tpb = kListsPerBuf / (kRuns * rl);
+    const uint32_t ring_bufs = kRing * W, ring_tiles = ring_bufs * tpb, seg_cap = W * tpb;
+    struct Group {
+        std::unique_ptr<Scratch> raw, lst, lcnt, tab, cand, unc, run, tc, tu, base, uoff, ok;
+        unsigned long long gen = 0;   // buffers generated (or queued)
+        unsigned long long pos = 0;   // tiles known to be scanned
+        unsigned long long start = 0;
+        uint32_t m = 0;
+        bool done = false;
+        unsigned head = 0, tail = 0;  // step batches queued / read back
+    } G[3];
+    for (auto& q : G) {
+        q.raw.reset(new Scratch(c, (size_t)ring_bufs * kBufDraws * 4));
+        q.lst.reset(new Scratch(c, (size_t)ring_bufs * kListsPerBuf * kListCap * 4));
+        q.lcnt.reset(new Scratch(c, (size_t)ring_bufs * kListsPerBuf * 4));
+        q.tab.reset(new Scratch(c, (size_t)ring_bufs * 4 * kTabEntries * sizeof(uint4)));
+        q.cand.reset(new Scratch(c, (size_t)W * kBufDraws * 4));
+        q.unc.reset(new Scratch(c, (size_t)seg_cap * kTileUnc * sizeof(uint2)));
+        q.run.reset(new Scratch(c, (size_t)seg_cap * kRuns * sizeof(FyRun)));
+        q.tc.reset(new Scratch(c, (size_t)seg_cap * 4));
+        q.tu.reset(new Scratch(c, (size_t)seg_cap * 4));
+        q.base.reset(new Scratch(c, (size_t)seg_cap * 4));
+        q.uoff.reset(new Scratch(c, (size_t)seg_cap * 4));
+        // a piece of k_fy_resolve takes at least one tile
+        q.ok.reset(new Scratch(c, (size_t)seg_cap * (kPieceUnc / 8)));
     }
-    Scratch state(c, 3 * sizeof(FyState));
-    Scratch refills(c, (size_t)3 * count * 4);
+    Scratch state(c, 3 * sizeof(FyState)), seg(c, 3 * sizeof(FySeg));
     ORQ_CUDA_CHECK(cudaMemsetAsync(state.p, 0, 3 * sizeof(FyState), c.stream));
-    Scratch stats(c, 3 * kFyStats * 8);
-    if (want_stats) ORQ_CUDA_CHECK(cudaMemsetAsync(stats.p, 0, 3 * kFyStats * 8, c.stream));
-    // the side streams start after these allocations and memsets, and are
+    // the side streams start after these allocations and the memset, and are
     // drained before the buffers above go back to the pool (declared after them)
     ORQ_CUDA_CHECK(cudaEventRecord(ev_start, c.stream));
     ORQ_CUDA_CHECK(cudaStreamWaitEvent(gs, ev_start, 0));
     for (int g = 0; g < 3; g++) ORQ_CUDA_CHECK(cudaStreamWaitEvent(ss[g], ev_start, 0));
     DrainSideStreams drain_ring{R};
-
     prep_aes_kernel(k_fy_gen);
-    ORQ_CUDA_CHECK(cudaFuncSetAttribute(k_fy_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScanSmem));
-
-    const unsigned gen_grid = (unsigned)std::max(1, c.num_sms - 3);
-    uint32_t* evp[kRing];
-    uint32_t* lastp[kRing];
-    uint32_t* cntp[kRing];
-    for (int k = 0; k < kRing; k++) {
-        evp[k] = ring_ev[k]->as<uint32_t>();
-        lastp[k] = ring_last[k]->as<uint32_t>();
-        cntp[k] = ring_cnt[k]->as<uint32_t>();
-    }
-
-    const unsigned long long limit_windows =
-        (unsigned long long)(count * (per_perm * 4.0 + 64.0) / W + 16);
-    std::vector<cudaEvent_t> tl;  // stats mode: [gen start, gen end, scan start, scan end] per window
-    auto tl_event = [&](cudaStream_t st) -> int {
-        if (!want_stats) return -1;
-        cudaEvent_t e;
-        ORQ_CUDA_CHECK(cudaEventCreate(&e));
-        ORQ_CUDA_CHECK(cudaEventRecord(e, st));
-        tl.push_back(e);
-        return (int)tl.size() - 1;
-    };
-    std::vector<std::array<int, 4>> tl_idx;
-    auto launch_gen = [&](unsigned long long w) {
-        const int b = (int)(w % kRing);
-        // buffer b was last read by the three scans of window w-kRing
-        if (w >= (unsigned long long)kRing)
-            for (int g = 0; g < 3; g++) ORQ_CUDA_CHECK(cudaStreamWaitEvent(gs, scan_done[g][b], 0));
-        FyGenArgs ga;
-        for (int g = 0; g < 3; g++) ga.st[g] = c.stream_arg(G01 + g, 4ull * W * w);
-        ga.n = (uint32_t)n;
-        ga.mask = mask;
-        ga.tiles = tiles;
-        ga.lay = lay;
-        ga.ev = evp[b];
-        ga.last = lastp[b];
-        ga.cnt = cntp[b];
-        ga.state = state.as<FyState>();
-        ga.err = c.d_err;
-        if (tl_idx.size() <= w) tl_idx.resize(w + 1, {-1, -1, -1, -1});
-        tl_idx[w][0] = tl_event(gs);
-        {
-            ProfScope ps(c, "fy_gen", 0.0, 3.0 * tiles * kTileBlocks, gs);
-            k_fy_gen<<<gen_grid, kGenThreads, kAesSmemBytes, gs>>>(ga);
-        }
-        tl_idx[w][1] = tl_event(gs);
-        ORQ_CUDA_CHECK(cudaGetLastError());
-        ORQ_CUDA_CHECK(cudaEventRecord(gen_done[b], gs));
-        c.kernels_launched++;
-    };
-    // Each group's scans are queued up to kRing-1 windows ahead of the host's
-    // completion check, so a scan stream always holds its next scan (its CTA
-    // takes the SM the previous one frees before any generator CTA can, by
-    // stream priority) and no host round trip idles a scanner. A scan queued
-    // after its group's last permutation completed sees `done` and returns.
     FyState* hst = static_cast<FyState*>(R.hst);
-    auto launch_scan = [&](unsigned long long w, int g) {
-        const int b = (int)(w % kRing);
-        ORQ_CUDA_CHECK(cudaStreamWaitEvent(ss[g], gen_done[b], 0));
-        FyScanArgs sa;
-        sa.n = (uint32_t)n;
-        sa.count = (uint32_t)count;
-        sa.tiles = tiles;
-        sa.g0 = (uint32_t)g;
-        sa.win_tile0 = (unsigned long long)w * tiles;
-        sa.lay = lay;
-        sa.ev = evp[b];
-        sa.last = lastp[b];
-        sa.cnt = cntp[b];
-        sa.state = state.as<FyState>();
-        sa.acc = acc.as<uint32_t>();
-        sa.refills = refills.as<uint32_t>();
-        sa.stats = want_stats ? stats.as<unsigned long long>() : nullptr;
-        if (tl_idx.size() <= w) tl_idx.resize(w + 1, {-1, -1, -1, -1});
-        if (g == 0) tl_idx[w][2] = tl_event(ss[0]);
-        {
-            ProfScope ps(c, "fy_scan", 0.0, 0.0, ss[g]);
-            k_fy_scan<<<1, kScanThreads, kScanSmem, ss[g]>>>(sa);
-        }
-        if (g == 0) tl_idx[w][3] = tl_event(ss[0]);
-        ORQ_CUDA_CHECK(cudaGetLastError());
-        ORQ_CUDA_CHECK(cudaEventRecord(scan_done[g][b], ss[g]));
-        c.kernels_launched++;
-        ORQ_CUDA_CHECK(cudaMemcpyAsync(hst + 3 * b + g, state.as<FyState>() + g, sizeof(FyState),
-                                       cudaMemcpyDeviceToHost, ss[g]));
-        ORQ_CUDA_CHECK(cudaEventRecord(st_ev[g][b], ss[g]));
-    };
-    // The host checks completion up to kRing-1 windows behind the launches
-    // while more windows are expected (no idle scanner, no host round trip on
-    // the critical path), then window by window, so a chain that ends early
-    // does not leave a ring's worth of windows queued.
-    const unsigned long long expect = (unsigned long long)std::ceil(per_perm * (double)count / W);
-    unsigned long long checked = 0;
-    bool finished = false;
-    for (unsigned long long w = 0; !finished; w++) {
-        if (w > limit_windows)
-            throw std::runtime_error("permutation generation did not converge");
-        launch_gen(w);
-        for (int g = 0; g < 3; g++) launch_scan(w, g);
-        const unsigned long long lag = (w + 1 < expect) ? (unsigned long long)(kRing - 1) : 0ull;
-        while (!finished && checked + lag <= w) {
-            const int pb = (int)(checked % kRing);
-            bool all = true;
-            size_t mmin = count;  // permutations every group has completed
-            for (int g = 0; g < 3; g++) {
-                ORQ_CUDA_CHECK(cudaEventSynchronize(st_ev[g][pb]));
-                all = all && hst[3 * pb + g].done;
-                mmin = std::min<size_t>(mmin, hst[3 * pb + g].done ? count : hst[3 * pb + g].m);
-            }
-            finished = all;
-            checked++;
-            if (!finished && fin_next + fin_b <= mmin) {
-                // their accepted offsets were written before this window's states
-                for (int g = 0; g < 3; g++) ORQ_CUDA_CHECK(cudaStreamWaitEvent(fs, st_ev[g][pb], 0));
-                for (; fin_next + fin_b <= mmin; fin_next += fin_b) launch_fin(fin_next, fin_next + fin_b);
-            }
-        }
-    }
-    const unsigned long long w = tl_idx.size();
-    ORQ_CUDA_CHECK(cudaStreamSynchronize(gs));
-    for (int g = 0; g < 3; g++) ORQ_CUDA_CHECK(cudaStreamSynchronize(ss[g]));
 
-    // nonce accounting: 4 nonces per getNext buffer
-    std::vector<uint32_t> hr(3 * count);
-    ORQ_CUDA_CHECK(cudaMemcpyAsync(hr.data(), refills.p, hr.size() * 4, cudaMemcpyDeviceToHost,
-                                   c.stream));
-    ORQ_CUDA_CHECK(cudaStreamSynchronize(c.stream));
+    const auto run_chain = [&](double width) -> bool {
+    FyScanArgs sa[3];
     for (int g = 0; g < 3; g++) {
-        unsigned long long used = 0;
-        for (size_t m = 0; m < count; m++) used += hr[g * count + m];
-        c.nonce[G01 + g] += 4ull * used;
+        FyScanArgs& x = sa[g];
+        x.n = (uint32_t)n;
+        x.count = (uint32_t)count;
+        x.g = (uint32_t)g;
+        x.mbits = (uint32_t)bitsw;
+        x.th = (uint32_t)(n >> 4);
+        x.rl = rl;
+        x.tpb = tpb;
+        x.ring_tiles = ring_tiles;
+        x.seg_cap = seg_cap;
+        x.limit = 0;
+        x.rate = std::log1p(-1.0 / M);
+        x.width = width;
+        x.raw = G[g].raw->as<uint32_t>();
+        x.lst = G[g].lst->as<uint32_t>();
+        x.lcnt = G[g].lcnt->as<uint32_t>();
+        x.state = state.as<FyState>() + g;
+        x.cand = G[g].cand->as<uint32_t>();
+        x.unc = G[g].unc->as<uint2>();
+        x.run = G[g].run->as<FyRun>();
+        x.tc = G[g].tc->as<uint32_t>();
+        x.tu = G[g].tu->as<uint32_t>();
+        x.base = G[g].base->as<uint32_t>();
+        x.uoff = G[g].uoff->as<uint32_t>();
+        x.ok = G[g].ok->as<uint32_t>();
+        x.seg = seg.as<FySeg>() + g;
+        x.acc = acc.as<uint32_t>();
     }
-    if (want_stats) {
-        std::fprintf(stderr, "[fy] windows %llu of %u buffers, %.3f ms\n", w, W,
-                     std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count());
-        for (size_t k = 0; k < tl_idx.size(); k++) {
-            float g0 = 0, g1 = 0, s0 = 0, s1 = 0;
-            if (tl_idx[k][0] >= 0) cudaEventElapsedTime(&g0, tl[0], tl[tl_idx[k][0]]);
-            if (tl_idx[k][1] >= 0) cudaEventElapsedTime(&g1, tl[0], tl[tl_idx[k][1]]);
-            if (tl_idx[k][2] >= 0) cudaEventElapsedTime(&s0, tl[0], tl[tl_idx[k][2]]);
-            if (tl_idx[k][3] >= 0) cudaEventElapsedTime(&s1, tl[0], tl[tl_idx[k][3]]);
-            std::fprintf(stderr, "[fy] window %zu: gen %.3f-%.3f scan %.3f-%.3f ms\n", k, g0, g1, s0, s1);
+    // a step ends with its permutation: a batch of steps covers the
+    // permutations a chunk of buffers can hold, and one step more
+    const int steps = (int)(W / per_perm) + 2;
+    const unsigned scan_grid = (unsigned)std::min<uint32_t>(seg_cap, (uint32_t)std::max(1, 2 * c.num_sms));
+    const auto queue_steps = [&](int g) {
+        Group& q = G[g];
+        const unsigned k = q.head % kFyInFlight;
+        for (int s = 0; s < steps; s++) {
+            ProfScope ps(c, "fy_scan", 0.0, 0.0, ss[g]);
+            k_fy_classify<<<scan_grid, kRuns * 32, 0, ss[g]>>>(sa[g]);
+            k_fy_resolve<<<1, kResThreads, 0, ss[g]>>>(sa[g]);
+            k_fy_emit<<<scan_grid, kRuns * 32, 0, ss[g]>>>(sa[g]);
+            c.kernels_launched += 3;
         }
-        for (auto e : tl) cudaEventDestroy(e);
-        unsigned long long hs[3 * kFyStats];
-        ORQ_CUDA_CHECK(cudaMemcpy(hs, stats.p, sizeof(hs), cudaMemcpyDeviceToHost));
-        for (int g = 0; g < 3; g++) {
-            const unsigned long long* h = hs + g * kFyStats;
-            std::fprintf(stderr,
-                         "[fy] n=%zu perms=%zu windows=%llu group %d: steps %llu unc_steps %llu entries %llu "
-                         "unc %llu cyc_load %llu cyc_list %llu cyc_unc %llu cyc_acc %llu cyc_all %llu\n",
-                         n, count, w, g, h[0], h[1], h[3], h[4], h[5], h[8], h[6], h[9], h[7]);
+        ORQ_CUDA_CHECK(cudaGetLastError());
+        ORQ_CUDA_CHECK(cudaMemcpyAsync(hst + kFyInFlight * g + k, state.as<FyState>() + g, sizeof(FyState),
+                                       cudaMemcpyDeviceToHost, ss[g]));
+        ORQ_CUDA_CHECK(cudaEventRecord(R.st_ev[g][k], ss[g]));
+        q.head++;
+    };
+    bool bad = false;
+    // waits for the oldest batch of steps queued for g
+    const auto read_back = [&](int g) {
+        Group& q = G[g];
+        if (q.head == q.tail) queue_steps(g);
+        const unsigned k = q.tail++ % kFyInFlight;
+        ORQ_CUDA_CHECK(cudaEventSynchronize(R.st_ev[g][k]));
+        const FyState& z = hst[kFyInFlight * g + k];
+        q.pos = z.pos;
+        q.start = z.start;
+        q.m = z.m;
+        q.done = z.done != 0;
+        bad = bad || z.bad;
+        const size_t mmin = std::min({G[0].m, G[1].m, G[2].m});
+        if (!bad && fin_next + fin_b <= mmin && mmin < count) {
+            // the accepted offsets of these permutations precede the states read
+            for (; fin_next + fin_b <= mmin; fin_next += fin_b) launch_fin(fin_next, fin_next + fin_b);
+        }
+    };
+    // Chunks shrink once a chain may end (a permutation's draws deviate by
+    // ~1.3 M), and then each waits for the scan of the one before it, so that
+    // little is generated past the end.
+    const double sure = per_perm * count - 2.6 * M * std::sqrt((double)count) / kBufDraws;
+    const double far = per_perm * 4.0 * count + 64.0 * count + 64.0;
+    while (!bad) {
+        int g = -1;
+        for (int k = 0; k < 3; k++)
+            if (!G[k].done && (g < 0 || G[k].gen < G[g].gen)) g = k;
+        if (g < 0) break;
+        Group& q = G[g];
+        if ((double)q.gen > far) throw std::runtime_error("permutation generation did not converge");
+        const bool tail = (double)q.gen >= sure;
+        unsigned long long b = q.gen;
+        // the chain never reads buffers before the current permutation's start
+        uint32_t take = tail ? std::max(1u, W / 4) : W;
+        take = (uint32_t)std::min<unsigned long long>(take, ring_bufs - b % ring_bufs);
+        // wait until the ring slots are free, and in the tail for every scan
+        if (q.head - q.tail == kFyInFlight || (b + take) * tpb > q.pos + ring_tiles ||
+            (tail && q.head != q.tail)) {
+            read_back(g);
+            continue;
+        }
+        if (tail && q.pos < b * tpb) {  // the queued steps stopped short of what is generated
+            read_back(g);
+            continue;
+        }
+        const size_t rb = b % ring_bufs;
+        uint4* tab = G[g].tab->as<uint4>() + rb * 4 * kTabEntries;
+        FyGenArgs ga;
+        ga.st = c.stream_arg(G01 + g, 4ull * b);
+        ga.tab = tab;
+        ga.mask = mask;
+        ga.th = (uint32_t)(n >> 4);
+        ga.lists = take * kListsPerBuf;
+        ga.raw = G[g].raw->as<uint32_t>() + rb * kBufDraws;
+        ga.lst = G[g].lst->as<uint32_t>() + rb * kListsPerBuf * kListCap;
+        ga.lcnt = G[g].lcnt->as<uint32_t>() + rb * kListsPerBuf;
+        ga.state = state.as<FyState>() + g;
+        {
+            ProfScope ps(c, "fy_gen", 0.0, (double)take * kBufDraws / 4, gs);
+            k_fy_tab<<<take * 4, 544, 0, gs>>>(ga.st, tab);
+            k_fy_gen<<<gen_sms, kGenThreads, kAesSmemBytes, gs>>>(ga);
+        }
+        ORQ_CUDA_CHECK(cudaGetLastError());
+        c.kernels_launched += 2;
+        q.gen = b + take;
+        sa[g].limit = q.gen * tpb;
+        ORQ_CUDA_CHECK(cudaEventRecord(R.gen_done[g][q.head % kFyInFlight], gs));
+        ORQ_CUDA_CHECK(cudaStreamWaitEvent(ss[g], R.gen_done[g][q.head % kFyInFlight], 0));
+        queue_steps(g);
+    }
+    // the last steps' emissions may still flag a window
+    for (int g = 0; g < 3; g++) ORQ_CUDA_CHECK(cudaStreamSynchronize(ss[g]));
+    ORQ_CUDA_CHECK(cudaMemcpyAsync(hst, state.p, 3 * sizeof(FyState), cudaMemcpyDeviceToHost, gs));
+    ORQ_CUDA_CHECK(cudaStreamSynchronize(gs));
+    for (int g = 0; g < 3; g++) {
+        bad = bad || hst[g].bad;
+        G[g].start = hst[g].start;
+    }
+    return !bad;
+    };
+    // A threshold outside its window (6 deviations: about once in 1e7
+    // permutations) shows up as `bad`: nothing has been consumed yet, so the
+    // chain runs again with wider windows. ORQ_FY_WIDTH sets the first width
+    // (tests narrow it).
+    const char* we = std::getenv("ORQ_FY_WIDTH");
+    double width = we ? std::clamp(std::atof(we), 0.25, 6.0) : 6.0;
+    while (!run_chain(width)) {
+        width *= 1.5;
+        if (width > 20.0) throw std::runtime_error("permutation generation did not converge");
+        ORQ_CUDA_CHECK(cudaStreamSynchronize(fs));
+        ORQ_CUDA_CHECK(cudaMemsetAsync(state.p, 0, 3 * sizeof(FyState), gs));
+        ORQ_CUDA_CHECK(cudaStreamSynchronize(gs));
+        for (auto& q : G) {
+            q.gen = q.pos = q.start = 0;
+            q.m = 0;
+            q.done = false;
+            q.head = q.tail = 0;
         }
     }
+    // nonce accounting: 4 nonces per getNext buffer
+    for (int g = 0; g < 3; g++) c.nonce[G01 + g] += 4ull * G[g].start;
 
     // the permutations completed since the last batch, then the runtime's
     // stream waits for the finalize stream

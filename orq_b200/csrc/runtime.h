@@ -113,7 +113,7 @@ struct BatchGraph {
 // Streams, events and pinned state of the permutation generator, created on
 // first use and kept for the runtime's life (creating them per call cost
 // device-wide synchronisation when the pinned buffer was freed).
-constexpr int kFyRingMax = 8;
+constexpr int kFyInFlight = 16;  // batches of scan steps queued per group
 struct FyRes {
     bool ready = false;
     cudaStream_t gs = nullptr;
@@ -121,10 +121,9 @@ struct FyRes {
     cudaStream_t fs = nullptr;  // finalize of completed permutations, during the chain
     cudaEvent_t ev_start = nullptr;
     cudaEvent_t fin_done = nullptr;
-    cudaEvent_t gen_done[kFyRingMax] = {};
-    cudaEvent_t scan_done[3][kFyRingMax] = {};
-    cudaEvent_t st_ev[3][kFyRingMax] = {};
-    void* hst = nullptr;  // pinned scanner states, [ring slot][group]
+    cudaEvent_t gen_done[3][kFyInFlight] = {};
+    cudaEvent_t st_ev[3][kFyInFlight] = {};
+    void* hst = nullptr;  // pinned scan states, [group][batch]
 };
 
 struct Ctx {

@@ -110,6 +110,35 @@ def test_permutations_match_restatement(orq, n, count):
         assert rt.nonce(orq.STREAM_G01 + g) == o.nonce(G01 + g)
 
 
+@pytest.mark.parametrize("n,count", [(32768, 3), (65535, 2), (65536, 4), (131071, 3), (262143, 2), (524288, 2),
+                                     (1048577, 1)])
+def test_permutation_chain_matches_restatement(orq, n, count):
+    """The windowed chain at the smallest size it takes, on both sides of the
+    powers of two where the mask, the runs and the expected draws change, and
+    with windows too narrow for the thresholds (every chain then starts over
+    with wider ones)."""
+    import os
+
+    from oracle.oracle import G01, Oracle
+
+    o = Oracle(5)
+    want = [[o.gen_perm(G01 + g, n)[0] for g in range(3)] for _ in range(count)]
+    for width in (None, "0.25"):
+        if width:
+            os.environ["ORQ_FY_WIDTH"] = width
+        try:
+            rt = orq.Runtime(seed=5)
+            rt.reserve_permutations(n, count)
+        finally:
+            os.environ.pop("ORQ_FY_WIDTH", None)
+        for m in range(count):
+            got = rt.next_permutation(n).cpu().numpy()
+            for g in range(3):
+                assert same(got[g], want[m][g]), (width, m, g)
+        for g in range(3):
+            assert rt.nonce(orq.STREAM_G01 + g) == o.nonce(G01 + g)
+
+
 def test_shuffle_matches_reference(orq, golden, digests):
     m = digests["shuffle_n1000"]["meta"]
     be = GpuBackend(m["shim_seed"])
