@@ -260,6 +260,8 @@ void op_prefix_sum_noalloc(Ctx& c, int w, size_t n, Sh3 s);
 
 // ---- sorting (radix.cu) ----
 void op_radix_sort(Ctx& c, int kw, size_t n, Sh3 key, int bits, bool desc, Sh3 perm_out /*int32*/);
+// the bit loop in one cooperative kernel (rbits.cu)
+void op_radix_bits(Ctx& c, int PW, size_t n, Sh3 P, int bits, bool invert_last);
 // `count` radix sorts whose shares equal `count` op_radix_sort calls in list
 // order, run back to back without host synchronisation between items.
 void op_radix_sort_batch(Ctx& c, int kw, int count, const size_t* n, void* const* keys, const int* bits,
