@@ -138,4 +138,48 @@ __device__ __forceinline__ uint4 keystream_block(const AesSmem& S, const StreamA
     return make_uint4(s0, s1, s2, s3);
 }
 
+// The first two rounds of a chunk's blocks without their constant parts. GCM's
+// counter block is (nonce, 0, BE32(j + 2)): in round 1 counter byte 15 reaches
+// column 0, byte 14 column 1 and byte 13 (1 for the chunk's last two blocks,
+// else 0) column 2, so round 2 is the XOR of two table words a column and a
+// constant of (key, nonce, byte 13). 10 lookups and two broadcast loads in
+// place of 32 lookups: 0.91 of a block's shared-memory cycles.
+struct __align__(16) CtrPre {
+    uint32_t c0, c1, pad0, pad1;  // columns 0 and 1 of round 1 without bytes 15 and 14
+    uint32_t k[4];                // round 2 without columns 0 and 1 of round 1
+};
+
+__device__ __forceinline__ CtrPre ctr_pre(const AesSmem& S, const AesRK& rk, unsigned long long nonce, uint32_t byte13) {
+    const uint32_t w0 = (uint32_t)nonce ^ rk.k[0], w1 = (uint32_t)(nonce >> 32) ^ rk.k[1], w2 = rk.k[2];
+    const uint32_t w3 = (byte13 << 8) ^ rk.k[3];
+    const uint32_t n2 = S.lk<0, 0>(w2) ^ S.lk<1, 1>(w3) ^ S.lk<2, 2>(w0) ^ S.lk<3, 3>(w1) ^ rk.k[6];
+    const uint32_t n3 = S.lk<0, 0>(w3) ^ S.lk<1, 1>(w0) ^ S.lk<2, 2>(w1) ^ S.lk<3, 3>(w2) ^ rk.k[7];
+    CtrPre r;
+    r.c0 = S.lk<0, 0>(w0) ^ S.lk<1, 1>(w1) ^ S.lk<2, 2>(w2) ^ rk.k[4];
+    r.c1 = S.lk<0, 0>(w1) ^ S.lk<1, 1>(w2) ^ S.lk<3, 3>(w0) ^ rk.k[5];
+    r.pad0 = r.pad1 = 0;
+    r.k[0] = S.lk<2, 2>(n2) ^ S.lk<3, 3>(n3) ^ rk.k[8];
+    r.k[1] = S.lk<1, 1>(n2) ^ S.lk<2, 2>(n3) ^ rk.k[9];
+    r.k[2] = S.lk<0, 0>(n2) ^ S.lk<1, 1>(n3) ^ rk.k[10];
+    r.k[3] = S.lk<0, 0>(n3) ^ S.lk<3, 3>(n2) ^ rk.k[11];
+    return r;
+}
+
+// Block j (of 65536) of the chunk whose constants are pre[0] (byte 13 = 0) and
+// pre[1] (byte 13 = 1).
+__device__ __forceinline__ uint4 keystream_block_pre(const AesSmem& S, const AesRK& rk, const CtrPre* pre, uint32_t j) {
+    const uint32_t ctr = j + 2;
+    const CtrPre* q = pre + (ctr >> 16);
+    const uint2 c = *reinterpret_cast<const uint2*>(q);
+    const uint4 k = *reinterpret_cast<const uint4*>(q->k);
+    const uint32_t w3 = __byte_perm(ctr, 0, 0x0123) ^ rk.k[3];
+    const uint32_t n0 = c.x ^ S.lk<3, 3>(w3), n1 = c.y ^ S.lk<2, 2>(w3);
+    uint32_t s0 = k.x ^ S.lk<0, 0>(n0) ^ S.lk<1, 1>(n1);
+    uint32_t s1 = k.y ^ S.lk<0, 0>(n1) ^ S.lk<3, 3>(n0);
+    uint32_t s2 = k.z ^ S.lk<2, 2>(n0) ^ S.lk<3, 3>(n1);
+    uint32_t s3 = k.w ^ S.lk<1, 1>(n0) ^ S.lk<2, 2>(n1);
+    aes256_rounds_from<3>(S, rk, s0, s1, s2, s3);
+    return make_uint4(s0, s1, s2, s3);
+}
+
 }  // namespace orqcu

@@ -327,6 +327,110 @@ __global__ void __launch_bounds__(cmp_threads<sizeof(T)>(), 1) k_cmp(CmpArgs<T> 
         cmp_tile<T, MODE>(a, a.pair, nonce, base, S, sm + kAesSmemBytes / 4, ksp, ballots);
 }
 
+// ---- _compare of 16-byte shares (padded int64 keys; quicksort's compares) ----
+// A keystream block is one pair's word here, so a lane computes the blocks of
+// its own pair call by call: nothing is staged through shared memory, and 16
+// warps run where the staged circuit had room for 8. Four warps (128 pairs)
+// make a packed word and meet at a barrier of their own; a CTA works on one
+// contiguous range, so the constant parts of rounds 1 and 2 (CtrPre) are built
+// once per 65536 pairs. Bound by the T-table lookups. Quicksort of 2^22 rows:
+// its 56 compares took 94 ms staged and take 79.6 ms.
+constexpr int kCmp16Threads = 512;
+constexpr int kCmp16Calls = cmp_levels<16>() + 1;
+
+__global__ void __launch_bounds__(kCmp16Threads, 1) k_cmp16(CmpArgs<u128> a) {
+    constexpr int L = cmp_levels<16>();
+    extern __shared__ __align__(16) uint32_t sm[];
+    __shared__ CtrPre pre[2][kCmp16Calls][3][2];  // [chunk - first][call][stream][byte 13]
+    __shared__ uint32_t ballots[2][kCmp16Threads / 32][3][3];
+    __shared__ uint4 kp[2][kCmp16Threads / 128][3];  // keystream of the packed AND
+    aes_stage_tables(sm);
+    const AesSmem S(sm);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gr = w >> 2;
+    const unsigned long long units = ceil_div(a.m, 128);
+    const unsigned long long u0 = units * blockIdx.x / gridDim.x, u1 = units * (blockIdx.x + 1) / gridDim.x;
+    int flip = 0;
+    for (unsigned long long s0 = u0; s0 < u1; s0 += 512) {  // spans of 65536 pairs: at most two chunks
+        const unsigned long long s1 = min(u1, s0 + 512), chunk0 = (s0 * 128) >> 16;
+        __syncthreads();  // the span before has read its constants
+        for (int i = threadIdx.x; i < 2 * kCmp16Calls * 3 * 2; i += kCmp16Threads) {
+            const int b13 = i & 1, q = (i >> 1) % 3, call = (i / 6) % kCmp16Calls, ch = i / (6 * kCmp16Calls);
+            pre[ch][call][q][b13] =
+                ctr_pre(S, a.pair[q].rk, a.pair[q].nonce + (unsigned long long)call * a.C + chunk0 + ch, (uint32_t)b13);
+        }
+        __syncthreads();
+        for (unsigned long long u = s0 + gr; u < s1; u += kCmp16Threads / 128, flip ^= 1) {
+            const unsigned long long p = u * 128 + (w & 3) * 32 + lane;
+            const bool valid = p < a.m;
+            u128 A[3] = {0, 0, 0}, Bv[3] = {0, 0, 0};
+            if (valid)
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    A[j] = Ring<16>::w(__ldg(reinterpret_cast<const uint4*>(a.x[j]) + p));
+                    Bv[j] = Ring<16>::w(__ldg(reinterpret_cast<const uint4*>(a.y[j]) + p));
+                }
+            const uint32_t ch = (uint32_t)((p >> 16) - chunk0), jb = (uint32_t)p & 0xffffu;
+            u128 Sm[3], G[3];
+#pragma unroll
+            for (int j = 0; j < 3; j++) Sm[j] = ~(A[j] ^ Bv[j]);
+            // rolled: three AES bodies stay inside the instruction cache
+#pragma unroll 1
+            for (int call = 0; call <= L; call++) {
+                u128 K[3], X[3], Y[3];
+#pragma unroll
+                for (int q = 0; q < 3; q++) K[q] = Ring<16>::w(keystream_block_pre(S, a.pair[q].rk, pre[ch][call][q], jb));
+                const int sh = call < L ? 1 << call : 1;
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    const u128 t = ashr(Sm[j], sh);
+                    X[j] = call < L ? Sm[j] : t ^ Sm[j];
+                    Y[j] = call < L ? t : A[j];
+                }
+                and3(X, Y, K, G);
+                if (call < L)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) Sm[j] = G[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const uint32_t b1 = __ballot_sync(0xffffffffu, valid && ((A[j] >> 127) & 1));
+                const uint32_t b2 = __ballot_sync(0xffffffffu, valid && ((Bv[j] >> 127) & 1));
+                const uint32_t br = __ballot_sync(0xffffffffu, valid && parity(G[j]));
+                if (lane == 0) {
+                    ballots[flip][w][0][j] = b1;
+                    ballots[flip][w][1][j] = b2;
+                    ballots[flip][w][2][j] = br;
+                }
+            }
+            if ((w & 3) == 0 && lane < 3) {
+                const unsigned long long nl =
+                    lane == 0 ? a.pair[0].nonce : (lane == 1 ? a.pair[1].nonce : a.pair[2].nonce);
+                kp[flip][gr][lane] = keystream_block_n(S, a.pair[lane].rk, nl + (unsigned long long)(L + 1) * a.C, u);
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + gr) : "memory");
+            // sign fix-up on this warp's 32 bits of the packed word (bitwise, so
+            // the words of the other warps do not matter): r ^= s2; s2 ^= s1;
+            // s2 = ~(~s2 & ~r); s1 ^= s2
+            uint32_t s1[3], ns2[3], nr[3], K[3], Z[3];
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                s1[j] = ballots[flip][w][0][j];
+                const uint32_t s2 = ballots[flip][w][1][j];
+                ns2[j] = ~(s2 ^ s1[j]);
+                nr[j] = ~(ballots[flip][w][2][j] ^ s2);
+                K[j] = reinterpret_cast<const uint32_t*>(&kp[flip][gr][j])[w & 3];
+            }
+            and3(ns2, nr, K, Z);
+            if (valid)
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    a.eq[j][p] = Sm[j] & 1;
+                    a.gt[j][p] = ((s1[j] ^ ~Z[j]) >> lane) & 1;
+                }
+        }
+    }
+}
+
 // ---- compare_rows and swap over several columns -------------------------------
 // compare_rows (operators/sorting.h:80-108) runs _compare on every key column,
 // in order, and folds key k >= 1 in with two ANDs: gt ^= new_gt & eq, then
@@ -709,6 +813,15 @@ void launch_cmp(Ctx& c, const CmpArgs<T>& a, const char* name) {
     c.kernels_launched++;
 }
 
+void launch_cmp16(Ctx& c, const CmpArgs<u128>& a) {
+    prep_aes_kernel(k_cmp16);
+    const unsigned grid = (unsigned)std::min<unsigned long long>(ceil_div(a.m, 128), (unsigned long long)c.num_sms);
+    ProfScope ps(c, "compare", 12.0 * 16 * a.m, kCmp16Calls * 3.0 * a.m + 3.0 * ceil_div(a.m, 128));
+    k_cmp16<<<grid, kCmp16Threads, kAesSmemBytes, c.stream>>>(a);
+    ORQ_CUDA_CHECK(cudaGetLastError());
+    c.kernels_launched++;
+}
+
 template <typename T>
 void compare_t(Ctx& c, size_t n, CSh3 x, CSh3 y, Sh3 eq, Sh3 gt) {
     constexpr int W = sizeof(T);
@@ -724,7 +837,12 @@ void compare_t(Ctx& c, size_t n, CSh3 x, CSh3 y, Sh3 eq, Sh3 gt) {
     a.C = chunks_of((unsigned long long)n * W);
     a.Cp = chunks_of(ceil_div(n, 8 * W) * W);
     a.m = n;
-    if (n) launch_cmp<T, 1>(c, a, "compare");
+    if constexpr (W == 16) {
+        if (n)
+            launch_cmp16(c, a);
+    } else if (n) {
+        launch_cmp<T, 1>(c, a, "compare");
+    }
     for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += (unsigned long long)(L + 1) * a.C + a.Cp;
 }
 
