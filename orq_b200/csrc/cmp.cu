@@ -50,6 +50,11 @@ struct CmpArgs {
     int hs;                    // bitonic half-box size h = 2^hs
     int first;                 // bitonic stage j == 0 (reversed partner)
     int desc;
+    // quicksort's compare: pair p is (key[idx[p]], key[head[idx[p]]]), and only
+    // the opened gt bit is kept, at cb[idx[p]]
+    const uint32_t* idx;
+    const int32_t* head;
+    uint8_t* cb;
 };
 
 template <typename T>
@@ -186,8 +191,8 @@ __device__ __forceinline__ void gt_bits3(const T (&A)[3], const T (&Bv)[3], cons
     for (int j = 0; j < 3; j++) gt[j] = (s1[j] >> bitpos) & 1;
 }
 
-// One CTA tile of a bitonic stage (MODE 0) or of a compare (MODE 1): the
-// pairs [base, base + blockDim.x).
+// One CTA tile of a bitonic stage (MODE 0), a compare (MODE 1), an equality
+// (MODE 2) or quicksort's compare (MODE 3): the pairs [base, base + blockDim.x).
 template <typename T, int MODE>
 __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&pairs)[3],
                                          const unsigned long long (&nonce)[3], unsigned long long base,
@@ -196,7 +201,7 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
     constexpr int W = sizeof(T);
     constexpr int B = 8 * W;               // pairs per packed word
     constexpr int L = cmp_levels<W>();     // bit_same rounds
-    constexpr int NFULL = MODE == 0 ? L + 3 : (MODE == 1 ? L + 1 : L);
+    constexpr int NFULL = MODE == 0 ? L + 3 : (MODE == 2 ? L : L + 1);
     constexpr int WORDS = 32 * W / 4;      // keystream words per call and stream per warp
     constexpr int NB = 32 * W / 16;        // AES blocks per call and stream per warp
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -212,11 +217,15 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
             xi = (cb << (a.hs + 1)) + k;
             yi = a.first ? (cb << (a.hs + 1)) + 2 * h - 1 - k : (cb << (a.hs + 1)) + h + k;
         }
+        if (MODE == 3 && valid) {
+            xi = a.idx[p];
+            yi = (unsigned long long)a.head[xi];
+        }
         T X[3] = {0, 0, 0}, Y[3] = {0, 0, 0};
         if (valid) {
 #pragma unroll
             for (int j = 0; j < 3; j++) {
-                if (MODE == 0) {
+                if (MODE == 0 || MODE == 3) {
                     X[j] = a.key[j][xi];
                     Y[j] = a.key[j][yi];
                 } else {
@@ -285,6 +294,8 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
                     a.eq[j][p] = eq[j];
                     a.gt[j][p] = gt[j];
                 }
+        } else if (MODE == 3) {
+            if (valid) a.cb[xi] = (uint8_t)((gt[0] ^ gt[1] ^ gt[2]) & 1);
         } else {
             // swap: x' = x ^ (ext(b) & (y ^ x)), y' = y ^ (ext(b) & (x ^ y))
             T E[3], D[3], K[3], Z[3];
@@ -313,7 +324,7 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
     }
 }
 
-template <typename T, int MODE>  // MODE 0: bitonic stage, MODE 1: compare
+template <typename T, int MODE>  // as cmp_tile
 __global__ void __launch_bounds__(cmp_threads<sizeof(T)>(), 1) k_cmp(CmpArgs<T> a) {
     constexpr int kCmpThreads = cmp_threads<sizeof(T)>();
     extern __shared__ __align__(16) uint32_t sm[];
@@ -338,6 +349,7 @@ __global__ void __launch_bounds__(cmp_threads<sizeof(T)>(), 1) k_cmp(CmpArgs<T> 
 constexpr int kCmp16Threads = 512;
 constexpr int kCmp16Calls = cmp_levels<16>() + 1;
 
+template <bool QS>  // quicksort's compare
 __global__ void __launch_bounds__(kCmp16Threads, 1) k_cmp16(CmpArgs<u128> a) {
     constexpr int L = cmp_levels<16>();
     extern __shared__ __align__(16) uint32_t sm[];
@@ -363,11 +375,16 @@ __global__ void __launch_bounds__(kCmp16Threads, 1) k_cmp16(CmpArgs<u128> a) {
             const unsigned long long p = u * 128 + (w & 3) * 32 + lane;
             const bool valid = p < a.m;
             u128 A[3] = {0, 0, 0}, Bv[3] = {0, 0, 0};
+            unsigned long long xi = p, yi = p;
+            if (QS && valid) {
+                xi = a.idx[p];
+                yi = (unsigned long long)a.head[xi];
+            }
             if (valid)
 #pragma unroll
                 for (int j = 0; j < 3; j++) {
-                    A[j] = Ring<16>::w(__ldg(reinterpret_cast<const uint4*>(a.x[j]) + p));
-                    Bv[j] = Ring<16>::w(__ldg(reinterpret_cast<const uint4*>(a.y[j]) + p));
+                    A[j] = Ring<16>::w(__ldg(reinterpret_cast<const uint4*>(QS ? a.key[j] : a.x[j]) + xi));
+                    Bv[j] = Ring<16>::w(__ldg(reinterpret_cast<const uint4*>(QS ? a.key[j] : a.y[j]) + yi));
                 }
             const uint32_t ch = (uint32_t)((p >> 16) - chunk0), jb = (uint32_t)p & 0xffffu;
             u128 Sm[3], G[3];
@@ -421,12 +438,15 @@ __global__ void __launch_bounds__(kCmp16Threads, 1) k_cmp16(CmpArgs<u128> a) {
                 K[j] = reinterpret_cast<const uint32_t*>(&kp[flip][gr][j])[w & 3];
             }
             and3(ns2, nr, K, Z);
-            if (valid)
+            if (QS) {
+                if (valid) a.cb[xi] = (uint8_t)(((s1[0] ^ s1[1] ^ s1[2] ^ ~(Z[0] ^ Z[1] ^ Z[2])) >> lane) & 1);
+            } else if (valid) {
 #pragma unroll
                 for (int j = 0; j < 3; j++) {
                     a.eq[j][p] = Sm[j] & 1;
                     a.gt[j][p] = ((s1[j] ^ ~Z[j]) >> lane) & 1;
                 }
+            }
         }
     }
 }
@@ -791,7 +811,7 @@ template <typename T, int MODE>
 void launch_cmp(Ctx& c, const CmpArgs<T>& a, const char* name) {
     constexpr int W = sizeof(T);
     constexpr int L = cmp_levels<W>();
-    constexpr int NFULL = MODE == 0 ? L + 3 : (MODE == 1 ? L + 1 : L);
+    constexpr int NFULL = MODE == 0 ? L + 3 : (MODE == 2 ? L : L + 1);
     constexpr int kCmpThreads = cmp_threads<W>();
     // spread small stages over every SM: threads per CTA a multiple of 64
     // (whole packed words for both widths) up to the maximum
@@ -813,11 +833,12 @@ void launch_cmp(Ctx& c, const CmpArgs<T>& a, const char* name) {
     c.kernels_launched++;
 }
 
+template <bool QS>
 void launch_cmp16(Ctx& c, const CmpArgs<u128>& a) {
-    prep_aes_kernel(k_cmp16);
+    prep_aes_kernel(k_cmp16<QS>);
     const unsigned grid = (unsigned)std::min<unsigned long long>(ceil_div(a.m, 128), (unsigned long long)c.num_sms);
     ProfScope ps(c, "compare", 12.0 * 16 * a.m, kCmp16Calls * 3.0 * a.m + 3.0 * ceil_div(a.m, 128));
-    k_cmp16<<<grid, kCmp16Threads, kAesSmemBytes, c.stream>>>(a);
+    k_cmp16<QS><<<grid, kCmp16Threads, kAesSmemBytes, c.stream>>>(a);
     ORQ_CUDA_CHECK(cudaGetLastError());
     c.kernels_launched++;
 }
@@ -839,9 +860,35 @@ void compare_t(Ctx& c, size_t n, CSh3 x, CSh3 y, Sh3 eq, Sh3 gt) {
     a.m = n;
     if constexpr (W == 16) {
         if (n)
-            launch_cmp16(c, a);
+            launch_cmp16<false>(c, a);
     } else if (n) {
         launch_cmp<T, 1>(c, a, "compare");
+    }
+    for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += (unsigned long long)(L + 1) * a.C + a.Cp;
+}
+
+// quicksort's compare of the rows idx[0..n) with their segments' heads
+// (quicksort.h:120-150): _compare's calls on the gathered rows, of which only
+// the opened gt bits are written. The gathered copies, the eq and gt shares
+// and the opened column that separate steps pass on are 400 bytes a row.
+template <typename T>
+void qs_compare_t(Ctx& c, size_t n, CSh3 rows, const uint32_t* idx, const int32_t* head, uint8_t* cb) {
+    constexpr int W = sizeof(T);
+    constexpr int L = cmp_levels<W>();
+    CmpArgs<T> a{};
+    for (int j = 0; j < 3; j++) {
+        a.key[j] = (T*)rows.p[j];
+        a.pair[j] = c.stream_arg(PAIR0 + j);
+    }
+    a.idx = idx;
+    a.head = head;
+    a.cb = cb;
+    a.C = chunks_of((unsigned long long)n * W);
+    a.Cp = chunks_of(ceil_div(n, 8 * W) * W);
+    a.m = n;
+    if (n) {
+        if constexpr (W == 16) launch_cmp16<true>(c, a);
+        else launch_cmp<T, 3>(c, a, "compare");
     }
     for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += (unsigned long long)(L + 1) * a.C + a.Cp;
 }
@@ -1317,6 +1364,11 @@ void op_compare(Ctx& c, int w, size_t n, CSh3 x, CSh3 y, Sh3 eq, Sh3 gt) {
     else throw std::invalid_argument("compare supports 4, 8 and 16-byte keys");
 }
 
+void op_qs_compare(Ctx& c, int w, size_t n, CSh3 rows, const uint32_t* idx, const int32_t* head, uint8_t* cb) {
+    if (w == 16) qs_compare_t<unsigned __int128>(c, n, rows, idx, head, cb);
+    else if (w == 8) qs_compare_t<unsigned long long>(c, n, rows, idx, head, cb);
+    else throw std::invalid_argument("quicksort rows are 8 or 16 bytes");
+}
 void op_equal(Ctx& c, int w, size_t n, CSh3 x, CSh3 y, Sh3 eq) {
     if (w == 4) equal_t<uint32_t>(c, n, x, y, eq);
     else if (w == 8) equal_t<unsigned long long>(c, n, x, y, eq);

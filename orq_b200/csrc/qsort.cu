@@ -202,27 +202,6 @@ __global__ void __launch_bounds__(kQsThreads) k_qs_zeros(QsRound a) {
     }
 }
 
-// rows compared this round: row idx[k] and the pivot heading its segment
-template <int PW>
-__global__ void k_qs_gather(QsRound a, CSh3 P, Sh3 R, Sh3 PV, uint32_t size) {
-    using V = typename std::conditional<PW == 16, uint4, unsigned long long>::type;
-    for (unsigned long long k = gtid(); k < size; k += gstride()) {
-        const uint32_t q = a.idx[k];
-        const uint32_t h = (uint32_t)a.head[q];
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            reinterpret_cast<V*>(R.p[j])[k] = reinterpret_cast<const V*>(P.p[j])[q];
-            reinterpret_cast<V*>(PV.p[j])[k] = reinterpret_cast<const V*>(P.p[j])[h];
-        }
-    }
-}
-
-// the opened comparison bit (LSB of the opened value) at its row's position
-template <int PW>
-__global__ void k_qs_bits(QsRound a, const uint8_t* opened, uint32_t size) {
-    for (unsigned long long k = gtid(); k < size; k += gstride()) a.cb[a.idx[k]] = opened[k * PW] & 1u;
-}
-
 // segment totals at the heads, and each zero's position by rank
 __global__ void k_qs_seg(QsRound a) {
     for (unsigned long long q = gtid(); q < a.n; q += gstride()) {
@@ -278,8 +257,7 @@ void quicksort_rounds(Ctx& c, size_t n, Sh3 P) {
     const uint32_t chunks = (uint32_t)ceil_div(n, (size_t)kQsChunk);
     Scratch pivb(c, n * 4), headb(c, n * 4), idxb(c, n * 4), cbb(c, n), gzb(c, n * 4), zsegb(c, n * 4),
         sendb(c, n * 4), zposb(c, n * 4), psb(c, chunks * 4), pmb(c, chunks * 4), npb(c, 4);
-    Scratch npbuf(c, 3 * n * PW), rbuf(c, 3 * n * PW), pvbuf(c, 3 * n * PW), ebuf(c, 3 * n * PW),
-        gbuf(c, 3 * n * PW), obuf(c, n * PW);
+    Scratch npbuf(c, 3 * n * PW);
     QsRound a;
     a.n = (uint32_t)n;
     a.chunks = chunks;
@@ -311,29 +289,25 @@ void quicksort_rounds(Ctx& c, size_t n, Sh3 P) {
     for (size_t round = 0; num_pivots < n; round++) {
         if (round > 4 * n + 64) throw std::runtime_error("quicksort did not converge");
         const uint32_t size = (uint32_t)(n - num_pivots);
-        Sh3 R = split(rbuf, size), PV = split(pvbuf, size), E = split(ebuf, size), G = split(gbuf, size);
         {
             ProfScope ps(c, "quicksort_round", 0.0);
             k_qs_part<0><<<chunks, kQsThreads, 0, c.stream>>>(a);
             k_qs_top<<<1, kQsThreads, 0, c.stream>>>(a);
             k_qs_heads<<<chunks, kQsThreads, 0, c.stream>>>(a);
-            k_qs_gather<PW><<<plain_grid(c, size), 256, 0, c.stream>>>(a, cc(cur), R, PV, size);
             ORQ_CUDA_CHECK(cudaGetLastError());
-            c.kernels_launched += 4;
+            c.kernels_launched += 3;
         }
         // reduced._compare(pivot): gt = row > pivot, opened
-        op_compare(c, PW, size, cc(R), cc(PV), E, G);
-        op_open(c, false, PW, size, cc(G), obuf.p);
+        op_qs_compare(c, PW, size, cc(cur), a.idx, a.head, a.cb);
         {
             ProfScope ps(c, "quicksort_round", 0.0);
-            k_qs_bits<PW><<<plain_grid(c, size), 256, 0, c.stream>>>(a, obuf.as<uint8_t>(), size);
             k_qs_part<1><<<chunks, kQsThreads, 0, c.stream>>>(a);
             k_qs_top<<<1, kQsThreads, 0, c.stream>>>(a);
             k_qs_zeros<<<chunks, kQsThreads, 0, c.stream>>>(a);
             k_qs_seg<<<gg, 256, 0, c.stream>>>(a);
             k_qs_move<PW><<<gg, 256, 0, c.stream>>>(a, cc(cur), nxt);
             ORQ_CUDA_CHECK(cudaGetLastError());
-            c.kernels_launched += 6;
+            c.kernels_launched += 5;
         }
         std::swap(cur, nxt);
         ORQ_CUDA_CHECK(cudaMemcpyAsync(&num_pivots, a.npiv, 4, cudaMemcpyDeviceToHost, c.stream));
