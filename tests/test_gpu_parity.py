@@ -813,6 +813,19 @@ def test_a2b_matches_restatement(orq, w, n):
     assert np.array_equal(gpu["open_xb"][0].view(x.dtype), x)
 
 
+@pytest.mark.parametrize("w,n", [(4, 32), (4, 1023), (4, 1025), (4, 2048), (8, 1024), (8, 1025),
+                                 (4, 148 * 1024 + 1), (8, 8 * 148 * 1024 + 33), (4, (1 << 23) + 1025)])
+def test_boolean_add_matches_restatement_at_tile_edges(orq, w, n):
+    """The adder's tiles are 1024 elements, a CTA with one tile shares its
+    keystream work, and a keystream chunk ends after 2^23 elements."""
+    from replay import replay_a2b
+
+    got, _ = replay_a2b(GpuBackend(3), n, 7, w)
+    want, _ = replay_a2b(OracleBackend(3), n, 7, w)
+    for name in want:
+        assert same(got[name], want[name]), name
+
+
 @pytest.mark.parametrize("tag,w", [("badd32_n500", 4), ("badd64_n333", 8)])
 def test_boolean_add_sub_match_reference_shares(orq, golden, digests, tag, w):
     """BSharedVector + and - (the ripple-carry adder), share for share"""
