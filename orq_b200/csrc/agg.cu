@@ -25,7 +25,12 @@ constexpr int kMaxAggKeys = 4;
 // arithmetic, with and without the table restriction) across the level's
 // calls, so it needs up to 255 registers: 256 threads per CTA, one CTA per SM
 // (the AES tables take 128 KiB of shared memory).
-constexpr int kAggThreads = 256;
+// Threads per CTA: the compare circuit of min / max needs 200 registers, a
+// level without one fits 128. Smaller CTAs while that spreads a level over
+// more SMs.
+template <bool MINMAX>
+constexpr int agg_threads() { return MINMAX ? 256 : 512; }
+constexpr int kAggSmall = 256;
 constexpr int kMaxAggSpecs = 8;
 
 struct AggLevelArgs {
@@ -197,7 +202,7 @@ __device__ __forceinline__ void compare_rows(const T (&X)[E][3], const T (&Y)[E]
 // MINMAX: whether the level has a min or max aggregation; without one the
 // compare circuit is compiled out (it holds most of the registers)
 template <int W, bool MINMAX>
-__global__ void __launch_bounds__(kAggThreads, 1) k_agg_level(AggLevelArgs a) {
+__global__ void __launch_bounds__(agg_threads<MINMAX>(), 1) k_agg_level(AggLevelArgs a) {
     using T = typename std::conditional<W == 4, uint32_t, unsigned long long>::type;
     constexpr int E = 16 / W;               // rows per unit
     constexpr int L = (W == 4) ? 5 : 6;     // bit_same rounds
@@ -210,22 +215,29 @@ __global__ void __launch_bounds__(kAggThreads, 1) k_agg_level(AggLevelArgs a) {
     for (unsigned long long wb = gtid() - lane; wb < units; wb += gstride()) {
         const unsigned long long u = wb + lane;
         unsigned long long off = 0;  // nonces consumed by the level's calls so far
-        T K[E][3];
+        T K[E][3] = {};
         // keystream of the next protocol call for this unit, split per row
+        // (the stream loop stays rolled: inlined at every call of the level,
+        // three AES bodies each overflowed the instruction cache, 19.2 ms for the
+        // levels of a join of 2^16 and 2^18 rows, 14.0 now; each pass
+        // appends stream q and moves the others down, so K[.][q] ends up in place)
         auto next_call = [&]() {
-#pragma unroll
+#pragma unroll 1
             for (int q = 0; q < 3; q++) {
-                StreamArg st = a.pair[q];
-                st.nonce += off;
-                const uint4 b = keystream_block(S, st, u);
+                const uint4 b = keystream_block_n(S, a.pair[q].rk, a.pair[q].nonce + off, u);
+#pragma unroll
+                for (int k = 0; k < E; k++) {
+                    K[k][0] = K[k][1];
+                    K[k][1] = K[k][2];
+                }
                 if constexpr (W == 4) {
-                    K[0][q] = b.x;
-                    K[1][q] = b.y;
-                    K[2][q] = b.z;
-                    K[3][q] = b.w;
+                    K[0][2] = b.x;
+                    K[1][2] = b.y;
+                    K[2][2] = b.z;
+                    K[3][2] = b.w;
                 } else {
-                    K[0][q] = (T)b.x | ((T)b.y << 32);
-                    K[1][q] = (T)b.z | ((T)b.w << 32);
+                    K[0][2] = (T)b.x | ((T)b.y << 32);
+                    K[1][2] = (T)b.z | ((T)b.w << 32);
                 }
             }
             off += a.C;
@@ -619,9 +631,10 @@ void op_aggregate(Ctx& c, int w, size_t n, int nkeys, const void* const* keys, i
             auto kern = w == 4 ? (minmax ? k_agg_level<4, true> : k_agg_level<4, false>)
                                : (minmax ? k_agg_level<8, true> : k_agg_level<8, false>);
             prep_aes_kernel(kern);
-            const unsigned grid = (unsigned)std::min<unsigned long long>(ceil_div(units, kAggThreads), (unsigned long long)c.num_sms);
+            const int nt = minmax || units <= (unsigned long long)c.num_sms * kAggSmall ? kAggSmall : agg_threads<false>();
+            const unsigned grid = (unsigned)std::min<unsigned long long>(ceil_div(units, nt), (unsigned long long)c.num_sms);
             ProfScope ps(c, "agg_level", bytes, 3.0 * calls * units + 3.0 * packed * units);
-            kern<<<grid, kAggThreads, kAesSmemBytes, c.stream>>>(a);
+            kern<<<grid, nt, kAesSmemBytes, c.stream>>>(a);
             ORQ_CUDA_CHECK(cudaGetLastError());
             c.kernels_launched++;
         }
