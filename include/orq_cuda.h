@@ -316,17 +316,17 @@ int orqcu_distinct(orqcu_runtime* rt, int width, size_t n, int nkeys, const void
 /* Batched bitonic_sort: `count` independent B-shared key columns of
  * power-of-two sizes n[i] (keys[3*i+p]), each ascending or descending. The
  * shares produced are exactly those of `count` orqcu_bitonic_sort calls in
- * list order. Execution is batched: one persistent launch per network round
- * walks a ragged work list of every column that still has a stage, the
- * threads per CTA are autotuned once per size class, and with use_graph the
- * rounds are captured once per batch shape into a CUDA graph that later calls
- * replay. No reference counterpart: ORQ sorts one vector per call. */
+ * list order. Execution is batched: one cooperative launch walks, network
+ * round by network round, the tiles of every column that still has a stage.
+ * use_graph is accepted for source compatibility and has no effect: there is
+ * one launch either way. No reference counterpart: ORQ sorts one vector per
+ * call. */
 int orqcu_bitonic_sort_batch(orqcu_runtime* rt, int width, int count, const size_t* n,
                              void* const* keys, const int* descending, int use_graph);
 
 /* Re-key the runtime as orqcu_runtime_create(seed) would (fresh keys, nonces
  * at zero, reserved permutations dropped) while keeping its stream, its
- * cached device memory, tuned launch shapes and captured graphs. A serving
+ * cached device memory. A serving
  * slot runs each request on its own seed this way, so a request's shares do
  * not depend on what ran before it. No reference counterpart (one
  * orq_init per process there). */

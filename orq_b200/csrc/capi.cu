@@ -318,7 +318,7 @@ int orqcu_runtime_destroy(orqcu_runtime* rt) {
         cudaStreamSynchronize(rt->ctx.stream);
         for (auto& sp : rt->ctx.perm_queue) rt->ctx.free_perm(sp);
         rt->ctx.perm_queue.clear();
-        rt->ctx.release_graphs();
+        rt->ctx.release_batch();
         orqcu::release_fy(rt->ctx);
         if (rt->ctx.owns_stream) cudaStreamDestroy(rt->ctx.stream);
         if (rt->ctx.d_err) cudaFree(rt->ctx.d_err);
@@ -776,7 +776,8 @@ int orqcu_bitonic_sort_batch(orqcu_runtime* rt, int width, int count, const size
             need_sh((const void* const*)keys + 3 * i, n[i], "null key share");
             k[i] = m3(keys + 3 * i);
         }
-        orqcu::op_bitonic_sort_batch(rt->ctx, width, count, n, k.data(), descending, use_graph != 0);
+        (void)use_graph;  // one launch either way
+        orqcu::op_bitonic_sort_batch(rt->ctx, width, count, n, k.data(), descending);
     });
 }
 

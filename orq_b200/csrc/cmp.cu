@@ -13,6 +13,7 @@
 // zero-sharing keystream of all its rounds into shared memory (every AES block
 // once), then each thread runs the circuit in registers. The packed fix-up
 // (a bit transpose of 8W consecutive pairs) is a warp ballot.
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <type_traits>
@@ -39,17 +40,14 @@ constexpr int cmp_levels() { return W == 4 ? 5 : (W == 8 ? 6 : 7); }
 
 template <typename T>
 struct CmpArgs {
-    T* key[3];          // bitonic: the sorted column (in place)
+    const T* key[3];    // quicksort: the rows
     const T* x[3];      // compare: this
     const T* y[3];      // compare: other
     T* eq[3];
     T* gt[3];
-    StreamArg pair[3];  // nonces at the start of the stage / compare
+    StreamArg pair[3];  // nonces at the start of the compare
     unsigned long long C, Cp;  // nonces per full-size and per packed AND call
     unsigned long long m;      // pairs
-    int hs;                    // bitonic half-box size h = 2^hs
-    int first;                 // bitonic stage j == 0 (reversed partner)
-    int desc;
     // quicksort's compare: pair p is (key[idx[p]], key[head[idx[p]]]), and only
     // the opened gt bit is kept, at cb[idx[p]]
     const uint32_t* idx;
@@ -108,8 +106,8 @@ __device__ __forceinline__ void bit_same3(const T (&A)[3], const T (&Bv)[3], con
 // parity(((eq >> 1) ^ eq) & this) on keystream call L, then the signed fix-up
 // on words of 8W packed pairs with one packed AND whose keystream block is kp
 // (this warp's [stream][word]). A warp holds pairs [p0w, p0w + 32); for 8-byte
-// shares two warps make one packed word, exchanged through `ballots` (every
-// thread of the CTA must call this). Returns the masked gt bit of the pair.
+// shares two warps make one packed word, exchanged through `ballots` (all of
+// a word's warps must call this). Returns the masked gt bit of the pair.
 template <typename T, typename KW>
 __device__ __forceinline__ void gt_bits3(const T (&A)[3], const T (&Bv)[3], const T (&Sm)[3], bool valid,
                                          unsigned long long p, unsigned long long p0w, int warp,
@@ -147,7 +145,9 @@ __device__ __forceinline__ void gt_bits3(const T (&A)[3], const T (&Bv)[3], cons
         // W / 4 warps per packed word of 8W pairs
         constexpr int WPW = W / 4;
         const int lane = threadIdx.x & 31;
-        __syncthreads();
+        // a barrier of the word's own warps (every warp of the CTA gets here)
+        const auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / WPW), "n"(32 * WPW) : "memory"); };
+        meet();
         if (lane == 0)
 #pragma unroll
             for (int j = 0; j < 3; j++) {
@@ -155,7 +155,7 @@ __device__ __forceinline__ void gt_bits3(const T (&A)[3], const T (&Bv)[3], cons
                 ballots[warp][1][j] = b2[j];
                 ballots[warp][2][j] = br[j];
             }
-        __syncthreads();
+        meet();
         const int w0 = warp & ~(WPW - 1);
 #pragma unroll
         for (int j = 0; j < 3; j++) {
@@ -191,8 +191,8 @@ __device__ __forceinline__ void gt_bits3(const T (&A)[3], const T (&Bv)[3], cons
     for (int j = 0; j < 3; j++) gt[j] = (s1[j] >> bitpos) & 1;
 }
 
-// One CTA tile of a bitonic stage (MODE 0), a compare (MODE 1), an equality
-// (MODE 2) or quicksort's compare (MODE 3): the pairs [base, base + blockDim.x).
+// One CTA tile of a compare (MODE 1), an equality (MODE 2) or quicksort's
+// compare (MODE 3): the pairs [base, base + blockDim.x).
 template <typename T, int MODE>
 __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&pairs)[3],
                                          const unsigned long long (&nonce)[3], unsigned long long base,
@@ -201,7 +201,7 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
     constexpr int W = sizeof(T);
     constexpr int B = 8 * W;               // pairs per packed word
     constexpr int L = cmp_levels<W>();     // bit_same rounds
-    constexpr int NFULL = MODE == 0 ? L + 3 : (MODE == 2 ? L : L + 1);
+    constexpr int NFULL = MODE == 2 ? L : L + 1;
     constexpr int WORDS = 32 * W / 4;      // keystream words per call and stream per warp
     constexpr int NB = 32 * W / 16;        // AES blocks per call and stream per warp
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -212,11 +212,6 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
         const bool valid = p < a.m;
         // ---- operands, loaded first so their latency hides under the AES work
         unsigned long long xi = p, yi = p;
-        if (MODE == 0) {
-            const unsigned long long h = 1ull << a.hs, cb = p >> a.hs, k = p & (h - 1);
-            xi = (cb << (a.hs + 1)) + k;
-            yi = a.first ? (cb << (a.hs + 1)) + 2 * h - 1 - k : (cb << (a.hs + 1)) + h + k;
-        }
         if (MODE == 3 && valid) {
             xi = a.idx[p];
             yi = (unsigned long long)a.head[xi];
@@ -225,7 +220,7 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
         if (valid) {
 #pragma unroll
             for (int j = 0; j < 3; j++) {
-                if (MODE == 0 || MODE == 3) {
+                if (MODE == 3) {
                     X[j] = a.key[j][xi];
                     Y[j] = a.key[j][yi];
                 } else {
@@ -234,37 +229,20 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
                 }
             }
         }
-        // ---- keystream of every round, each AES block once per warp
-        for (int idx = lane; idx < NFULL * 3 * NB; idx += 32) {
-            const int call = idx / (3 * NB), q = (idx / NB) % 3, b = idx % NB;
-            unsigned long long off = (unsigned long long)call * a.C;
-            if (call > L) off = (unsigned long long)(L + 1) * a.C + a.Cp + (unsigned long long)(call - L - 1) * a.C;
-            const uint4 ks = keystream_block_n(S, pairs[q].rk, nonce[q] + off, p0w * W / 16 + b);
-            uint32_t* o = myks + (call * 3 + q) * WORDS + b * 4;
-            o[0] = ks.x;
-            o[1] = ks.y;
-            o[2] = ks.z;
-            o[3] = ks.w;
-        }
-        if (MODE != 2 && lane < 3) {
-            // the packed AND: word c = pair / B covers pairs [cB, cB+B)
-            const unsigned long long c = p0w / B;
-            const unsigned long long nl = lane == 0 ? nonce[0] : (lane == 1 ? nonce[1] : nonce[2]);
-            const uint4 ks = keystream_block_n(S, pairs[lane].rk, nl + (unsigned long long)(L + 1) * a.C,
-                                               c * W / 16);
-            ksp[warp][lane][0] = ks.x;
-            ksp[warp][lane][1] = ks.y;
-            ksp[warp][lane][2] = ks.z;
-            ksp[warp][lane][3] = ks.w;
+        // ---- keystream of every round, each AES block once per warp; the packed
+        // AND's three blocks ride in the last, partly filled pass (word c = pair /
+        // B covers pairs [cB, cB + B))
+        constexpr int MAIN = NFULL * 3 * NB;
+        for (int idx = lane; idx < MAIN + (MODE == 2 ? 0 : 3); idx += 32) {
+            const int call = idx / (3 * NB), q = idx < MAIN ? (idx / NB) % 3 : idx - MAIN;
+            const unsigned long long off = (unsigned long long)(idx < MAIN ? call : L + 1) * a.C;
+            const unsigned long long blk = idx < MAIN ? p0w * W / 16 + idx % NB : (p0w / B) * W / 16;
+            uint32_t* o = idx < MAIN ? myks + 4 * idx : ksp[warp][q];
+            *reinterpret_cast<uint4*>(o) = keystream_block_n(S, pairs[q].rk, nonce[q] + off, blk);
         }
         __syncwarp();
-        // compare_rows: ASC compares x > y, DESC compares y > x
-        T A[3], Bv[3];
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            A[j] = (MODE == 0 && a.desc) ? Y[j] : X[j];
-            Bv[j] = (MODE == 0 && a.desc) ? X[j] : Y[j];
-        }
+        const T(&A)[3] = X;
+        const T(&Bv)[3] = Y;
         auto kword = [&](int call, int q) -> T {
             const uint32_t* w = myks + (call * 3 + q) * WORDS;
             if constexpr (W == 4) return (T)w[lane];
@@ -294,31 +272,8 @@ __device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&
                     a.eq[j][p] = eq[j];
                     a.gt[j][p] = gt[j];
                 }
-        } else if (MODE == 3) {
-            if (valid) a.cb[xi] = (uint8_t)((gt[0] ^ gt[1] ^ gt[2]) & 1);
-        } else {
-            // swap: x' = x ^ (ext(b) & (y ^ x)), y' = y ^ (ext(b) & (x ^ y))
-            T E[3], D[3], K[3], Z[3];
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                E[j] = gt[j] ? ~(T)0 : (T)0;
-                D[j] = X[j] ^ Y[j];
-                K[j] = kword(L + 1, j);
-            }
-            and3(E, D, K, Z);
-            T Xn[3];
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                Xn[j] = X[j] ^ Z[j];
-                K[j] = kword(L + 2, j);
-            }
-            and3(E, D, K, Z);
-            if (valid)
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    a.key[j][xi] = Xn[j];
-                    a.key[j][yi] = Y[j] ^ Z[j];
-                }
+        } else if (valid) {
+            a.cb[xi] = (uint8_t)((gt[0] ^ gt[1] ^ gt[2]) & 1);
         }
         __syncthreads();  // keystream buffers are rewritten by the next tile
     }
@@ -328,7 +283,7 @@ template <typename T, int MODE>  // as cmp_tile
 __global__ void __launch_bounds__(cmp_threads<sizeof(T)>(), 1) k_cmp(CmpArgs<T> a) {
     constexpr int kCmpThreads = cmp_threads<sizeof(T)>();
     extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ uint32_t ksp[kCmpThreads / 32][3][4];      // packed call block per warp
+    __shared__ __align__(16) uint32_t ksp[kCmpThreads / 32][3][4];  // packed call block per warp
     __shared__ uint32_t ballots[kCmpThreads / 32][3][3];  // [warp][s1,s2,r][share]
     aes_stage_tables(sm);
     const AesSmem S(sm);
@@ -750,60 +705,200 @@ __global__ void k_extend_lsb(CSh3 x, Sh3 y, unsigned long long n) {
             reinterpret_cast<T*>(y.p[j])[i] = (T)0 - (reinterpret_cast<const T*>(x.p[j])[i] & 1);
 }
 
-// ---- batched bitonic sorting -------------------------------------------------
-// Many independent sorts advance one network stage per launch ("round"): a
-// round's work list holds (item, first pair) tiles of every item that still
-// has a stage; stage r has the same (box size, reversal) for every item, and
-// item i's nonces at stage r are its base plus r times its per-stage use, so
-// the shares equal those of sequential plain calls in list order.
-struct CmpBatchItem {
+// ---- bitonic sorting -----------------------------------------------------------
+// One cooperative launch sorts one column or many: stage r of a bitonic network
+// has the same box size and reversal for every size, so round r is a list of
+// tiles (np pairs) of every item that still has a stage, and a grid barrier
+// ends it. Item i's nonces at stage r are its base (where items 0..i-1 of the
+// call end) plus r times its per-stage use, so the shares equal those of
+// sequential calls. All threads compute a tile's keystream, for the round's
+// first tile before the barrier is waited for; then each pair's thread runs
+// the circuit. Bound by the T-table lookups, below 2^17 rows also by the
+// barriers: 2^16 int32 rows took 136 launches, each staging 128 KB of tables,
+// and 2.10 ms, and take 1.06 ms.
+constexpr int kBitThreads = 512;
+// pairs per tile: the keystream of 32 pairs is 3 KB (int32) or 6.75 KB. For
+// int32 two tiles' worth is held, so that a tile costs one block barrier and
+// the warps that are done with its circuit start on the next tile's keystream
+// (2^20 rows: 23.6 and 21.1 ms); int64 keeps larger tiles instead (2^16 rows
+// are then one tile an SM: 2.4 ms, and 3.4 with two buffers of 192 pairs).
+template <int W>
+constexpr int bitonic_max_pairs() { return W == 4 ? 512 : 448; }
+template <int W>
+constexpr int bitonic_bufs() { return W == 4 ? 2 : 1; }
+
+struct BitonicItem {
     void* key[3];
     unsigned long long m;          // pairs (n / 2)
     unsigned long long nonce0[3];  // PAIR nonces at the item's first stage
     unsigned long long C, Cp;      // nonces per full / packed AND call
-    int stages;
+    uint32_t stages;
     int desc;
 };
 
-template <typename T>
-struct CmpBatchArgs {
-    CmpArgs<T> proto;  // keys of the PAIR streams
-    const CmpBatchItem* items;
-    const uint2* work;  // (item, first pair) per tile
-    unsigned nwork;
-    int round, hs, first;
+struct BitonicArgs {
+    AesRK rk[3];
+    BitonicItem one;           // the item of a call with one
+    const BitonicItem* items;  // by stages, most first (null: `one`)
+    const uint32_t* toff;      // [nitems + 1] tiles before each item
+    uint32_t nitems, rounds, np;
+    uint32_t* bar;             // arrivals, counted from 0
+    int* err;
 };
 
-// at most 512 threads per CTA (the item bookkeeping needs registers)
-template <int W>
-constexpr int batch_max_threads() { return W == 4 ? 512 : 448; }
-
 template <typename T>
-__global__ void __launch_bounds__(batch_max_threads<sizeof(T)>(), 1) k_cmp_batch(CmpBatchArgs<T> ba) {
+__global__ void __launch_bounds__(kBitThreads, 1) k_bitonic(BitonicArgs a) {
     constexpr int W = sizeof(T);
     constexpr int L = cmp_levels<W>();
-    constexpr int kCmpThreads = batch_max_threads<W>();
+    constexpr uint32_t NFULL = L + 3;
+    constexpr uint32_t WORDS = 32 * W / 4;  // keystream words per call and stream per warp
+    constexpr uint32_t NB = 32 * W / 16;    // AES blocks of the same
+    constexpr uint32_t PER = NFULL * 3 * NB;
     extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ uint32_t ksp[kCmpThreads / 32][3][4];
-    __shared__ uint32_t ballots[kCmpThreads / 32][3][3];
+    __shared__ __align__(16) uint32_t ksp2[2][kBitThreads / 128 + 1][3][4];  // packed call's block per 128 pairs
+    __shared__ uint32_t ballots[kBitThreads / 32][3][3];
+    __shared__ int s_dead;
+    int flip = 0;
     aes_stage_tables(sm);
     const AesSmem S(sm);
-    for (unsigned w = blockIdx.x; w < ba.nwork; w += gridDim.x) {
-        const uint2 wk = ba.work[w];
-        const CmpBatchItem& it = ba.items[wk.x];
-        CmpArgs<T> a;  // the stream keys stay in the kernel parameters (ba.proto)
-        unsigned long long nonce[3];
-        for (int j = 0; j < 3; j++) {
-            a.key[j] = (T*)it.key[j];
-            nonce[j] = it.nonce0[j] + (unsigned long long)ba.round * ((L + 3) * it.C + it.Cp);
+    const uint32_t tid = threadIdx.x;
+    const int lane = tid & 31, w = tid >> 5;
+    const uint32_t G = gridDim.x, nw = a.np / 32;
+    if (tid == 0) s_dead = 0;
+    uint32_t target = 0, nact = a.nitems;
+    int lev = 0, sub = 0;  // network round and substage
+    for (uint32_t r = 0; r < a.rounds; r++) {
+        const int hs = lev - sub;
+        const bool first = sub == 0;
+        if (a.items)
+            while (nact > 1 && a.items[nact - 1].stages <= r) nact--;
+        const uint32_t total = a.items ? a.toff[nact] : (uint32_t)ceil_div(a.one.m, a.np);
+        bool waited = target == 0;
+        // the previous round is complete everywhere
+        const auto wait = [&]() {
+            if (tid == 0) {
+                // a cooperative launch's CTAs are all resident, so this ends; the
+                // limit turns a lost arrival into an error
+                uint32_t v, spins = 0;
+                do {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+                } while (v < target && ++spins < (1u << 24));
+                if (v < target) {
+                    atomicOr(a.err, 64);
+                    s_dead = 1;
+                }
+            }
+        };
+        for (uint32_t t = blockIdx.x; t < total; t += G, flip ^= bitonic_bufs<W>() - 1) {
+            uint32_t* ksw = sm + kAesSmemBytes / 4 + flip * (nw * PER * 4);
+            uint32_t(*ksp)[3][4] = ksp2[flip];
+            uint32_t idx = 0, hi = nact - 1;  // item of tile t
+            while (idx < hi) {
+                const uint32_t mid = (idx + hi + 1) >> 1;
+                if (a.toff[mid] <= t) idx = mid;
+                else hi = mid - 1;
+            }
+            const BitonicItem& it = a.items ? a.items[idx] : a.one;
+            const unsigned long long m = it.m, C = it.C, Cp = it.Cp;
+            const unsigned long long base = (unsigned long long)(t - (a.items ? a.toff[idx] : 0u)) * a.np;
+            const unsigned long long roff = (unsigned long long)r * ((L + 3) * C + Cp);
+            const uint32_t wn = (uint32_t)min((unsigned long long)nw, ceil_div(m - base, 32));  // warps with pairs
+            // this warp's pairs; past the round's first tile their rows are loaded
+            // ahead of the keystream
+            const bool mine = w < (int)nw;
+            const unsigned long long p0w = base + 32 * w, p = p0w + lane;
+            const bool valid = mine && p < m;
+            unsigned long long xi, yi;
+            bitonic_rows(p, hs, first, xi, yi);
+            T* const* key = reinterpret_cast<T* const*>(it.key);
+            T X[3] = {0, 0, 0}, Y[3] = {0, 0, 0};
+            const auto rows = [&]() {
+                if (valid)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        X[j] = __ldcg(key[j] + xi);
+                        Y[j] = __ldcg(key[j] + yi);
+                    }
+            };
+            if (waited) rows();
+            // a packed block covers 128 pairs: groups base / 128 on
+            const uint32_t np3 = 3 * (((uint32_t)(base & 127) + 32 * wn + 127) / 128);
+            for (uint32_t i = tid; i < np3 + wn * PER; i += kBitThreads) {
+                uint32_t q;
+                unsigned long long off, blk;
+                uint32_t* o;
+                if (i < np3) {
+                    q = i % 3;
+                    off = (unsigned long long)(L + 1) * C;
+                    blk = base / 128 + i / 3;
+                    o = ksp[i / 3][q];
+                } else {
+                    const uint32_t q2 = (i - np3) / PER, rem = (i - np3) - q2 * PER;
+                    const uint32_t call = rem / (3 * NB);
+                    q = (rem / NB) % 3;
+                    off = call <= L ? call * C : call * C + Cp;  // the packed call is the (L + 2)nd
+                    blk = (base + 32 * q2) * W / 16 + rem % NB;
+                    o = ksw + q2 * PER * 4 + rem * 4;
+                }
+                *reinterpret_cast<uint4*>(o) = keystream_block_n(S, a.rk[q], it.nonce0[q] + roff + off, blk);
+            }
+            const bool late = !waited;
+            if (late) wait();
+            waited = true;
+            __syncthreads();
+            if (s_dead) return;  // uniform: written before the barrier above
+            if (late) rows();
+            if (mine) {  // (all warps of a packed word)
+                T A[3], Bv[3], Sm[3], gt[3];
+                // compare_rows: ASC compares x > y, DESC compares y > x
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    A[j] = it.desc ? Y[j] : X[j];
+                    Bv[j] = it.desc ? X[j] : Y[j];
+                }
+                const uint32_t* myks = ksw + w * (NFULL * 3 * WORDS);
+                const auto kword = [&](int call, int q) -> T {
+                    const uint32_t* k = myks + (call * 3 + q) * WORDS;
+                    if constexpr (W == 4) return (T)k[lane];
+                    else return *reinterpret_cast<const T*>(k + 2 * lane);
+                };
+                bit_same3(A, Bv, kword, Sm);
+                gt_bits3(A, Bv, Sm, valid, p, p0w, w, kword, ksp[p0w / 128 - base / 128], ballots, gt);
+                // swap: x' = x ^ (ext(b) & (y ^ x)), y' = y ^ (ext(b) & (x ^ y))
+                T E[3], D[3], K[3], Zx[3], Zy[3];
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    E[j] = gt[j] ? ~(T)0 : (T)0;
+                    D[j] = X[j] ^ Y[j];
+                    K[j] = kword(L + 1, j);
+                }
+                and3(E, D, K, Zx);
+#pragma unroll
+                for (int j = 0; j < 3; j++) K[j] = kword(L + 2, j);
+                and3(E, D, K, Zy);
+                if (valid)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        key[j][xi] = X[j] ^ Zx[j];
+                        key[j][yi] = Y[j] ^ Zy[j];
+                    }
+            }
+            if constexpr (bitonic_bufs<W>() == 1) __syncthreads();  // the next tile rewrites the keystream
         }
-        a.m = it.m;
-        a.C = it.C;
-        a.Cp = it.Cp;
-        a.hs = ba.hs;
-        a.first = ba.first;
-        a.desc = it.desc;
-        cmp_tile<T, 0>(a, ba.proto.pair, nonce, wk.y, S, sm + kAesSmemBytes / 4, ksp, ballots);
+        if (!waited) {  // a CTA without a tile still keeps step: arrivals are counted per round
+            wait();
+        }
+        __syncthreads();
+        if (s_dead) return;
+        target += G;
+        if (tid == 0) {
+            __threadfence();
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+        }
+        if (sub++ == lev) {
+            lev++;
+            sub = 0;
+        }
     }
 }
 
@@ -811,7 +906,7 @@ template <typename T, int MODE>
 void launch_cmp(Ctx& c, const CmpArgs<T>& a, const char* name) {
     constexpr int W = sizeof(T);
     constexpr int L = cmp_levels<W>();
-    constexpr int NFULL = MODE == 0 ? L + 3 : (MODE == 2 ? L : L + 1);
+    constexpr int NFULL = MODE == 2 ? L : L + 1;
     constexpr int kCmpThreads = cmp_threads<W>();
     // spread small stages over every SM: threads per CTA a multiple of 64
     // (whole packed words for both widths) up to the maximum
@@ -877,7 +972,7 @@ void qs_compare_t(Ctx& c, size_t n, CSh3 rows, const uint32_t* idx, const int32_
     constexpr int L = cmp_levels<W>();
     CmpArgs<T> a{};
     for (int j = 0; j < 3; j++) {
-        a.key[j] = (T*)rows.p[j];
+        a.key[j] = (const T*)rows.p[j];
         a.pair[j] = c.stream_arg(PAIR0 + j);
     }
     a.idx = idx;
@@ -919,259 +1014,78 @@ __global__ void k_not1(CSh3 x, Sh3 y, unsigned long long n) {
             reinterpret_cast<T*>(y.p[j])[i] = (reinterpret_cast<const T*>(x.p[j])[i] & 1) ^ 1;
 }
 
+// Sorts `count` columns of power-of-two sizes in one launch; the shares of
+// `count` calls in list order.
 template <typename T>
-void bitonic_t(Ctx& c, size_t n, Sh3 key, bool desc) {
+void bitonic_t(Ctx& c, int count, const size_t* n, const Sh3* keys, const int* desc) {
     constexpr int W = sizeof(T);
     constexpr int L = cmp_levels<W>();
-    int rounds = 0;
-    while (((size_t)1 << rounds) < n) rounds++;
-    const size_t m = n / 2;
-    CmpArgs<T> a{};
-    for (int j = 0; j < 3; j++) a.key[j] = (T*)key.p[j];
-    a.C = chunks_of((unsigned long long)m * W);
-    a.Cp = chunks_of(ceil_div(m, 8 * W) * W);
-    a.m = m;
-    a.desc = desc;
-    for (int i = 0; i < rounds; i++)
-        for (int jj = 0; jj <= i; jj++) {
-            a.hs = i - jj;
-            a.first = jj == 0;
-            for (int q = 0; q < 3; q++) a.pair[q] = c.stream_arg(PAIR0 + q);
-            launch_cmp<T, 0>(c, a, "bitonic_stage");
-            for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += (unsigned long long)(L + 3) * a.C + a.Cp;
-        }
-}
-
-// stage r of a bitonic network: round i with i(i+1)/2 <= r, substage jj
-void stage_of(int r, int& hs, int& first) {
-    int i = 0;
-    while ((i + 1) * (i + 2) / 2 <= r) i++;
-    const int jj = r - i * (i + 1) / 2;
-    hs = i - jj;
-    first = jj == 0;
-}
-
-template <typename T>
-void build_items(Ctx& c, int count, const size_t* n, const Sh3* keys, const int* desc,
-                 std::vector<CmpBatchItem>& items, unsigned long long advance[1], int& rounds) {
-    constexpr int W = sizeof(T);
-    constexpr int L = cmp_levels<W>();
-    items.resize(count);
-    unsigned long long off = 0;
-    rounds = 0;
+    std::vector<BitonicItem> items;
+    unsigned long long off = 0, pairs = 0;
+    double blocks = 0, bytes = 0;
     for (int i = 0; i < count; i++) {
-        CmpBatchItem& it = items[i];
-        int k = 0;
+        uint32_t k = 0;
         while (((size_t)1 << k) < n[i]) k++;
+        if (!k) continue;
+        BitonicItem it;
         it.m = n[i] / 2;
         it.C = chunks_of(it.m * W);
         it.Cp = chunks_of(ceil_div(it.m, 8ull * W) * W);
-        it.stages = n[i] < 2 ? 0 : k * (k + 1) / 2;
+        it.stages = k * (k + 1) / 2;
         it.desc = desc[i];
         for (int j = 0; j < 3; j++) {
             it.key[j] = keys[i].p[j];
             it.nonce0[j] = c.nonce[PAIR0 + j] + off;
         }
         off += (unsigned long long)it.stages * ((L + 3) * it.C + it.Cp);
-        rounds = std::max(rounds, it.stages);
+        pairs += it.m;
+        blocks += it.stages * 3.0 * ((L + 3) * (double)ceil_div(it.m * W, 16) + (double)ceil_div(it.m, 128));
+        bytes += it.stages * 12.0 * W * (double)it.m;
+        items.push_back(it);
     }
-    advance[0] = off;
-}
-
-void build_work(const std::vector<CmpBatchItem>& items, int rounds, int nt, std::vector<uint2>& work,
-                std::vector<size_t>& round_off) {
-    work.clear();
-    round_off.assign(rounds + 1, 0);
-    for (int r = 0; r < rounds; r++) {
-        round_off[r] = work.size();
-        for (size_t i = 0; i < items.size(); i++) {
-            if (items[i].stages <= r) continue;
-            for (unsigned long long p = 0; p < items[i].m; p += nt) work.push_back(make_uint2((unsigned)i, (unsigned)p));
-        }
+    if (items.empty()) return;
+    std::stable_sort(items.begin(), items.end(),
+                     [](const BitonicItem& x, const BitonicItem& y) { return x.stages > y.stages; });
+    // tiles that spread the first round over the SMs, whole packed words each
+    constexpr unsigned long long step = 8 * W;
+    const unsigned long long per_sm = ceil_div(pairs, (unsigned long long)c.num_sms);
+    BitonicArgs a;
+    a.np = (uint32_t)std::min<unsigned long long>(bitonic_max_pairs<W>(), ceil_div(per_sm, step) * step);
+    for (int q = 0; q < 3; q++) a.rk[q] = c.rk[PAIR0 + q];
+    a.one = items[0];
+    a.nitems = (uint32_t)items.size();
+    a.rounds = items[0].stages;
+    a.items = nullptr;
+    a.toff = nullptr;
+    a.err = c.d_err;
+    std::vector<uint32_t> toff(items.size() + 1, 0);
+    for (size_t i = 0; i < items.size(); i++) toff[i + 1] = toff[i] + (uint32_t)ceil_div(items[i].m, a.np);
+    const size_t ib = items.size() * sizeof(BitonicItem), tb = toff.size() * 4;
+    Scratch bar(c, 4), table(c, items.size() > 1 ? ib + tb : 16);
+    if (items.size() > 1) {
+        uint8_t* h = (uint8_t*)c.batch_table(ib + tb);
+        std::memcpy(h, items.data(), ib);
+        std::memcpy(h + ib, toff.data(), tb);
+        ORQ_CUDA_CHECK(cudaMemcpyAsync(table.p, h, ib + tb, cudaMemcpyHostToDevice, c.stream));
+        ORQ_CUDA_CHECK(cudaEventRecord(c.batch.read, c.stream));
+        a.items = table.as<BitonicItem>();
+        a.toff = reinterpret_cast<const uint32_t*>(table.as<uint8_t>() + ib);
     }
-    round_off[rounds] = work.size();
-}
-
-template <typename T>
-size_t batch_smem(int nt) {
-    constexpr int W = sizeof(T);
-    constexpr int L = cmp_levels<W>();
-    return kAesSmemBytes + (size_t)(nt / 32) * (L + 3) * 3 * (32 * W / 4) * 4;
-}
-
-template <typename T>
-CmpArgs<T> batch_proto(Ctx& c) {
-    CmpArgs<T> p{};
-    for (int q = 0; q < 3; q++) p.pair[q] = c.stream_arg(PAIR0 + q);
-    return p;
-}
-
-template <typename T>
-void launch_rounds(Ctx& c, cudaStream_t st, const CmpArgs<T>& proto, const CmpBatchItem* items_dev,
-                   const uint2* work_dev, const std::vector<size_t>& round_off, int rounds, int nt,
-                   bool profile) {
-    auto kern = k_cmp_batch<T>;
+    a.bar = bar.as<uint32_t>();
+    ORQ_CUDA_CHECK(cudaMemsetAsync(bar.p, 0, 4, c.stream));
+    constexpr size_t per_warp = (size_t)(L + 3) * 3 * (32 * W / 4) * 4;
+    const size_t smem = kAesSmemBytes + bitonic_bufs<W>() * (a.np / 32) * per_warp;
+    const auto kern = &k_bitonic<T>;
     ORQ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)batch_smem<T>(batch_max_threads<sizeof(T)>())));
-    for (int r = 0; r < rounds; r++) {
-        CmpBatchArgs<T> ba;
-        ba.proto = proto;
-        ba.items = items_dev;
-        ba.work = work_dev + round_off[r];
-        ba.nwork = (unsigned)(round_off[r + 1] - round_off[r]);
-        ba.round = r;
-        stage_of(r, ba.hs, ba.first);
-        if (!ba.nwork) continue;
-        const unsigned grid = std::min<unsigned>(ba.nwork, (unsigned)c.num_sms);
-        if (profile) {
-            ProfScope ps(c, "bitonic_batch_round", 0.0, 0.0, st);
-            kern<<<grid, nt, batch_smem<T>(nt), st>>>(ba);
-        } else {
-            kern<<<grid, nt, batch_smem<T>(nt), st>>>(ba);
-        }
-        ORQ_CUDA_CHECK(cudaGetLastError());
+                                        (int)(kAesSmemBytes + bitonic_bufs<W>() * (bitonic_max_pairs<W>() / 32) * per_warp)));
+    const unsigned grid = std::min<unsigned>(toff.back(), (unsigned)c.num_sms);
+    {
+        ProfScope ps(c, "bitonic", bytes, blocks);
+        void* args[] = {&a};
+        ORQ_CUDA_CHECK(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kBitThreads), args, smem, c.stream));
     }
-}
-
-// Autotuner: threads per CTA for a size class, chosen by timing round 0 of
-// the batch on scratch copies of (a prefix of) its keys with every candidate.
-template <typename T>
-int autotune(Ctx& c, const std::vector<CmpBatchItem>& items) {
-    constexpr int W = sizeof(T);
-    const int cands4[] = {256, 384, 512};
-    const int cands8[] = {256, 448};
-    const int* cands = W == 4 ? cands4 : cands8;
-    const int nc = W == 4 ? 3 : 2;
-    // a prefix of items of at most 256 MB of shares
-    std::vector<CmpBatchItem> sub;
-    size_t bytes = 0;
-    for (const auto& it : items) {
-        const size_t b = 2 * it.m * W * 3;
-        if (!sub.empty() && bytes + b > (256u << 20)) break;
-        sub.push_back(it);
-        bytes += b;
-    }
-    Scratch keys(c, bytes + 16), itb(c, sub.size() * sizeof(CmpBatchItem) + 16);
-    size_t off = 0;
-    for (auto& it : sub) {
-        for (int j = 0; j < 3; j++) {
-            void* dst = keys.as<uint8_t>() + off;
-            ORQ_CUDA_CHECK(cudaMemcpyAsync(dst, it.key[j], 2 * it.m * W, cudaMemcpyDeviceToDevice, c.stream));
-            it.key[j] = dst;
-            off += 2 * it.m * W;
-        }
-    }
-    ORQ_CUDA_CHECK(cudaMemcpyAsync(itb.p, sub.data(), sub.size() * sizeof(CmpBatchItem),
-                                   cudaMemcpyHostToDevice, c.stream));
-    const CmpArgs<T> proto = batch_proto<T>(c);
-    cudaEvent_t e0, e1;
-    ORQ_CUDA_CHECK(cudaEventCreate(&e0));
-    ORQ_CUDA_CHECK(cudaEventCreate(&e1));
-    int best = cands[0];
-    float best_ms = 1e30f;
-    for (int k = 0; k < nc; k++) {
-        std::vector<uint2> work;
-        std::vector<size_t> roff;
-        build_work(sub, 1, cands[k], work, roff);
-        Scratch wb(c, work.size() * sizeof(uint2) + 16);
-        ORQ_CUDA_CHECK(cudaMemcpyAsync(wb.p, work.data(), work.size() * sizeof(uint2),
-                                       cudaMemcpyHostToDevice, c.stream));
-        float ms = 0;
-        for (int rep = 0; rep < 2; rep++) {
-            ORQ_CUDA_CHECK(cudaEventRecord(e0, c.stream));
-            launch_rounds<T>(c, c.stream, proto, itb.as<CmpBatchItem>(), wb.as<uint2>(), roff, 1, cands[k], false);
-            ORQ_CUDA_CHECK(cudaEventRecord(e1, c.stream));
-            ORQ_CUDA_CHECK(cudaEventSynchronize(e1));
-            ORQ_CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
-        }
-        c.kernels_launched += 2;
-        if (ms < best_ms) {
-            best_ms = ms;
-            best = cands[k];
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    return best;
-}
-
-template <typename T>
-void bitonic_batch_t(Ctx& c, int count, const size_t* n, const Sh3* keys, const int* desc, bool use_graph) {
-    constexpr int W = sizeof(T);
-    std::vector<CmpBatchItem> items;
-    unsigned long long advance[1];
-    int rounds;
-    build_items<T>(c, count, n, keys, desc, items, advance, rounds);
-    if (rounds == 0) return;
-    // size class: key width and log2 of round 0's pairs
-    unsigned long long pairs0 = 0;
-    for (const auto& it : items) pairs0 += it.stages ? it.m : 0;
-    int lg = 0;
-    while ((1ull << lg) < pairs0) lg++;
-    const std::string cls = "bitonic:" + std::to_string(W) + ":" + std::to_string(lg);
-    int nt;
-    if (auto f = c.tuned.find(cls); f != c.tuned.end()) {
-        nt = f->second;
-    } else {
-        nt = autotune<T>(c, items);
-        c.tuned[cls] = nt;
-    }
-    const CmpArgs<T> proto = batch_proto<T>(c);
-    const size_t ibytes = items.size() * sizeof(CmpBatchItem);
-    if (use_graph) {
-        std::string shape = cls + ":" + std::to_string(nt) + ":";
-        for (int i = 0; i < count; i++) shape += std::to_string(n[i]) + ",";
-        BatchGraph& g = c.graphs[shape];
-        if (!g.exec) {
-            std::vector<uint2> work;
-            std::vector<size_t> roff;
-            build_work(items, rounds, nt, work, roff);
-            ORQ_CUDA_CHECK(cudaMalloc(&g.work, std::max<size_t>(16, work.size() * sizeof(uint2))));
-            ORQ_CUDA_CHECK(cudaMemcpy(g.work, work.data(), work.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-            ORQ_CUDA_CHECK(cudaMalloc(&g.items_dev, ibytes));
-            ORQ_CUDA_CHECK(cudaHostAlloc(&g.items_host, ibytes, cudaHostAllocDefault));
-            ORQ_CUDA_CHECK(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming));
-            g.items_bytes = ibytes;
-            g.nt = nt;
-            if (!c.capture_stream)
-                ORQ_CUDA_CHECK(cudaStreamCreateWithFlags(&c.capture_stream, cudaStreamNonBlocking));
-            // the proto's nonces are overwritten per item, so the graph only
-            // depends on the stream keys and the shape
-            cudaGraph_t graph;
-            ORQ_CUDA_CHECK(cudaStreamBeginCapture(c.capture_stream, cudaStreamCaptureModeThreadLocal));
-            ORQ_CUDA_CHECK(cudaMemcpyAsync(g.items_dev, g.items_host, ibytes, cudaMemcpyHostToDevice,
-                                           c.capture_stream));
-            launch_rounds<T>(c, c.capture_stream, proto, (const CmpBatchItem*)g.items_dev,
-                             (const uint2*)g.work, roff, rounds, nt, false);
-            ORQ_CUDA_CHECK(cudaStreamEndCapture(c.capture_stream, &graph));
-            ORQ_CUDA_CHECK(cudaGraphInstantiate(&g.exec, graph, 0));
-            ORQ_CUDA_CHECK(cudaGraphDestroy(graph));
-            for (int r = 0; r < rounds; r++) g.launches += roff[r + 1] > roff[r];
-        }
-        ORQ_CUDA_CHECK(cudaEventSynchronize(g.done));  // the previous replay has read the table
-        std::memcpy(g.items_host, items.data(), ibytes);
-        {
-            ProfScope ps(c, "bitonic_batch_graph", 0.0, 0.0);
-            ORQ_CUDA_CHECK(cudaGraphLaunch(g.exec, c.stream));
-        }
-        ORQ_CUDA_CHECK(cudaEventRecord(g.done, c.stream));
-        c.kernels_launched += g.launches;
-    } else {
-        std::vector<uint2> work;
-        std::vector<size_t> roff;
-        build_work(items, rounds, nt, work, roff);
-        Scratch wb(c, work.size() * sizeof(uint2) + 16), itb(c, ibytes + 16);
-        ORQ_CUDA_CHECK(cudaMemcpyAsync(wb.p, work.data(), work.size() * sizeof(uint2), cudaMemcpyHostToDevice,
-                                       c.stream));
-        ORQ_CUDA_CHECK(cudaMemcpyAsync(itb.p, items.data(), ibytes, cudaMemcpyHostToDevice, c.stream));
-        launch_rounds<T>(c, c.stream, proto, itb.as<CmpBatchItem>(), wb.as<uint2>(), roff, rounds, nt,
-                         c.profiling);
-        for (int r = 0; r < rounds; r++) c.kernels_launched += roff[r + 1] > roff[r];
-        // the host vectors are read by the copies above before they return
-        // (pageable memory), and the scratch goes back to the pool in stream order
-        ORQ_CUDA_CHECK(cudaStreamSynchronize(c.stream));
-    }
-    for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += advance[0];
+    c.kernels_launched++;
+    for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += off;
 }
 
 // nonces of one compare_rows over nkeys keys (each call of m pairs)
@@ -1390,18 +1304,13 @@ void op_not1(Ctx& c, int w, size_t n, CSh3 x, Sh3 y) {
 void op_bitonic_sort(Ctx& c, int w, size_t n, Sh3 key, bool desc) {
     if (n & (n - 1)) throw std::invalid_argument("bitonic sort needs a power-of-two size");
     if (n < 2) return;
-    if (w == 4) bitonic_t<uint32_t>(c, n, key, desc);
-    else if (w == 8) bitonic_t<unsigned long long>(c, n, key, desc);
+    const int d = desc;
+    op_bitonic_sort_batch(c, w, 1, &n, &key, &d);
+}
+void op_bitonic_sort_batch(Ctx& c, int w, int count, const size_t* n, const Sh3* keys, const int* desc) {
+    if (w == 4) bitonic_t<uint32_t>(c, count, n, keys, desc);
+    else if (w == 8) bitonic_t<unsigned long long>(c, count, n, keys, desc);
     else throw std::invalid_argument("bitonic sort supports int32 and int64 keys");
 }
 
-}  // namespace orqcu
-
-namespace orqcu {
-void op_bitonic_sort_batch(Ctx& c, int w, int count, const size_t* n, const Sh3* keys, const int* desc,
-                           bool use_graph) {
-    if (w == 4) bitonic_batch_t<uint32_t>(c, count, n, keys, desc, use_graph);
-    else if (w == 8) bitonic_batch_t<unsigned long long>(c, count, n, keys, desc, use_graph);
-    else throw std::invalid_argument("bitonic sort supports int32 and int64 keys");
-}
 }  // namespace orqcu

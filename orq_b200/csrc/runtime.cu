@@ -317,19 +317,26 @@ Pool::~Pool() {
     for (auto& kv : live_) cudaFree(kv.first);
 }
 
-void Ctx::release_graphs() {
-    for (auto& kv : graphs) {
-        BatchGraph& g = kv.second;
-        if (g.done) cudaEventSynchronize(g.done);
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        if (g.work) cudaFree(g.work);
-        if (g.items_dev) cudaFree(g.items_dev);
-        if (g.items_host) cudaFreeHost(g.items_host);
-        if (g.done) cudaEventDestroy(g.done);
+void* Ctx::batch_table(size_t bytes) {
+    if (!batch.read) ORQ_CUDA_CHECK(cudaEventCreateWithFlags(&batch.read, cudaEventDisableTiming));
+    ORQ_CUDA_CHECK(cudaEventSynchronize(batch.read));
+    if (batch.bytes < bytes) {
+        if (batch.host) cudaFreeHost(batch.host);
+        batch.host = nullptr;
+        batch.bytes = 0;
+        ORQ_CUDA_CHECK(cudaHostAlloc(&batch.host, bytes, cudaHostAllocDefault));
+        batch.bytes = bytes;
     }
-    graphs.clear();
-    if (capture_stream) cudaStreamDestroy(capture_stream);
-    capture_stream = nullptr;
+    return batch.host;
+}
+
+void Ctx::release_batch() {
+    if (batch.read) {
+        cudaEventSynchronize(batch.read);
+        cudaEventDestroy(batch.read);
+    }
+    if (batch.host) cudaFreeHost(batch.host);
+    batch = BatchTable{};
 }
 
 void Ctx::check_device_error() {

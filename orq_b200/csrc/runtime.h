@@ -96,18 +96,11 @@ struct ProfAgg {
     double ms = 0, bytes = 0, aes_blocks = 0;
 };
 
-// A captured batch of launches, cached per batch shape: the work lists and
-// the item table live on the device; the item table is refreshed from the
-// pinned host copy by the graph's first node on every replay.
-struct BatchGraph {
-    cudaGraphExec_t exec = nullptr;
-    void* work = nullptr;        // device work lists (all rounds)
-    void* items_dev = nullptr;   // device item table
-    void* items_host = nullptr;  // pinned item table (source of the graph's copy)
-    size_t items_bytes = 0;
-    cudaEvent_t done = nullptr;  // last replay finished reading items_host
-    int nt = 0;
-    unsigned long long launches = 0;
+// Pinned staging of a batch's item table; `read` marks the last copy out of it.
+struct BatchTable {
+    void* host = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t read = nullptr;
 };
 
 // Streams, events and pinned state of the permutation generator, created on
@@ -145,10 +138,9 @@ struct Ctx {
     int* d_err = nullptr;
     void check_device_error();
     FyRes fy;
-    std::map<std::string, BatchGraph> graphs;  // batched launches by shape
-    std::map<std::string, int> tuned;          // autotuned threads per CTA by size class
-    cudaStream_t capture_stream = nullptr;     // private stream for graph capture
-    void release_graphs();
+    BatchTable batch;
+    void* batch_table(size_t bytes);  // the staging, once its last copy is done
+    void release_batch();
     bool profiling = false;
     std::vector<ProfEvent> prof_pending;
     std::map<std::string, ProfAgg> prof_agg;
@@ -304,7 +296,6 @@ void op_table_sort(Ctx& c, int w, size_t n, int ncols, const Sh3* cols, const in
 void op_distinct(Ctx& c, int w, size_t n, int nkeys, const CSh3* keys, Sh3 res);
 
 // ---- batched bitonic sort (cmp.cu) ----
-void op_bitonic_sort_batch(Ctx& c, int w, int count, const size_t* n, const Sh3* keys, const int* desc,
-                           bool use_graph);
+void op_bitonic_sort_batch(Ctx& c, int w, int count, const size_t* n, const Sh3* keys, const int* desc);
 
 }  // namespace orqcu
