@@ -78,9 +78,24 @@ def _tdtype(width: int):
     return {1: torch.int8, 2: torch.int16, 4: torch.int32, 8: torch.int64, 16: torch.int64}[width]
 
 
+_P3 = ctypes.c_void_p * 3
+
+
+def _rows3(t):
+    """(3, ...) tensor -> the three share row pointers. Computed from the base
+    pointer and the row stride: indexing a tensor costs more than a small
+    call's launch (1000-element AND: 25 us a call with nine row views, 15
+    without)."""
+    b = t.data_ptr()
+    if not b:  # an empty tensor
+        return 0, 0, 0
+    s = t.stride(0) * t.element_size()
+    return b, b + s, b + 2 * s
+
+
 def _p3(t):
     """(3, ...) tensor -> ctypes array of the three share row pointers."""
-    return (ctypes.c_void_p * 3)(*[t[j].data_ptr() for j in range(3)])
+    return _P3(*_rows3(t))
 
 
 class Runtime:
@@ -243,7 +258,6 @@ class SharedVector:
         """open_shares_a/b (replicated_3pc.h:310-330); returns a device tensor."""
         rt = self.rt
         n, w = self.size(), self.width
-        out = rt._alloc(1, w)[0] if n == 0 else None
         torch = _torch()
         shape = (n, 2) if w == 16 else (n,)
         out = torch.empty(shape, dtype=self.shares.dtype, device=self.shares.device)
@@ -550,15 +564,14 @@ def aggregate(keys, agg_spec_b, agg_spec_a, direction: int = Direction.Forward, 
     outputs are overwritten in place."""
     first = keys[0] if keys else (agg_spec_b or agg_spec_a)[0][1]
     rt, n, w = first.rt, first.size(), first.width
-    kp = (ctypes.c_void_p * max(1, 3 * len(keys)))(*[k.shares[j].data_ptr() for k in keys for j in range(3)])
+    kp = _flat(keys)
 
     def specs(lst):
         arr = (_AggSpec * max(1, len(lst)))()
         for i, (inp, out, f) in enumerate(lst):
             src = inp if inp is not None else out
-            for j in range(3):
-                arr[i].inp[j] = src.shares[j].data_ptr()
-                arr[i].out[j] = out.shares[j].data_ptr()
+            arr[i].inp[:] = _rows3(src.shares)
+            arr[i].out[:] = _rows3(out.shares)
             arr[i].func = int(f)
         return arr
 
@@ -569,7 +582,7 @@ def aggregate(keys, agg_spec_b, agg_spec_a, direction: int = Direction.Forward, 
 
 
 def _flat(vecs):
-    return (ctypes.c_void_p * max(1, 3 * len(vecs)))(*[v.shares[j].data_ptr() for v in vecs for j in range(3)])
+    return (ctypes.c_void_p * max(1, 3 * len(vecs)))(*[p for v in vecs for p in _rows3(v.shares)])
 
 
 def compose_permutations(sigma: ASharedVector, rho: ASharedVector) -> ASharedVector:
