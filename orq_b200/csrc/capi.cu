@@ -593,6 +593,7 @@ int orqcu_next_permutation(orqcu_runtime* rt, size_t n, int32_t* const perm_dev[
         need_rt(rt);
         need(perm_dev != nullptr, "null output");
         orqcu::ShardedPerm sp = orqcu::next_perm(rt->ctx, n);
+        orqcu::ensure_perm(rt->ctx, sp);
         for (int g = 0; g < 3; g++)
             if (n)
                 ORQ_CUDA_CHECK(cudaMemcpyAsync(perm_dev[g], sp.perm[g], n * 4, cudaMemcpyDeviceToDevice,

@@ -24,8 +24,9 @@
 //  * fy_small (M <= 2^15, one buffer per permutation almost always):
 //    every (permutation, group) in its own CTA at once from predicted start
 //    buffers, re-run from the first wrong prediction until all are verified;
-//  * fy_finalize: turns the accepted offsets into the final permutation in
-//    parallel and writes its inverse.
+//  * fy_finalize: turns the accepted offsets into the inverse permutation in
+//    parallel (the gather index of an application; the permutation itself,
+//    which only inverse applications read, is derived when one asks for it).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -687,6 +688,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_fy_small(FySmallArgs a) {
 // cursor ends at the bucket's end, which is also the next bucket's start).
 constexpr int kFinThreads = 1024;
 constexpr uint32_t kFinChunk = kFinThreads * 8;  // scan chunk
+// Positions finalized at once: the random accesses of a batch's five arrays
+// then stay in L2. 44 permutations of 2^22 rows (three groups): 111 ms with
+// batches of 12 local permutations, 98 with 6, 87 with 2; smaller sizes take
+// more per batch, down to one batch for all.
+constexpr size_t kFinBatch = (size_t)1 << 23;
 
 struct FinArgs {
     const uint32_t* acc;  // [P][n]
@@ -696,7 +702,6 @@ struct FinArgs {
     int32_t* bucket;      // [P][n] steps grouped by target
     int32_t* par;         // [P][n] max(bucket(k)), -1 when empty
     int32_t* A;           // [P][n]
-    int32_t* const* perm_out;  // [P] -> n
     int32_t* const* inv_out;   // [P] -> n
     int* err;
 };
@@ -834,7 +839,6 @@ __device__ __forceinline__ void fin_emit(const FinArgs& a, size_t pm, uint32_t s
         atomicOr(a.err, 4);
         val = (int32_t)s;
     }
-    a.perm_out[pm][s] = val;
     a.inv_out[pm][val] = (int32_t)s;
 }
 
@@ -919,10 +923,8 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     out.resize(count);
     for (auto& sp : out) {
         sp.n = n;
-        for (int g = 0; g < 3; g++) {
-            sp.perm[g] = (int32_t*)c.alloc(std::max<size_t>(n, 1) * 4);
-            sp.inv[g] = (int32_t*)c.alloc(std::max<size_t>(n, 1) * 4);
-        }
+        int32_t* inv = (int32_t*)c.alloc(3 * std::max<size_t>(n, 1) * 4);
+        for (int g = 0; g < 3; g++) sp.inv[g] = inv + g * n;
     }
     if (n == 0) {
         // gen_perm still draws one buffer (4 nonces) per permutation
@@ -955,32 +957,28 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     // Finalize runs on its own low-priority stream for the permutations the
     // scanners have completed, while the chain goes on (the generator leaves
     // SMs idle while the scanners work through dense windows). acc is laid out
-    // [permutation][group], so B permutations of all three groups are one
+    // [permutation][group], so consecutive local permutations are one
     // contiguous batch; the scratch holds one batch.
-    const size_t fin_b = std::max<size_t>(1, std::min<size_t>({(size_t)4, count,
-                                                               ((size_t)1 << 27) / (3 * std::max<size_t>(n, 1))}));
-    const size_t fin_el = 3 * fin_b * n;
+    const size_t fin_p = std::clamp<size_t>(kFinBatch / n, 1, 3 * count);
+    const size_t fin_el = fin_p * n;
     const uint32_t fin_chunks = (uint32_t)ceil_div(n, (size_t)kFinChunk);
-    Scratch f_cur(c, fin_el * 4), f_part(c, 3 * fin_b * fin_chunks * 4), f_bucket(c, fin_el * 4),
-        f_par(c, fin_el * 4), f_A(c, fin_el * 4), f_ptrs(c, 2 * 3 * count * sizeof(void*));
+    Scratch f_cur(c, fin_el * 4), f_part(c, fin_p * fin_chunks * 4), f_bucket(c, fin_el * 4),
+        f_par(c, fin_el * 4), f_A(c, fin_el * 4), f_ptrs(c, 3 * count * sizeof(void*));
     {
-        std::vector<int32_t*> hp(2 * 3 * count);
+        std::vector<int32_t*> hp(3 * count);
         for (size_t m = 0; m < count; m++)
-            for (int g = 0; g < 3; g++) {
-                hp[3 * m + g] = out[m].perm[g];
-                hp[3 * count + 3 * m + g] = out[m].inv[g];
-            }
+            for (int g = 0; g < 3; g++) hp[3 * m + g] = out[m].inv[g];
         ORQ_CUDA_CHECK(cudaMemcpyAsync(f_ptrs.p, hp.data(), hp.size() * sizeof(void*), cudaMemcpyHostToDevice,
                                        c.stream));
         ORQ_CUDA_CHECK(cudaStreamSynchronize(c.stream));  // hp is pageable and leaves scope
     }
     cudaStream_t fs = R.fs;
-    size_t fin_next = 0;  // permutations [0, fin_next) are queued for finalize
-    auto launch_fin = [&](size_t m0, size_t m1) {
-        const size_t P = 3 * (m1 - m0);
+    size_t fin_next = 0;  // local permutations [0, fin_next) are queued for finalize
+    auto launch_fin = [&](size_t q0, size_t q1) {
+        const size_t P = q1 - q0;
         const size_t el = P * n;
         FinArgs fa;
-        fa.acc = acc.as<uint32_t>() + 3 * m0 * n;
+        fa.acc = acc.as<uint32_t>() + q0 * n;
         fa.n = (uint32_t)n;
         fa.P = (uint32_t)P;
         fa.chunks = fin_chunks;
@@ -989,8 +987,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         fa.bucket = f_bucket.as<int32_t>();
         fa.par = f_par.as<int32_t>();
         fa.A = f_A.as<int32_t>();
-        fa.perm_out = f_ptrs.as<int32_t*>() + 3 * m0;
-        fa.inv_out = f_ptrs.as<int32_t*>() + 3 * count + 3 * m0;
+        fa.inv_out = f_ptrs.as<int32_t*>() + q0;
         fa.err = c.d_err;
         const unsigned gg = plain_grid(c, el);
         const unsigned gc = (unsigned)(P * fin_chunks);
@@ -1088,7 +1085,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         if (ok) {
             for (int g = 0; g < 3; g++)
                 c.nonce[G01 + g] += 4ull * (hstart[g * count + count - 1] + hused[g * count + count - 1]);
-            for (; fin_next < count; fin_next += fin_b) launch_fin(fin_next, std::min(count, fin_next + fin_b));
+            for (; fin_next < 3 * count; fin_next += fin_p) launch_fin(fin_next, std::min(3 * count, fin_next + fin_p));
             ORQ_CUDA_CHECK(cudaEventRecord(R.fin_done, fs));
             ORQ_CUDA_CHECK(cudaStreamWaitEvent(c.stream, R.fin_done, 0));
             c.check_device_error();
@@ -1213,10 +1210,9 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         q.done = z.done != 0;
         bad = bad || z.bad;
         const size_t mmin = std::min({G[0].m, G[1].m, G[2].m});
-        if (!bad && fin_next + fin_b <= mmin && mmin < count) {
-            // the accepted offsets of these permutations precede the states read
-            for (; fin_next + fin_b <= mmin; fin_next += fin_b) launch_fin(fin_next, fin_next + fin_b);
-        }
+        // the accepted offsets of these permutations precede the states read
+        if (!bad && mmin < count)
+            for (; fin_next + fin_p <= 3 * mmin; fin_next += fin_p) launch_fin(fin_next, fin_next + fin_p);
     };
     // Chunks shrink once a chain may end (a permutation's draws deviate by
     // ~1.3 M), and then each waits for the scan of the one before it, so that
@@ -1304,11 +1300,33 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
 
     // the permutations completed since the last batch, then the runtime's
     // stream waits for the finalize stream
-    for (; fin_next < count; fin_next += fin_b) launch_fin(fin_next, std::min(count, fin_next + fin_b));
+    for (; fin_next < 3 * count; fin_next += fin_p) launch_fin(fin_next, std::min(3 * count, fin_next + fin_p));
     ORQ_CUDA_CHECK(cudaEventRecord(R.fin_done, fs));
     ORQ_CUDA_CHECK(cudaStreamWaitEvent(c.stream, R.fin_done, 0));
     c.check_device_error();
 
+}
+
+namespace {
+__global__ void k_invert(const int32_t* inv, int32_t* perm, unsigned long long n, int* err) {
+    for (unsigned long long v = gtid(); v < n; v += gstride()) {
+        const uint32_t s = (uint32_t)inv[v];
+        if (s < n) perm[s] = (int32_t)v;
+        else atomicOr(err, 4);
+    }
+}
+}  // namespace
+
+void ensure_perm(Ctx& c, ShardedPerm& sp) {
+    if (sp.perm[0]) return;
+    int32_t* p = (int32_t*)c.alloc(3 * std::max<size_t>(sp.n, 1) * 4);
+    for (int g = 0; g < 3; g++) sp.perm[g] = p + g * sp.n;
+    if (!sp.n) return;
+    for (int g = 0; g < 3; g++) {
+        k_invert<<<plain_grid(c, sp.n), 256, 0, c.stream>>>(sp.inv[g], sp.perm[g], sp.n, c.d_err);
+        ORQ_CUDA_CHECK(cudaGetLastError());
+        c.kernels_launched++;
+    }
 }
 
 // PermutationManager::reserve (permutation_manager.h:102-181): keep a queue of

@@ -259,12 +259,12 @@ void dispatch_apply(Ctx& c, int w1, bool a1, int w2, bool a2, const ApplyArgs& a
 }  // namespace
 
 // hm_oblivious_apply_sharded_perm / _inverse (shuffle.h:349-412) on one vector.
-void op_apply_sharded(Ctx& c, bool arith, int w, size_t n, Sh3 s, const ShardedPerm& sp,
-                      bool inverse) {
+void op_apply_sharded(Ctx& c, bool arith, int w, size_t n, Sh3 s, ShardedPerm& sp, bool inverse) {
     if (w != 4 && w != 8 && w != 16)
         throw std::invalid_argument("permutation application supports 4, 8 and 16-byte shares");
     const unsigned long long ch = chunks_of((unsigned long long)n * w);
     if (n == 0) return;
+    if (inverse) ensure_perm(c, sp);
     Scratch tmp(c, 3 * n * (size_t)w);
     void* other[3] = {tmp.as<uint8_t>(), tmp.as<uint8_t>() + n * (size_t)w,
                       tmp.as<uint8_t>() + 2 * n * (size_t)w};

@@ -383,11 +383,9 @@ void Ctx::prof_collect() {
 }
 
 void Ctx::free_perm(ShardedPerm& sp) {
-    for (int g = 0; g < 3; g++) {
-        release(sp.perm[g]);
-        release(sp.inv[g]);
-        sp.perm[g] = sp.inv[g] = nullptr;
-    }
+    release(sp.perm[0]);
+    release(sp.inv[0]);
+    for (int g = 0; g < 3; g++) sp.perm[g] = sp.inv[g] = nullptr;
 }
 
 }  // namespace orqcu

@@ -75,7 +75,8 @@ void keep_pool_memory(int device);
 void release_pool_memory(int device);
 
 // A sharded permutation: one local permutation per 2-party group
-// ({0,1},{0,2},{1,2}), each with its inverse, all device-resident int32.
+// ({0,1},{0,2},{1,2}), device-resident int32. Generation produces the inverses
+// (one block of 3n, inv[0]); ensure_perm adds the permutations (perm[0]).
 struct ShardedPerm {
     size_t n = 0;
     int32_t* perm[3] = {nullptr, nullptr, nullptr};
@@ -236,10 +237,10 @@ void release_fy(Ctx& c);
 void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>& out);
 void reserve_perms(Ctx& c, size_t n, size_t count);
 ShardedPerm next_perm(Ctx& c, size_t n);
+void ensure_perm(Ctx& c, ShardedPerm& sp);
 // y = local permutation of x under one group's permutation followed by that
 // group's reshare; idx gives dst[k] = src[idx[k]].
-void op_apply_sharded(Ctx& c, bool arith, int w, size_t n, Sh3 s, const ShardedPerm& sp,
-                      bool inverse);
+void op_apply_sharded(Ctx& c, bool arith, int w, size_t n, Sh3 s, ShardedPerm& sp, bool inverse);
 void op_apply_elementwise(Ctx& c, bool x_arith, int xw, size_t n, Sh3 x, CSh3 perm /*int32 A*/);
 void op_scatter(Ctx& c, int w, size_t n, CSh3 src, Sh3 dst, const int32_t* sigma);
 void op_shuffle(Ctx& c, bool arith, int w, size_t n, Sh3 s);
