@@ -249,18 +249,38 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_classify(FyScanArgs a) {
         uint32_t cnt;
         source(0, src, cnt);
         uint32_t q = 0, e = 0;
-        uint4 nx = make_uint4(0, 0, 0, 0);
-        if (4 * (uint32_t)lane < cnt) nx = *reinterpret_cast<const uint4*>(src + 4 * lane);
-        while (q < a.rl) {
-            const uint32_t left = cnt - min(cnt, e);
-            const uint4 v4 = nx;
-            // the next 128 entries are loaded before these are decided
+        // three chunks of 128 entries in flight; left: entries of a chunk
+        constexpr int kAhead = 3;
+        uint4 nx[kAhead];
+        uint32_t left[kAhead];
+        const auto next = [&](uint4& x, uint32_t& l) {
+            l = 0;
+            if (q >= a.rl) return;
+            if (e + 4 * lane < cnt) x = *reinterpret_cast<const uint4*>(src + e + 4 * lane);
+            l = cnt - e < 128 ? cnt - e : 128;
             e += 128;
-            if (e >= cnt) {
+            while (e >= cnt) {  // (an empty list holds no chunk)
+                if (++q >= a.rl) break;
                 e = 0;
-                if (++q < a.rl) source(q, src, cnt);
+                source(q, src, cnt);
+                if (cnt) break;
             }
-            if (q < a.rl && e + 4 * lane < cnt) nx = *reinterpret_cast<const uint4*>(src + e + 4 * lane);
+        };
+        while (cnt == 0 && ++q < a.rl) source(q, src, cnt);
+#pragma unroll
+        for (int i = 0; i < kAhead; i++) {
+            nx[i] = make_uint4(0, 0, 0, 0);
+            next(nx[i], left[i]);
+        }
+        while (left[0]) {
+            const uint4 v4 = nx[0];
+            const uint32_t n4 = left[0];
+#pragma unroll
+            for (int i = 0; i + 1 < kAhead; i++) {
+                nx[i] = nx[i + 1];
+                left[i] = left[i + 1];
+            }
+            next(nx[kAhead - 1], left[kAhead - 1]);
             const uint32_t v[4] = {v4.x, v4.y, v4.z, v4.w};
             const uint32_t c = k - nu;
             bool cd[4], un[4];
@@ -269,7 +289,7 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_classify(FyScanArgs a) {
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 const uint32_t j = 4u * lane + r;
-                cd[r] = j < left && v[r] + c <= hiu;
+                cd[r] = j < n4 && v[r] + c <= hiu;
                 un[r] = cd[r] && !(some && v[r] + k + j <= lou);
                 any = any || un[r];
                 m[r] = __ballot_sync(0xffffffffu, cd[r]);
@@ -341,7 +361,8 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_classify(FyScanArgs a) {
 constexpr int kResThreads = 512;
 constexpr int kResEach = kPieceUnc / kResThreads;  // 16
 __global__ void __launch_bounds__(kResThreads, 1) k_fy_resolve(FyScanArgs a) {
-    __shared__ __align__(16) uint32_t su[kPieceUnc];
+    // entry k at k + k / 16: a thread reads its 16 without bank conflicts
+    __shared__ uint32_t su[kPieceUnc + kPieceUnc / kResEach];
     __shared__ uint32_t smask[kResThreads], sbef[kResThreads + 1];
     __shared__ uint32_t sc[kResThreads], so[kResThreads + 1];
     __shared__ uint32_t red[33];
@@ -349,7 +370,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_fy_resolve(FyScanArgs a) {
     const FyState s = *a.state;
     const uint32_t nt = fy_step_tiles(a, s);
     const uint32_t tid = threadIdx.x;
-    const int lane = tid & 31, w = tid >> 5;
     if (!nt) {
         if (tid == 0) *a.seg = FySeg{0, s.m};
         return;
@@ -380,18 +400,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_fy_resolve(FyScanArgs a) {
         }
         __syncthreads();
         const uint32_t tot = so[take], call = s_call;
-        for (uint32_t q = w; q < take; q += kResThreads / 32) {
-            const uint2* src = a.unc + (size_t)(t0 + q) * kTileUnc;
-            const uint32_t o = so[q], cnt = so[q + 1] - o, add = cbase + sc[q];
+        // entry i of the piece: the last tile whose entries start at or before it
 #pragma unroll 4
-            for (uint32_t j = lane; j < cnt; j += 32) su[o + j] = src[j].x + add;
+        for (uint32_t i = tid; i < tot; i += kResThreads) {
+            uint32_t q = 0;
+#pragma unroll
+            for (uint32_t b = kResThreads / 2; b; b >>= 1)
+                if (q + b < take && so[q + b] <= i) q += b;
+            su[i + i / kResEach] = a.unc[(size_t)(t0 + q) * kTileUnc + (i - so[q])].x + cbase + sc[q];
         }
         __syncthreads();
         int d[kResEach];  // accepted iff d >= a
 #pragma unroll
         for (int e = 0; e < kResEach; e++) {
             const uint32_t k = tid * kResEach + e;
-            d[e] = k < tot ? top - (int)su[k] : INT32_MIN;
+            d[e] = k < tot ? top - (int)su[k + tid] : INT32_MIN;
         }
         uint32_t start = abase + tid * kResEach / 2, mask = 0;
         for (int pass = 0; pass <= kResThreads; pass++) {  // thread k is settled after pass k at the latest
@@ -1100,8 +1123,11 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     // it). W buffers of 2^20 draws keep every SM busy for ~6 us each.
     constexpr uint32_t kRing = 4;
     // Three SMs are left to k_fy_resolve, whose registers do not fit beside a
-    // generator CTA's; W is rounded so that the last wave of lists is full.
-    const uint32_t gen_sms = (uint32_t)std::max(1, c.num_sms - 3), gen_warps = gen_sms * (kGenThreads / 32);
+    // generator CTA's; up to M = 2^19, where the chain waits for its steps and
+    // not for the generator, 24 (44 permutations of 100003 rows 4.8 and 4.0 ms,
+    // of 262143 7.4 and 6.4; of 2^19 rows, M = 2^20, 11.6 and 11.4). W is
+    // rounded so that the last wave of lists is full.
+    const uint32_t gen_sms = (uint32_t)std::max(1, c.num_sms - (bitsw <= 19 ? 24 : 3)), gen_warps = gen_sms * (kGenThreads / 32);
     const double want = std::clamp(per_perm * count / 8.0, 2.0, 64.0);
     const uint32_t waves = std::max(1u, (uint32_t)(want * kListsPerBuf / gen_warps));
     const uint32_t W = std::max(2u, waves * gen_warps / kListsPerBuf);
