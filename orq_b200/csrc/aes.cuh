@@ -76,21 +76,25 @@ struct AesSmem {
     }
 };
 
+// One full round (1..13) in place.
+__device__ __forceinline__ void aes256_round(const AesSmem& S, const AesRK& rk, const int r, uint32_t& s0, uint32_t& s1,
+                                             uint32_t& s2, uint32_t& s3) {
+    const uint32_t n0 = S.lk<0, 0>(s0) ^ S.lk<1, 1>(s1) ^ S.lk<2, 2>(s2) ^ S.lk<3, 3>(s3) ^ rk.k[4 * r + 0];
+    const uint32_t n1 = S.lk<0, 0>(s1) ^ S.lk<1, 1>(s2) ^ S.lk<2, 2>(s3) ^ S.lk<3, 3>(s0) ^ rk.k[4 * r + 1];
+    const uint32_t n2 = S.lk<0, 0>(s2) ^ S.lk<1, 1>(s3) ^ S.lk<2, 2>(s0) ^ S.lk<3, 3>(s1) ^ rk.k[4 * r + 2];
+    const uint32_t n3 = S.lk<0, 0>(s3) ^ S.lk<1, 1>(s0) ^ S.lk<2, 2>(s1) ^ S.lk<3, 3>(s2) ^ rk.k[4 * r + 3];
+    s0 = n0;
+    s1 = n1;
+    s2 = n2;
+    s3 = n3;
+}
+
 // Rounds R0..14 of one block, in place, from the state after round R0 - 1.
 template <int R0>
 __device__ __forceinline__ void aes256_rounds_from(const AesSmem& S, const AesRK& rk, uint32_t& s0,
                                                    uint32_t& s1, uint32_t& s2, uint32_t& s3) {
 #pragma unroll
-    for (int r = R0; r < 14; r++) {
-        const uint32_t n0 = S.lk<0, 0>(s0) ^ S.lk<1, 1>(s1) ^ S.lk<2, 2>(s2) ^ S.lk<3, 3>(s3) ^ rk.k[4 * r + 0];
-        const uint32_t n1 = S.lk<0, 0>(s1) ^ S.lk<1, 1>(s2) ^ S.lk<2, 2>(s3) ^ S.lk<3, 3>(s0) ^ rk.k[4 * r + 1];
-        const uint32_t n2 = S.lk<0, 0>(s2) ^ S.lk<1, 1>(s3) ^ S.lk<2, 2>(s0) ^ S.lk<3, 3>(s1) ^ rk.k[4 * r + 2];
-        const uint32_t n3 = S.lk<0, 0>(s3) ^ S.lk<1, 1>(s0) ^ S.lk<2, 2>(s1) ^ S.lk<3, 3>(s2) ^ rk.k[4 * r + 3];
-        s0 = n0;
-        s1 = n1;
-        s2 = n2;
-        s3 = n3;
-    }
+    for (int r = R0; r < 14; r++) aes256_round(S, rk, r, s0, s1, s2, s3);
     // last round: S-box bytes read out of the T tables (T2 byte0, T3 byte1,
     // T0 byte2 and T1 byte3 all hold S[x])
     const uint32_t n0 = (S.lk<2, 0>(s0) & 0xffu) | (S.lk<3, 1>(s1) & 0xff00u) |
@@ -165,19 +169,33 @@ __device__ __forceinline__ CtrPre ctr_pre(const AesSmem& S, const AesRK& rk, uns
     return r;
 }
 
-// Block j (of 65536) of the chunk whose constants are pre[0] (byte 13 = 0) and
-// pre[1] (byte 13 = 1).
-__device__ __forceinline__ uint4 keystream_block_pre(const AesSmem& S, const AesRK& rk, const CtrPre* pre, uint32_t j) {
-    const uint32_t ctr = j + 2;
-    const CtrPre* q = pre + (ctr >> 16);
-    const uint2 c = *reinterpret_cast<const uint2*>(q);
-    const uint4 k = *reinterpret_cast<const uint4*>(q->k);
+// Block `blk` of a draw that starts at nonce `nonce0`. With the constants of
+// its chunk in pre[0] (byte 13 = 0) and pre[1] (byte 13 = 1), or without
+// (null); both share the code of rounds 3 to 14: how much code a loop holds
+// decides its speed (the instruction cache), and a short call's latency.
+__device__ __forceinline__ uint4 keystream_block_pre(const AesSmem& S, const AesRK& rk, const CtrPre* pre,
+                                                     unsigned long long nonce0, unsigned long long blk) {
+    const uint32_t ctr = ((uint32_t)blk & 0xffffu) + 2;
+    uint32_t s0, s1, s2, s3;
     const uint32_t w3 = __byte_perm(ctr, 0, 0x0123) ^ rk.k[3];
-    const uint32_t n0 = c.x ^ S.lk<3, 3>(w3), n1 = c.y ^ S.lk<2, 2>(w3);
-    uint32_t s0 = k.x ^ S.lk<0, 0>(n0) ^ S.lk<1, 1>(n1);
-    uint32_t s1 = k.y ^ S.lk<0, 0>(n1) ^ S.lk<3, 3>(n0);
-    uint32_t s2 = k.z ^ S.lk<2, 2>(n0) ^ S.lk<3, 3>(n1);
-    uint32_t s3 = k.w ^ S.lk<1, 1>(n0) ^ S.lk<2, 2>(n1);
+    if (pre) {
+        const CtrPre* q = pre + (ctr >> 16);
+        const uint2 c = *reinterpret_cast<const uint2*>(q);
+        const uint4 k = *reinterpret_cast<const uint4*>(q->k);
+        const uint32_t n0 = c.x ^ S.lk<3, 3>(w3), n1 = c.y ^ S.lk<2, 2>(w3);
+        s0 = k.x ^ S.lk<0, 0>(n0) ^ S.lk<1, 1>(n1);
+        s1 = k.y ^ S.lk<0, 0>(n1) ^ S.lk<3, 3>(n0);
+        s2 = k.z ^ S.lk<2, 2>(n0) ^ S.lk<3, 3>(n1);
+        s3 = k.w ^ S.lk<1, 1>(n0) ^ S.lk<2, 2>(n1);
+    } else {
+        const unsigned long long nonce = nonce0 + (blk >> 16);
+        s0 = (uint32_t)nonce ^ rk.k[0];
+        s1 = (uint32_t)(nonce >> 32) ^ rk.k[1];
+        s2 = rk.k[2];
+        s3 = w3;
+#pragma unroll
+        for (int r = 1; r < 3; r++) aes256_round(S, rk, r, s0, s1, s2, s3);
+    }
     aes256_rounds_from<3>(S, rk, s0, s1, s2, s3);
     return make_uint4(s0, s1, s2, s3);
 }

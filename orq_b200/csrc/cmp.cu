@@ -9,10 +9,8 @@
 // by two multiplexes (operators/common.h:20-28).
 //
 // In loopback every AND round of a pair is local to the thread that holds the
-// pair, so a whole stage is one kernel: each warp first computes the
-// zero-sharing keystream of all its rounds into shared memory (every AES block
-// once), then each thread runs the circuit in registers. The packed fix-up
-// (a bit transpose of 8W consecutive pairs) is a warp ballot.
+// pair, so a whole compare or network stage is one kernel and the circuit runs
+// in registers.
 #include <algorithm>
 #include <cstring>
 #include <string>
@@ -25,14 +23,11 @@ namespace orqcu {
 
 namespace {
 
-// Threads (= pairs) per CTA iteration. The AES tables take 128 KiB of shared
+// Threads (= pairs) per CTA of k_rows_cmp. The AES tables take 128 KiB of shared
 // memory, so one CTA runs per SM; the per-warp keystream buffers take the rest
-// (3 KiB per warp for int32 stages, 6.75 KiB for int64; 512 threads keep the
-// int32 tile within 128 registers a thread).
-// 16-byte shares (padded int64 keys) only run compares (MODE 1) and equality:
-// 256 threads keep 8 keystream calls of 128 words per warp within shared memory.
+// (3 KiB per warp for int32, 6.75 KiB for int64).
 template <int W>
-constexpr int cmp_threads() { return W == 4 ? 512 : (W == 8 ? 448 : 256); }
+constexpr int cmp_threads() { return W == 4 ? 512 : 448; }
 
 // bit_same rounds: log2 of the share's bit width
 template <int W>
@@ -191,218 +186,193 @@ __device__ __forceinline__ void gt_bits3(const T (&A)[3], const T (&Bv)[3], cons
     for (int j = 0; j < 3; j++) gt[j] = (s1[j] >> bitpos) & 1;
 }
 
-// One CTA tile of a compare (MODE 1), an equality (MODE 2) or quicksort's
-// compare (MODE 3): the pairs [base, base + blockDim.x).
-template <typename T, int MODE>
-__device__ __forceinline__ void cmp_tile(const CmpArgs<T>& a, const StreamArg (&pairs)[3],
-                                         const unsigned long long (&nonce)[3], unsigned long long base,
-                                         const AesSmem& S, uint32_t* ksw,
-                                         uint32_t (*ksp)[3][4], uint32_t (*ballots)[3][3]) {
-    constexpr int W = sizeof(T);
-    constexpr int B = 8 * W;               // pairs per packed word
-    constexpr int L = cmp_levels<W>();     // bit_same rounds
-    constexpr int NFULL = MODE == 2 ? L : L + 1;
-    constexpr int WORDS = 32 * W / 4;      // keystream words per call and stream per warp
-    constexpr int NB = 32 * W / 16;        // AES blocks per call and stream per warp
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t* myks = ksw + (size_t)warp * NFULL * 3 * WORDS;
-    {
-        const unsigned long long p0w = base + warp * 32;  // this warp's first pair
-        const unsigned long long p = p0w + lane;
-        const bool valid = p < a.m;
-        // ---- operands, loaded first so their latency hides under the AES work
-        unsigned long long xi = p, yi = p;
-        if (MODE == 3 && valid) {
-            xi = a.idx[p];
-            yi = (unsigned long long)a.head[xi];
-        }
-        T X[3] = {0, 0, 0}, Y[3] = {0, 0, 0};
-        if (valid) {
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                if (MODE == 3) {
-                    X[j] = a.key[j][xi];
-                    Y[j] = a.key[j][yi];
-                } else {
-                    X[j] = a.x[j][p];
-                    Y[j] = a.y[j][p];
-                }
-            }
-        }
-        // ---- keystream of every round, each AES block once per warp; the packed
-        // AND's three blocks ride in the last, partly filled pass (word c = pair /
-        // B covers pairs [cB, cB + B))
-        constexpr int MAIN = NFULL * 3 * NB;
-        for (int idx = lane; idx < MAIN + (MODE == 2 ? 0 : 3); idx += 32) {
-            const int call = idx / (3 * NB), q = idx < MAIN ? (idx / NB) % 3 : idx - MAIN;
-            const unsigned long long off = (unsigned long long)(idx < MAIN ? call : L + 1) * a.C;
-            const unsigned long long blk = idx < MAIN ? p0w * W / 16 + idx % NB : (p0w / B) * W / 16;
-            uint32_t* o = idx < MAIN ? myks + 4 * idx : ksp[warp][q];
-            *reinterpret_cast<uint4*>(o) = keystream_block_n(S, pairs[q].rk, nonce[q] + off, blk);
-        }
-        __syncwarp();
-        const T(&A)[3] = X;
-        const T(&Bv)[3] = Y;
-        auto kword = [&](int call, int q) -> T {
-            const uint32_t* w = myks + (call * 3 + q) * WORDS;
-            if constexpr (W == 4) return (T)w[lane];
-            else if constexpr (W == 8) return (T)w[2 * lane] | ((T)w[2 * lane + 1] << 32);
-            else
-                return (T)w[4 * lane] | ((T)w[4 * lane + 1] << 32) | ((T)w[4 * lane + 2] << 64) |
-                       ((T)w[4 * lane + 3] << 96);
-        };
-        T Sm[3];
-        bit_same3(A, Bv, kword, Sm);
-        if constexpr (MODE == 2) {
-            // operator== : bit_same then mask(1)
-            if (valid)
-#pragma unroll
-                for (int j = 0; j < 3; j++) a.eq[j][p] = Sm[j] & 1;
-            __syncthreads();  // keystream buffers are rewritten by the next tile
-            return;
-        }
-        T gt[3], eq[3];
-        gt_bits3(A, Bv, Sm, valid, p, p0w, warp, kword, ksp[warp], ballots, gt);
-#pragma unroll
-        for (int j = 0; j < 3; j++) eq[j] = Sm[j] & 1;
-        if (MODE == 1) {
-            if (valid)
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    a.eq[j][p] = eq[j];
-                    a.gt[j][p] = gt[j];
-                }
-        } else if (valid) {
-            a.cb[xi] = (uint8_t)((gt[0] ^ gt[1] ^ gt[2]) & 1);
-        }
-        __syncthreads();  // keystream buffers are rewritten by the next tile
-    }
-}
+// ---- _compare and operator== of a whole vector --------------------------------
+// A lane takes one 16-byte unit of every share, E = 16 / W pairs, so a call's
+// keystream is one block a stream that the lane computes itself: nothing is
+// staged, no block is computed for padding, and 16 warps run. The packed sign
+// fix-up is bitwise, and word c's draw sits in block c W / 16: pair p needs bit
+// p % 128 of block p / 128, so the lane works on its own E bits; a warp computes
+// the packed blocks of its next 32 passes at once. CTAs take contiguous ranges;
+// long ones go chunk by chunk with the constant parts of AES rounds 1 and 2
+// (CtrPre). Bound by the T-table lookups. Staged through shared memory (a warp's
+// blocks spread over its lanes) and now: 2^24 int32 pairs == 1.81 and 1.47 ms, >
+// 2.73 and 1.81 ms; the 56 compares of a quicksort of 2^22 int64 rows 94 and 68 ms.
+constexpr int kCmpWarps = kAesThreads / 32;
+// A CTA with at most this many passes (a small call) first computes their
+// keystream with all its warps: the three blocks of up to eight calls in a row
+// took one warp 11 us (> of 1000 int32 pairs: 22.6 and 11.2 us).
+constexpr int kCmpSolo = 4;
+template <int W, int MODE>
+constexpr int cmp_calls() { return cmp_levels<W>() + (MODE == 2 ? 0 : 1); }
 
-template <typename T, int MODE>  // as cmp_tile
-__global__ void __launch_bounds__(cmp_threads<sizeof(T)>(), 1) k_cmp(CmpArgs<T> a) {
-    constexpr int kCmpThreads = cmp_threads<sizeof(T)>();
+template <typename T, int MODE>  // 1: compare, 2: equality, 3: quicksort's compare
+__global__ void __launch_bounds__(kAesThreads, 1) k_cmp(CmpArgs<T> a) {
+    constexpr int W = sizeof(T), E = 16 / W, L = cmp_levels<W>();
+    constexpr int CALLS = cmp_calls<W, MODE>();
     extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ __align__(16) uint32_t ksp[kCmpThreads / 32][3][4];  // packed call block per warp
-    __shared__ uint32_t ballots[kCmpThreads / 32][3][3];  // [warp][s1,s2,r][share]
+    uint4* solo_ks = reinterpret_cast<uint4*>(sm + kAesSmemBytes / 4);  // [pass][call][stream][lane]
+    __shared__ CtrPre pre[CALLS][3][2];       // [call][stream][byte 13]
+    __shared__ uint4 pk[kCmpWarps][3][32];    // packed blocks of a warp's next passes
     aes_stage_tables(sm);
     const AesSmem S(sm);
-    const unsigned long long nonce[3] = {a.pair[0].nonce, a.pair[1].nonce, a.pair[2].nonce};
-    for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < a.m;
-         base += (unsigned long long)gridDim.x * blockDim.x)
-        cmp_tile<T, MODE>(a, a.pair, nonce, base, S, sm + kAesSmemBytes / 4, ksp, ballots);
-}
-
-// ---- _compare of 16-byte shares (padded int64 keys; quicksort's compares) ----
-// A keystream block is one pair's word here, so a lane computes the blocks of
-// its own pair call by call: nothing is staged through shared memory, and 16
-// warps run where the staged circuit had room for 8. Four warps (128 pairs)
-// make a packed word and meet at a barrier of their own; a CTA works on one
-// contiguous range, so the constant parts of rounds 1 and 2 (CtrPre) are built
-// once per 65536 pairs. Bound by the T-table lookups. Quicksort of 2^22 rows:
-// its 56 compares took 94 ms staged and take 79.6 ms.
-constexpr int kCmp16Threads = 512;
-constexpr int kCmp16Calls = cmp_levels<16>() + 1;
-
-template <bool QS>  // quicksort's compare
-__global__ void __launch_bounds__(kCmp16Threads, 1) k_cmp16(CmpArgs<u128> a) {
-    constexpr int L = cmp_levels<16>();
-    extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ CtrPre pre[2][kCmp16Calls][3][2];  // [chunk - first][call][stream][byte 13]
-    __shared__ uint32_t ballots[2][kCmp16Threads / 32][3][3];
-    __shared__ uint4 kp[2][kCmp16Threads / 128][3];  // keystream of the packed AND
-    aes_stage_tables(sm);
-    const AesSmem S(sm);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gr = w >> 2;
-    const unsigned long long units = ceil_div(a.m, 128);
-    const unsigned long long u0 = units * blockIdx.x / gridDim.x, u1 = units * (blockIdx.x + 1) / gridDim.x;
-    int flip = 0;
-    for (unsigned long long s0 = u0; s0 < u1; s0 += 512) {  // spans of 65536 pairs: at most two chunks
-        const unsigned long long s1 = min(u1, s0 + 512), chunk0 = (s0 * 128) >> 16;
-        __syncthreads();  // the span before has read its constants
-        for (int i = threadIdx.x; i < 2 * kCmp16Calls * 3 * 2; i += kCmp16Threads) {
-            const int b13 = i & 1, q = (i >> 1) % 3, call = (i / 6) % kCmp16Calls, ch = i / (6 * kCmp16Calls);
-            pre[ch][call][q][b13] =
-                ctr_pre(S, a.pair[q].rk, a.pair[q].nonce + (unsigned long long)call * a.C + chunk0 + ch, (uint32_t)b13);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // passes: 32 lanes, 32 units each
+    const unsigned long long passes = ceil_div(a.m, 32 * E);
+    const unsigned long long i0 = passes * blockIdx.x / gridDim.x, i1 = passes * (blockIdx.x + 1) / gridDim.x;
+    const bool big = i1 - i0 >= 4 * kCmpWarps, solo = passes <= (unsigned long long)gridDim.x * kCmpSolo;
+    if (solo) {
+        constexpr int JOBS = (CALLS + (MODE != 2)) * 3;  // per pass; the packed call last
+#pragma unroll 1
+        for (int i = w; i < (int)(i1 - i0) * JOBS; i += kCmpWarps) {
+            const int ps = i / JOBS, call = (i % JOBS) / 3, q = i % 3;
+            const unsigned long long it = i0 + ps;
+            const bool packed = call == CALLS;
+            const uint4 k = keystream_block_n(S, a.pair[q].rk, a.pair[q].nonce + (unsigned long long)(packed ? L + 1 : call) * a.C,
+                                              packed ? it * (32 * E) / 128 : it * 32 + lane);
+            if (packed) pk[ps][q][0] = k;  // (the same in every lane)
+            else solo_ks[((ps * CALLS + call) * 3 + q) * 32 + lane] = k;
         }
         __syncthreads();
-        for (unsigned long long u = s0 + gr; u < s1; u += kCmp16Threads / 128, flip ^= 1) {
-            const unsigned long long p = u * 128 + (w & 3) * 32 + lane;
-            const bool valid = p < a.m;
-            u128 A[3] = {0, 0, 0}, Bv[3] = {0, 0, 0};
-            unsigned long long xi = p, yi = p;
-            if (QS && valid) {
-                xi = a.idx[p];
-                yi = (unsigned long long)a.head[xi];
+    }
+    for (unsigned long long s0 = i0; s0 < i1;) {
+        const unsigned long long s1 = big ? min(i1, (s0 / 2048 + 1) * 2048) : i1;  // one chunk: 65536 units
+        if (big) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < CALLS * 6; i += kAesThreads) {
+                const int q = (i >> 1) % 3, call = i / 6;
+                pre[call][q][i & 1] =
+                    ctr_pre(S, a.pair[q].rk, a.pair[q].nonce + (unsigned long long)call * a.C + s0 / 2048, (uint32_t)i & 1u);
             }
-            if (valid)
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    A[j] = Ring<16>::w(__ldg(reinterpret_cast<const uint4*>(QS ? a.key[j] : a.x[j]) + xi));
-                    Bv[j] = Ring<16>::w(__ldg(reinterpret_cast<const uint4*>(QS ? a.key[j] : a.y[j]) + yi));
-                }
-            const uint32_t ch = (uint32_t)((p >> 16) - chunk0), jb = (uint32_t)p & 0xffffu;
-            u128 Sm[3], G[3];
-#pragma unroll
-            for (int j = 0; j < 3; j++) Sm[j] = ~(A[j] ^ Bv[j]);
-            // rolled: three AES bodies stay inside the instruction cache
+            __syncthreads();
+        }
+        for (unsigned long long ib = s0 + w; ib < s1; ib += 32 * kCmpWarps) {
+            if (MODE != 2 && !solo) {
+                const unsigned long long it = ib + (unsigned long long)lane * kCmpWarps;
+                __syncwarp();
+                if (it < s1)
 #pragma unroll 1
-            for (int call = 0; call <= L; call++) {
-                u128 K[3], X[3], Y[3];
-#pragma unroll
-                for (int q = 0; q < 3; q++) K[q] = Ring<16>::w(keystream_block_pre(S, a.pair[q].rk, pre[ch][call][q], jb));
-                const int sh = call < L ? 1 << call : 1;
+                    for (int q = 0; q < 3; q++)
+                        pk[w][q][lane] = keystream_block_n(
+                            S, a.pair[q].rk, a.pair[q].nonce + (unsigned long long)(L + 1) * a.C, it * (32 * E) / 128);
+                __syncwarp();
+            }
+            for (int g = 0; g < 32; g++) {
+                const unsigned long long it = ib + (unsigned long long)g * kCmpWarps;
+                if (it >= s1) break;
+                const unsigned long long u = it * 32 + lane, p = u * E;
+                T A[E][3], Sm[E][3], G[E][3];
+                uint32_t sa[3] = {0, 0, 0}, sb[3] = {0, 0, 0};  // sign bits, bit e = pair p + e
+                unsigned long long xi[E];
 #pragma unroll
                 for (int j = 0; j < 3; j++) {
-                    const u128 t = ashr(Sm[j], sh);
-                    X[j] = call < L ? Sm[j] : t ^ Sm[j];
-                    Y[j] = call < L ? t : A[j];
+                    union {
+                        uint4 v;
+                        T t[E];
+                    } x, y;
+                    if constexpr (MODE == 3) {
+#pragma unroll
+                        for (int e = 0; e < E; e++) {
+                            x.t[e] = y.t[e] = 0;
+                            if (p + e < a.m) {
+                                if (j == 0) xi[e] = a.idx[p + e];
+                                x.t[e] = a.key[j][xi[e]];
+                                y.t[e] = a.key[j][(unsigned long long)a.head[xi[e]]];
+                            }
+                        }
+                    } else {
+                        x.v = ld16(a.x[j], u, a.m * W);
+                        y.v = ld16(a.y[j], u, a.m * W);
+                    }
+#pragma unroll
+                    for (int e = 0; e < E; e++) {
+                        A[e][j] = x.t[e];
+                        Sm[e][j] = ~(x.t[e] ^ y.t[e]);
+                        sa[j] |= (uint32_t)(x.t[e] >> (8 * W - 1)) << e;
+                        sb[j] |= (uint32_t)(y.t[e] >> (8 * W - 1)) << e;
+                    }
                 }
-                and3(X, Y, K, G);
-                if (call < L)
+                // bit_same's L prefix ANDs, then gt = ((eq >> 1) ^ eq) & this
+#pragma unroll 1
+                for (int call = 0; call < CALLS; call++) {
+                    union {
+                        uint4 v;
+                        T t[E];
+                    } k[3];
+                    // the stream loop is rolled: with one AES body the loop stays
+                    // inside the instruction cache (three took 1.2 times as long);
+                    // each pass appends stream q
+                    k[1].v = k[2].v = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+                    for (int q = 0; q < 3; q++) {
+                        k[0].v = k[1].v;
+                        k[1].v = k[2].v;
+                        if (solo)
+                            k[2].v = solo_ks[((w * CALLS + call) * 3 + q) * 32 + lane];
+                        else
+                            k[2].v = keystream_block_pre(S, a.pair[q].rk, big ? pre[call][q] : nullptr,
+                                                         a.pair[q].nonce + (unsigned long long)call * a.C, u);
+                    }
+                    const int sh = call < L ? 1 << call : 1;
 #pragma unroll
-                    for (int j = 0; j < 3; j++) Sm[j] = G[j];
-            }
+                    for (int e = 0; e < E; e++) {
+                        const T K[3] = {k[0].t[e], k[1].t[e], k[2].t[e]};
+                        T X[3], Y[3];
 #pragma unroll
-            for (int j = 0; j < 3; j++) {
-                const uint32_t b1 = __ballot_sync(0xffffffffu, valid && ((A[j] >> 127) & 1));
-                const uint32_t b2 = __ballot_sync(0xffffffffu, valid && ((Bv[j] >> 127) & 1));
-                const uint32_t br = __ballot_sync(0xffffffffu, valid && parity(G[j]));
-                if (lane == 0) {
-                    ballots[flip][w][0][j] = b1;
-                    ballots[flip][w][1][j] = b2;
-                    ballots[flip][w][2][j] = br;
+                        for (int j = 0; j < 3; j++) {
+                            const T t = ashr(Sm[e][j], sh);
+                            X[j] = call < L ? Sm[e][j] : t ^ Sm[e][j];
+                            Y[j] = call < L ? t : A[e][j];
+                        }
+                        and3(X, Y, K, G[e]);
+                        if (call < L)
+#pragma unroll
+                            for (int j = 0; j < 3; j++) Sm[e][j] = G[e][j];
+                    }
                 }
-            }
-            if ((w & 3) == 0 && lane < 3) {
-                const unsigned long long nl =
-                    lane == 0 ? a.pair[0].nonce : (lane == 1 ? a.pair[1].nonce : a.pair[2].nonce);
-                kp[flip][gr][lane] = keystream_block_n(S, a.pair[lane].rk, nl + (unsigned long long)(L + 1) * a.C, u);
-            }
-            asm volatile("bar.sync %0, 128;" ::"r"(1 + gr) : "memory");
-            // sign fix-up on this warp's 32 bits of the packed word (bitwise, so
-            // the words of the other warps do not matter): r ^= s2; s2 ^= s1;
-            // s2 = ~(~s2 & ~r); s1 ^= s2
-            uint32_t s1[3], ns2[3], nr[3], K[3], Z[3];
+                union {
+                    uint4 v;
+                    T t[E];
+                } o;
+                if constexpr (MODE != 3) {
 #pragma unroll
-            for (int j = 0; j < 3; j++) {
-                s1[j] = ballots[flip][w][0][j];
-                const uint32_t s2 = ballots[flip][w][1][j];
-                ns2[j] = ~(s2 ^ s1[j]);
-                nr[j] = ~(ballots[flip][w][2][j] ^ s2);
-                K[j] = reinterpret_cast<const uint32_t*>(&kp[flip][gr][j])[w & 3];
-            }
-            and3(ns2, nr, K, Z);
-            if (QS) {
-                if (valid) a.cb[xi] = (uint8_t)(((s1[0] ^ s1[1] ^ s1[2] ^ ~(Z[0] ^ Z[1] ^ Z[2])) >> lane) & 1);
-            } else if (valid) {
+                    for (int j = 0; j < 3; j++) {
 #pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    a.eq[j][p] = Sm[j] & 1;
-                    a.gt[j][p] = ((s1[j] ^ ~Z[j]) >> lane) & 1;
+                        for (int e = 0; e < E; e++) o.t[e] = Sm[e][j] & 1;
+                        st16(a.eq[j], u, a.m * W, o.v);
+                    }
+                }
+                if constexpr (MODE != 2) {
+                    // r = parity ^ s2; s2 ^= s1; s2 = ~(~s2 & ~r) (one AND); gt = s1 ^ s2
+                    uint32_t ns2[3], nr[3], K[3], Z[3];
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        uint32_t r = sb[j];
+#pragma unroll
+                        for (int e = 0; e < E; e++) r ^= (uint32_t)parity(G[e][j]) << e;
+                        ns2[j] = ~(sb[j] ^ sa[j]);
+                        nr[j] = ~r;
+                        const uint32_t bit = (uint32_t)p & 127u;
+                        K[j] = reinterpret_cast<const uint32_t*>(&pk[w][j][g])[bit >> 5] >> (bit & 31u);
+                    }
+                    and3(ns2, nr, K, Z);
+                    if constexpr (MODE == 3) {
+                        const uint32_t gt = sa[0] ^ sa[1] ^ sa[2] ^ ~(Z[0] ^ Z[1] ^ Z[2]);
+#pragma unroll
+                        for (int e = 0; e < E; e++)
+                            if (p + e < a.m) a.cb[xi[e]] = (uint8_t)((gt >> e) & 1);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 3; j++) {
+                            const uint32_t gt = sa[j] ^ ~Z[j];
+#pragma unroll
+                            for (int e = 0; e < E; e++) o.t[e] = (gt >> e) & 1;
+                            st16(a.gt[j], u, a.m * W, o.v);
+                        }
+                    }
                 }
             }
         }
+        s0 = s1;
     }
 }
 
@@ -904,36 +874,17 @@ __global__ void __launch_bounds__(kBitThreads, 1) k_bitonic(BitonicArgs a) {
 
 template <typename T, int MODE>
 void launch_cmp(Ctx& c, const CmpArgs<T>& a, const char* name) {
-    constexpr int W = sizeof(T);
-    constexpr int L = cmp_levels<W>();
-    constexpr int NFULL = MODE == 2 ? L : L + 1;
-    constexpr int kCmpThreads = cmp_threads<W>();
-    // spread small stages over every SM: threads per CTA a multiple of 64
-    // (whole packed words for both widths) up to the maximum
-    const unsigned long long per_sm = ceil_div(a.m, (unsigned long long)c.num_sms);
-    constexpr unsigned long long G = W == 16 ? 128 : 64;  // threads of whole packed words
-    const int nt = (int)std::min<unsigned long long>(kCmpThreads, std::max<unsigned long long>(G, ceil_div(per_sm, G) * G));
-    const size_t ks_bytes = (size_t)(nt / 32) * NFULL * 3 * (32 * W / 4) * 4;
-    const size_t smem = kAesSmemBytes + ks_bytes;
-    const size_t smem_max = kAesSmemBytes + (size_t)(kCmpThreads / 32) * NFULL * 3 * (32 * W / 4) * 4;
-    auto kern = k_cmp<T, MODE>;
-    ORQ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-    const unsigned long long units = ceil_div(a.m, nt);
-    const unsigned grid = (unsigned)std::min<unsigned long long>(units ? units : 1, (unsigned long long)c.num_sms);
-    const double calls = NFULL;
+    constexpr int W = sizeof(T), L = cmp_levels<W>();
+    const auto kern = k_cmp<T, MODE>;
+    constexpr int solo = kCmpSolo * cmp_calls<W, MODE>() * 3 * 32 * 16;
+    ORQ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAesSmemBytes + solo));
+    // a small call spreads over the SMs, a warp's pass each
+    const unsigned long long units = ceil_div(a.m * W, 16);
+    const unsigned grid = (unsigned)std::min<unsigned long long>(ceil_div(units, 32), (unsigned long long)c.num_sms);
     ProfScope ps(c, name, (MODE == 2 ? 9.0 : 12.0) * W * a.m,
-                 calls * 3.0 * ceil_div(a.m * W, 16) + (MODE == 2 ? 0.0 : 3.0 * ceil_div(ceil_div(a.m, 8 * W) * W, 16)));
-    kern<<<grid, nt, smem, c.stream>>>(a);
-    ORQ_CUDA_CHECK(cudaGetLastError());
-    c.kernels_launched++;
-}
-
-template <bool QS>
-void launch_cmp16(Ctx& c, const CmpArgs<u128>& a) {
-    prep_aes_kernel(k_cmp16<QS>);
-    const unsigned grid = (unsigned)std::min<unsigned long long>(ceil_div(a.m, 128), (unsigned long long)c.num_sms);
-    ProfScope ps(c, "compare", 12.0 * 16 * a.m, kCmp16Calls * 3.0 * a.m + 3.0 * ceil_div(a.m, 128));
-    k_cmp16<QS><<<grid, kCmp16Threads, kAesSmemBytes, c.stream>>>(a);
+                 3.0 * ((MODE == 2 ? L : L + 1) * (double)units + (MODE == 2 ? 0.0 : (double)ceil_div(a.m, 128))));
+    const bool small = ceil_div(units, 32) <= (unsigned long long)grid * kCmpSolo;  // as the kernel's `solo`
+    kern<<<grid, kAesThreads, kAesSmemBytes + (small ? solo : 0), c.stream>>>(a);
     ORQ_CUDA_CHECK(cudaGetLastError());
     c.kernels_launched++;
 }
@@ -953,12 +904,7 @@ void compare_t(Ctx& c, size_t n, CSh3 x, CSh3 y, Sh3 eq, Sh3 gt) {
     a.C = chunks_of((unsigned long long)n * W);
     a.Cp = chunks_of(ceil_div(n, 8 * W) * W);
     a.m = n;
-    if constexpr (W == 16) {
-        if (n)
-            launch_cmp16<false>(c, a);
-    } else if (n) {
-        launch_cmp<T, 1>(c, a, "compare");
-    }
+    if (n) launch_cmp<T, 1>(c, a, "compare");
     for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += (unsigned long long)(L + 1) * a.C + a.Cp;
 }
 
@@ -981,10 +927,7 @@ void qs_compare_t(Ctx& c, size_t n, CSh3 rows, const uint32_t* idx, const int32_
     a.C = chunks_of((unsigned long long)n * W);
     a.Cp = chunks_of(ceil_div(n, 8 * W) * W);
     a.m = n;
-    if (n) {
-        if constexpr (W == 16) launch_cmp16<true>(c, a);
-        else launch_cmp<T, 3>(c, a, "compare");
-    }
+    if (n) launch_cmp<T, 3>(c, a, "compare");
     for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += (unsigned long long)(L + 1) * a.C + a.Cp;
 }
 

@@ -62,6 +62,11 @@ __device__ __forceinline__ uint4 ld16(const void* base, unsigned long long blk,
     const uint8_t* p = reinterpret_cast<const uint8_t*>(base) + off;
     if (off + 16 <= nbytes && ((reinterpret_cast<uintptr_t>(p) & 15) == 0))
         return __ldg(reinterpret_cast<const uint4*>(p));
+    // rows of an odd length start on an element: word accesses, not bytes
+    if (off + 16 <= nbytes && ((reinterpret_cast<uintptr_t>(p) & 3) == 0)) {
+        const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
+        return make_uint4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+    }
     union {
         uint4 v;
         uint8_t b[16];
@@ -78,6 +83,14 @@ __device__ __forceinline__ void st16(void* base, unsigned long long blk, unsigne
     uint8_t* p = reinterpret_cast<uint8_t*>(base) + off;
     if (off + 16 <= nbytes && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
         *reinterpret_cast<uint4*>(p) = v;
+        return;
+    }
+    if (off + 16 <= nbytes && ((reinterpret_cast<uintptr_t>(p) & 3) == 0)) {
+        uint32_t* q = reinterpret_cast<uint32_t*>(p);
+        q[0] = v.x;
+        q[1] = v.y;
+        q[2] = v.z;
+        q[3] = v.w;
         return;
     }
     union {

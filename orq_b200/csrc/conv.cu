@@ -85,10 +85,10 @@ __global__ void __launch_bounds__(kRcaThreads, 1) k_rca(RcaArgs a) {
     const auto fill = [&](uint32_t* out, int s, int g, uint32_t blk) {
         const int r = 4 * g + (lane >> 3);
         const int round = min(16 * s + r, B - 2);  // the top bit has no carry out
-#pragma unroll
-        for (int q = 0; q < 3; q++)
+#pragma unroll 1
+        for (int q = 0; q < 3; q++)  // (rolled: one AES body)
             *reinterpret_cast<uint4*>(out + (r * 3 + q) * 32 + 4 * (lane & 7)) =
-                keystream_block_pre(S, a.pair[q].rk, pre + (round * 3 + q) * 2, blk + (lane & 7));
+                keystream_block_pre(S, a.pair[q].rk, pre + (round * 3 + q) * 2, 0, blk + (lane & 7));
     };
     // word wd of this warp's elements of one array, coalesced. Elements past n
     // repeat the last one: their sums are not stored, and no element's sum

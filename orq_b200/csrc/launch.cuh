@@ -24,6 +24,44 @@ inline unsigned plain_grid(const Ctx& c, unsigned long long units, int threads =
     return (unsigned)(g < cap ? g : cap);
 }
 
+// Runs body(b, v, k) for this CTA's contiguous share of the keystream blocks
+// [0, nblk): k[q] is block b of stream q (keys rk(q), draw starting at nonce
+// nonce(q)), v = load(b) the operands, loaded ahead of the keystream. With
+// enough blocks the constant parts of rounds 1 and 2 are built once per chunk
+// in `pre` ([NS][2], shared); a short range does without them, since building
+// them takes about the time of three blocks.
+constexpr unsigned long long kPreMinBlocks = 8 * kAesThreads;
+template <int NS, typename RK, typename NONCE, typename LD, typename F>
+__device__ __forceinline__ void for_keystream(const AesSmem& S, CtrPre* pre, unsigned long long nblk, RK rk,
+                                              NONCE nonce, LD load, F body) {
+    const unsigned long long units = (nblk + 63) / 64;  // ranges start on 1 KiB
+    const unsigned long long lo = units * blockIdx.x / gridDim.x * 64;
+    unsigned long long hi = units * (blockIdx.x + 1) / gridDim.x * 64;
+    if (hi > nblk) hi = nblk;
+    const bool big = hi >= lo + kPreMinBlocks;
+    for (unsigned long long s0 = lo; s0 < hi;) {
+        const unsigned long long chunk = s0 >> 16, end = (chunk + 1) << 16, s1 = big && end < hi ? end : hi;
+        if (big) {
+            __syncthreads();
+            if (threadIdx.x < 2 * NS)
+                pre[threadIdx.x] = ctr_pre(S, rk(threadIdx.x >> 1), nonce(threadIdx.x >> 1) + chunk, threadIdx.x & 1);
+            __syncthreads();
+        }
+        for (unsigned long long b = s0 + threadIdx.x; b < s1; b += blockDim.x) {
+            const auto v = load(b);
+            uint4 k[NS] = {};
+#pragma unroll 1
+            for (int q = 0; q < NS; q++) {  // one AES body; each pass appends its block
+#pragma unroll
+                for (int i = 0; i + 1 < NS; i++) k[i] = k[i + 1];
+                k[NS - 1] = keystream_block_pre(S, rk(q), big ? pre + 2 * q : nullptr, nonce(q), b);
+            }
+            body(b, v, k);
+        }
+        s0 = s1;
+    }
+}
+
 template <typename K>
 inline void prep_aes_kernel(K kern) {
     ORQ_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,

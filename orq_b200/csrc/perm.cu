@@ -100,11 +100,14 @@ __device__ __forceinline__ void load_idx(const int32_t* idx, unsigned long long 
 // of two per block keep the kernel's loop inside the instruction cache (fully
 // unrolled, ten AES-256 bodies stalled every warp on instruction fetch).
 template <int W, bool A, int B>
-__device__ __forceinline__ void reshare_block(const AesSmem& S, StreamArg gs, unsigned long long ch,
+__device__ __forceinline__ void reshare_block(const AesSmem& S, const StreamArg& gs, unsigned long long ch,
                                               unsigned long long blk, uint4 (&v)[3][B]) {
-    const uint4 r0 = keystream_block(S, gs, blk);
-    gs.nonce += ch;
-    const uint4 r1 = keystream_block(S, gs, blk);
+    uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
+#pragma unroll 1
+    for (int c = 0; c < 2; c++) {  // (rolled: one AES body)
+        r0 = r1;
+        r1 = keystream_block_n(S, gs.rk, gs.nonce + c * ch, blk);
+    }
     uint4 r2;
     if constexpr (A) r2 = Ring<W>::sub(Ring<W>::sub(make_uint4(0, 0, 0, 0), r0), r1);
     else r2 = r0 ^ r1;

@@ -23,7 +23,7 @@ __device__ __forceinline__ uint4 lsb_mask() {
 }
 
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kAesThreads) k_keystream(StreamArg st, uint8_t* out,
+__global__ void __launch_bounds__(kAesThreads, 1) k_keystream(StreamArg st, uint8_t* out,
                                                            unsigned long long nbytes) {
     extern __shared__ __align__(16) uint32_t sm[];
     aes_stage_tables(sm);
@@ -36,23 +36,21 @@ __global__ void __launch_bounds__(kAesThreads) k_keystream(StreamArg st, uint8_t
 // secret_share_b/a on the owner (replicated_3pc.h:353-448): share_1, share_2
 // are two consecutive draws of the owner's local PRG.
 template <int W, bool ARITH>
-__global__ void __launch_bounds__(kAesThreads)
+__global__ void __launch_bounds__(kAesThreads, 1)
     k_share(const uint8_t* data, void* s1, void* s2, void* s3, StreamArg st,
             unsigned long long chunks, unsigned long long nbytes) {
     extern __shared__ __align__(16) uint32_t sm[];
     aes_stage_tables(sm);
     const AesSmem S(sm);
-    StreamArg st2 = st;
-    st2.nonce += chunks;
-    const unsigned long long nblk = ceil_div(nbytes, 16);
-    for (unsigned long long b = gtid(); b < nblk; b += gstride()) {
-        const uint4 a = keystream_block(S, st, b);
-        const uint4 c = keystream_block(S, st2, b);
-        const uint4 d = ld16(data, b, nbytes);
-        st16(s1, b, nbytes, a);
-        st16(s2, b, nbytes, c);
-        st16(s3, b, nbytes, Share<W, ARITH>::minus(Share<W, ARITH>::minus(d, a), c));
-    }
+    __shared__ CtrPre pre[4];
+    for_keystream<2>(
+        S, pre, ceil_div(nbytes, 16), [&](int) -> const AesRK& { return st.rk; },
+        [&](int q) { return st.nonce + q * chunks; }, [&](unsigned long long b) { return ld16(data, b, nbytes); },
+        [&](unsigned long long b, const uint4& d, const uint4 (&k)[2]) {
+            st16(s1, b, nbytes, k[0]);
+            st16(s2, b, nbytes, k[1]);
+            st16(s3, b, nbytes, Share<W, ARITH>::minus(Share<W, ARITH>::minus(d, k[0]), k[1]));
+        });
 }
 
 struct MultArgs {
@@ -67,32 +65,40 @@ struct MultArgs {
 // of ZeroSharingGenerator::getNextBinary/Arithmetic (zero_sharing_generator.h:
 // 101-148): r_p = PAIR[p-1] (-|^) PAIR[p].
 template <int W, bool ARITH>
-__global__ void __launch_bounds__(kAesThreads) k_mult(MultArgs a) {
+__global__ void __launch_bounds__(kAesThreads, 1) k_mult(MultArgs a) {
     using Sh = Share<W, ARITH>;
     extern __shared__ __align__(16) uint32_t sm[];
     aes_stage_tables(sm);
     const AesSmem S(sm);
-    const unsigned long long nblk = ceil_div(a.nbytes, 16);
-    for (unsigned long long b = gtid(); b < nblk; b += gstride()) {
-        const uint4 k0 = keystream_block(S, a.pair[0], b);
-        const uint4 k1 = keystream_block(S, a.pair[1], b);
-        const uint4 k2 = keystream_block(S, a.pair[2], b);
+    struct Operands {
         uint4 x[3], y[3];
+    };
+    __shared__ CtrPre pre[6];
+    for_keystream<3>(
+        S, pre, ceil_div(a.nbytes, 16), [&](int q) -> const AesRK& { return a.pair[q].rk; },
+        [&](int q) { return a.pair[q].nonce; },
+        [&](unsigned long long b) {
+            Operands v;
 #pragma unroll
-        for (int p = 0; p < 3; p++) {
-            x[p] = ld16(a.x[p], b, a.nbytes);
-            y[p] = ld16(a.y[p], b, a.nbytes);
-        }
-        const uint4 r[3] = {Sh::minus(k2, k0), Sh::minus(k0, k1), Sh::minus(k1, k2)};
+            for (int p = 0; p < 3; p++) {
+                v.x[p] = ld16(a.x[p], b, a.nbytes);
+                v.y[p] = ld16(a.y[p], b, a.nbytes);
+            }
+            return v;
+        },
+        [&](unsigned long long b, const Operands& o, const uint4 (&k)[3]) {
+            const uint4(&x)[3] = o.x;
+            const uint4(&y)[3] = o.y;
+            const uint4 r[3] = {Sh::minus(k[2], k[0]), Sh::minus(k[0], k[1]), Sh::minus(k[1], k[2])};
 #pragma unroll
-        for (int p = 0; p < 3; p++) {
-            const int q = (p + 1) % 3;
-            uint4 v = Sh::plus(r[p], Sh::times(x[p], y[p]));
-            v = Sh::plus(v, Sh::times(x[p], y[q]));
-            v = Sh::plus(v, Sh::times(x[q], y[p]));
-            st16(a.z[p], b, a.nbytes, v);
-        }
-    }
+            for (int p = 0; p < 3; p++) {
+                const int q = (p + 1) % 3;
+                uint4 v = Sh::plus(r[p], Sh::times(x[p], y[p]));
+                v = Sh::plus(v, Sh::times(x[p], y[q]));
+                v = Sh::plus(v, Sh::times(x[q], y[p]));
+                st16(a.z[p], b, a.nbytes, v);
+            }
+        });
 }
 
 struct B2AArgs {
@@ -107,59 +113,77 @@ struct B2AArgs {
 // s0/s1, one inside multiply_a) and the two exchanges are element-local in
 // loopback, so the whole conversion is one pass.
 template <int W>
-__global__ void __launch_bounds__(kAesThreads) k_b2a(B2AArgs a) {
+__global__ void __launch_bounds__(kAesThreads, 1) k_b2a(B2AArgs a) {
     using R = Ring<W>;
     extern __shared__ __align__(16) uint32_t sm[];
     aes_stage_tables(sm);
     const AesSmem S(sm);
     const uint4 one = lsb_mask<W>();
-    const unsigned long long nblk = ceil_div(a.nbytes, 16);
-    for (unsigned long long b = gtid(); b < nblk; b += gstride()) {
-        // z[call][party]; the call loop stays rolled (three AES bodies, not
-        // nine, keep the loop inside the instruction cache): each call shifts
-        // the rows up and appends its own, so z[c] ends up holding call c
-        uint4 z[3][3] = {};
-#pragma unroll 1
-        for (int c = 0; c < 3; c++) {
-            uint4 k[3];
-#pragma unroll
-            for (int q = 0; q < 3; q++) {
-                StreamArg st = a.pair[q];
-                st.nonce += (unsigned long long)c * a.chunks;
-                k[q] = keystream_block(S, st, b);
+    __shared__ CtrPre pre[3][3][2];  // [call][stream][byte 13]
+    const unsigned long long units = (ceil_div(a.nbytes, 16) + 63) / 64;
+    const unsigned long long lo = units * blockIdx.x / gridDim.x * 64;
+    const unsigned long long hi = min(ceil_div(a.nbytes, 16), units * (blockIdx.x + 1) / gridDim.x * 64);
+    // contiguous ranges; long ones with the constants of rounds 1 and 2 built
+    // once per chunk (as for_keystream, for nine calls)
+    const bool big = hi >= lo + kPreMinBlocks;
+    for (unsigned long long s0 = lo; s0 < hi;) {
+        const unsigned long long chunk = s0 >> 16, s1 = big ? min(hi, (chunk + 1) << 16) : hi;
+        if (big) {
+            __syncthreads();
+            if (threadIdx.x < 18) {
+                const int c = threadIdx.x / 6, q = (threadIdx.x / 2) % 3;
+                pre[c][q][threadIdx.x & 1] = ctr_pre(S, a.pair[q].rk, a.pair[q].nonce + c * a.chunks + chunk, threadIdx.x & 1);
             }
+            __syncthreads();
+        }
+        for (unsigned long long b = s0 + threadIdx.x; b < s1; b += blockDim.x) {
+            // z[call][party]; calls and streams in rolled loops (one AES body keeps
+            // the loop inside the instruction cache): each pass appends its block,
+            // each call shifts the rows up and appends its own
+            uint4 z[3][3] = {}, k[3] = {};
+#pragma unroll 1
+            for (int c = 0; c < 3; c++) {
+#pragma unroll 1
+                for (int q = 0; q < 3; q++) {
+                    k[0] = k[1];
+                    k[1] = k[2];
+                    k[2] = keystream_block_pre(S, a.pair[q].rk, big ? pre[c][q] : nullptr,
+                                               a.pair[q].nonce + c * a.chunks, b);
+                }
+#pragma unroll
+                for (int p = 0; p < 3; p++) {
+                    z[0][p] = z[1][p];
+                    z[1][p] = z[2][p];
+                }
+                z[2][0] = R::sub(k[2], k[0]);
+                z[2][1] = R::sub(k[0], k[1]);
+                z[2][2] = R::sub(k[1], k[2]);
+            }
+            const uint4 x0 = ld16(a.x[0], b, a.nbytes), x1 = ld16(a.x[1], b, a.nbytes),
+                        x2 = ld16(a.x[2], b, a.nbytes);
+            const uint4 abit = (x0 ^ x1) & one;  // P0 folds its two masked shares
+            const uint4 bbit = x2 & one;         // P1 adds its second masked share
+            uint4 d[3];
+            d[0] = R::sub(R::add(z[0][0], abit), z[1][0]);
+            d[1] = R::sub(z[0][1], R::add(z[1][1], bbit));
+            d[2] = R::sub(z[0][2], z[1][2]);
 #pragma unroll
             for (int p = 0; p < 3; p++) {
-                z[0][p] = z[1][p];
-                z[1][p] = z[2][p];
+                const int q = (p + 1) % 3;
+                uint4 v = R::add(z[2][p], R::mul(d[p], d[p]));
+                v = R::add(v, R::mul(d[p], d[q]));
+                v = R::add(v, R::mul(d[q], d[p]));
+                st16(a.y[p], b, a.nbytes, v);
             }
-            z[2][0] = R::sub(k[2], k[0]);
-            z[2][1] = R::sub(k[0], k[1]);
-            z[2][2] = R::sub(k[1], k[2]);
         }
-        const uint4 x0 = ld16(a.x[0], b, a.nbytes), x1 = ld16(a.x[1], b, a.nbytes),
-                    x2 = ld16(a.x[2], b, a.nbytes);
-        const uint4 abit = (x0 ^ x1) & one;  // P0 folds its two masked shares
-        const uint4 bbit = x2 & one;         // P1 adds its second masked share
-        uint4 d[3];
-        d[0] = R::sub(R::add(z[0][0], abit), z[1][0]);
-        d[1] = R::sub(z[0][1], R::add(z[1][1], bbit));
-        d[2] = R::sub(z[0][2], z[1][2]);
-#pragma unroll
-        for (int p = 0; p < 3; p++) {
-            const int q = (p + 1) % 3;
-            uint4 v = R::add(z[2][p], R::mul(d[p], d[p]));
-            v = R::add(v, R::mul(d[p], d[q]));
-            v = R::add(v, R::mul(d[q], d[p]));
-            st16(a.y[p], b, a.nbytes, v);
-        }
+        s0 = s1;
     }
 }
 
 // Protocol::reshare (protocol.h:500-541) in place: r0, r1 from the group
 // stream, r2 = r0^r1 or -r0-r1 (zero_sharing_generator.h:158-183).
 template <int W, bool ARITH>
-__global__ void __launch_bounds__(kAesThreads)
+__global__ void __launch_bounds__(kAesThreads, 1)
     k_reshare(void* s0, void* s1, void* s2, StreamArg g, unsigned long long chunks,
               unsigned long long nbytes) {
     extern __shared__ __align__(16) uint32_t sm[];
@@ -181,7 +205,7 @@ __global__ void __launch_bounds__(kAesThreads)
 }
 
 template <int W, bool ARITH>
-__global__ void __launch_bounds__(kAesThreads)
+__global__ void __launch_bounds__(kAesThreads, 1)
     k_zero(void* r0o, void* r1o, void* r2o, StreamArg p0, StreamArg p1, StreamArg p2,
            unsigned long long nbytes) {
     using Sh = Share<W, ARITH>;
