@@ -562,11 +562,15 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_emit(FyScanArgs a) {
 // d ≈ M·H_n draws (std ≈ 1.3·M) and 1 + floor(d / 2^20) getNext buffers, a
 // count that is predictable: permutation m of a group is assumed to start at
 // buffer m·b̂ of the chain, and every (permutation, group) pair runs at once,
-// one CTA each, with no host round trip. Warps 1.. generate the draws chunk
-// by chunk into shared memory (two chunk buffers), warp 0 replays the
-// acceptance 32 draws at a time (lane j is certainly accepted if v + j <= T,
-// rejected if v > T, and the rest are decided in order) and reports the
-// buffers the permutation used. The host then checks the assumed starts
+// one CTA each, with no host round trip. The CTA generates 8192 draws into
+// shared memory and replays the acceptance on them min(8192, M) at a time: a
+// thread holds consecutive draws and decides them from an assumed number of
+// acceptances before its first, the block's prefix sums give the next
+// assumption, until nothing changes (thread 0 starts from the true count; a
+// threshold moves little over M draws, so a few passes do). A warp that walked
+// the draws beside the generating warps was the bottleneck: 42 permutations of
+// 20000 rows 1.77 and 0.93 ms, of 10000 rows 1.29 and 0.58, of 1000 rows 0.70
+// and 0.21. The CTA reports the buffers used. The host then checks the assumed starts
 // against the used counts; from the first permutation of a group whose start
 // was wrong, the rest are run again from the corrected start (each pass
 // fixes at least that one). A permutation needing more than `max_chunks`
@@ -578,7 +582,8 @@ constexpr int kSmallThreads = 512;
 // rows took 20.2 ms with this path and takes 19.5 with the chain
 constexpr uint32_t kSmallMaxM = 1u << 15;
 constexpr uint32_t kChunksPerBuffer = (1u << 20) / kSmallChunk;  // 128
-constexpr size_t kSmallSmem = (size_t)kAesSmemBytes + 2 * kSmallChunk * 4;
+constexpr size_t kSmallSmem = (size_t)kAesSmemBytes + kSmallChunk * 4;
+constexpr int kSmallEach = kSmallChunk / kSmallThreads;  // 16: draws a thread decides at most at once
 
 struct FySmallArgs {
     StreamArg st[3];  // chain start of each group (buffer 0)
@@ -597,100 +602,78 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_fy_small(FySmallArgs a) {
     __shared__ uint32_t s_dlast;
     aes_stage_tables(sm);
     const AesSmem S(sm);
-    uint32_t* buf = sm + kAesSmemBytes / 4;  // [2][kSmallChunk]
-    StreamArg st = a.st[g];
-    st.nonce += 4ull * a.start[g * a.count + m];  // 4 nonces per buffer
-    const uint32_t n = a.n;
+    uint32_t* buf = sm + kAesSmemBytes / 4;  // [kSmallChunk]
+    __shared__ uint32_t red[33];
+    __shared__ CtrPre pre[2];
+    const AesRK& rk = a.st[g].rk;
+    const unsigned long long nonce = a.st[g].nonce + 4ull * a.start[g * a.count + m];  // 4 nonces per buffer
+    const uint32_t n = a.n, tid = threadIdx.x;
     uint32_t* acc = a.acc + ((size_t)m * 3 + g) * n;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t i = 0;  // accepted so far (warp 0)
-    // iteration k produces chunk k into buf[k & 1] and consumes chunk k - 1
-    // from buf[(k - 1) & 1]; the barrier that opens an iteration publishes
-    // chunk k - 1, frees the buffer chunk k - 2 held, and stops every thread
-    // at once when the permutation is complete
-    for (uint32_t k = 0; k <= a.max_chunks; k++) {
-        if (__syncthreads_or(warp == 0 && i >= n)) break;
-        if (warp > 0) {
-            if (k < a.max_chunks) {
-                uint4* dst = reinterpret_cast<uint4*>(buf + (k & 1) * kSmallChunk);
-                const unsigned long long blk0 = (unsigned long long)k * (kSmallChunk / 4);
-                for (uint32_t b = threadIdx.x - 32; b < kSmallChunk / 4; b += kSmallThreads - 32) {
-                    const uint4 ks = keystream_block(S, st, blk0 + b);
-                    dst[b] = make_uint4(ks.x & a.mask, ks.y & a.mask, ks.z & a.mask, ks.w & a.mask);
-                }
-            }
-        } else if (k > 0) {
-            const uint32_t* src = buf + ((k - 1) & 1) * kSmallChunk;
-            const uint32_t d0 = (k - 1) * kSmallChunk;  // draw index of the chunk's first draw
-            // 128 draws at a time (lane l holds draws 32u + l): T only
-            // decreases, so a group with no draw <= T now has no acceptance
-            // and is skipped whole (most groups, late in a permutation)
-            for (uint32_t base = 0; base < kSmallChunk && i < n; base += 128) {
-                uint32_t v4[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) v4[u] = src[base + 32u * u + lane];
-                const uint32_t mn = min(min(v4[0], v4[1]), min(v4[2], v4[3]));
-                const uint32_t T0 = n - 1 - i;
-                if (!__any_sync(0xffffffffu, mn <= T0)) continue;
-                // draw q = 32u + l of the group is certainly accepted if
-                // v + q <= T0 (at most q acceptances precede it) and rejected if
-                // v > T0; when no draw lies in between, every fate is known and
-                // the ranks are prefix counts in draw order (one pass, no
-                // dependence between the four rounds)
-                uint32_t cm[4];
-                bool und = false;
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const uint32_t q = 32u * u + (uint32_t)lane;
-                    const bool cert = v4[u] + q <= T0;
-                    cm[u] = __ballot_sync(0xffffffffu, cert);
-                    und = und || (!cert && v4[u] <= T0);
-                }
-                if (!__any_sync(0xffffffffu, und)) {
-                    uint32_t run = i;
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        if ((cm[u] >> lane) & 1u) {
-                            const uint32_t r = run + (uint32_t)__popc(cm[u] & lt);
-                            if (r < n) {
-                                acc[r] = v4[u];
-                                if (r == n - 1) s_dlast = d0 + base + 32u * u + (uint32_t)lane;
-                            }
-                        }
-                        run += (uint32_t)__popc(cm[u]);
-                    }
-                    i = run;
-                    continue;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    if (i >= n) break;
-                    const uint32_t v = v4[u];  // v <= mask < 2^17: v + lane cannot wrap
-                    const uint32_t T = n - 1 - i;
-                    const bool cert = v + (uint32_t)lane <= T;
-                    uint32_t ok = __ballot_sync(0xffffffffu, cert);
-                    uint32_t pend = __ballot_sync(0xffffffffu, !cert && v <= T);
-                    while (pend) {
-                        const int j = __ffs(pend) - 1;
-                        pend &= pend - 1;
-                        const uint32_t vj = __shfl_sync(0xffffffffu, v, j);
-                        if (vj + (uint32_t)__popc(ok & ((1u << j) - 1u)) <= T) ok |= 1u << j;
-                    }
-                    if ((ok >> lane) & 1u) {
-                        const uint32_t r = i + (uint32_t)__popc(ok & lt);
-                        if (r < n) {
-                            acc[r] = v;
-                            if (r == n - 1) s_dlast = d0 + base + 32u * u + (uint32_t)lane;
-                        }
-                    }
-                    i += (uint32_t)__popc(ok);
-                }
-            }
+    const uint32_t mbits = 32 - __clz(a.mask);
+    // draws a thread takes at once: at most M for the block
+    const uint32_t each = min((uint32_t)kSmallEach, max(1u, (1u << mbits) / kSmallThreads));
+    uint32_t i = 0;  // accepted so far
+    for (uint32_t k = 0; k < a.max_chunks && i < n; k++) {
+        const unsigned long long blk0 = (unsigned long long)k * (kSmallChunk / 4);
+        if (!(blk0 & 0xffffu)) {  // a new nonce (the barrier below it has freed pre)
+            if (tid < 2) pre[tid] = ctr_pre(S, rk, nonce + (blk0 >> 16), tid);
+            __syncthreads();
         }
+        for (uint32_t b = tid; b < kSmallChunk / 4; b += kSmallThreads) {
+            const uint4 ks = keystream_block_pre(S, rk, pre, 0, blk0 + b);
+            reinterpret_cast<uint4*>(buf)[b] = make_uint4(ks.x & a.mask, ks.y & a.mask, ks.z & a.mask, ks.w & a.mask);
+        }
+        __syncthreads();
+        for (uint32_t s0 = 0; s0 < kSmallChunk && i < n; s0 += each * kSmallThreads) {
+            const uint32_t T = n - 1 - i;
+            const uint32_t d0 = s0 + tid * each;  // this thread's first draw of the chunk
+            uint32_t v[kSmallEach];
+            bool any = false;
+#pragma unroll
+            for (int e = 0; e < kSmallEach; e += 4) {
+                uint4 x = make_uint4(0x7fffffffu, 0x7fffffffu, 0x7fffffffu, 0x7fffffffu);
+                if ((uint32_t)e + 4 <= each) {  // (each is a power of two)
+                    x = *reinterpret_cast<const uint4*>(buf + d0 + e);
+                } else if (e == 0) {
+                    x.x = buf[d0];
+                    if (each > 1) x.y = buf[d0 + 1];
+                }
+                v[e] = x.x;
+                v[e + 1] = x.y;
+                v[e + 2] = x.z;
+                v[e + 3] = x.w;
+                any = any || min(min(x.x, x.y), min(x.z, x.w)) <= T;
+            }
+            // T only decreases: a stretch without a draw <= T has no acceptance
+            if (!__syncthreads_or(any)) continue;
+            uint32_t before = (uint32_t)(((unsigned long long)tid * each * (T + 1)) >> mbits), got = 0, all = 0;
+            for (int pass = 0; pass <= kSmallThreads; pass++) {  // thread k is settled after pass k at the latest
+                uint32_t x = before;
+                got = 0;
+#pragma unroll
+                for (int e = 0; e < kSmallEach; e++)
+                    if (v[e] + x <= T) {
+                        got |= 1u << e;
+                        x++;
+                    }
+                const uint32_t next = block_excl_sum(x - before, red, all);
+                const bool moved = next != before;
+                before = next;
+                if (!__syncthreads_or(moved)) break;
+            }
+            uint32_t o = i + before;
+#pragma unroll
+            for (int e = 0; e < kSmallEach; e++)
+                if ((got >> e) & 1u) {
+                    acc[o] = v[e];  // o < n: an acceptance needs v + (acceptances before it) <= T
+                    if (o == n - 1) s_dlast = k * kSmallChunk + d0 + e;
+                    o++;
+                }
+            i += all;
+        }
+        __syncthreads();  // the next chunk rewrites the draws
     }
-    __syncwarp();
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         // gen_perm refills each time its index reaches the end of a buffer,
         // the last accepted draw included: 1 + floor(draws / 2^20) buffers
         if (i >= n) a.used[g * a.count + m] = 1u + (s_dlast + 1u) / (1u << 20);
@@ -786,19 +769,35 @@ __global__ void __launch_bounds__(kFinThreads) k_fin_starts(FinArgs a) {
     __shared__ uint32_t red[33];
     const size_t pm = blockIdx.x / a.chunks, ch = blockIdx.x % a.chunks;
     uint32_t* c = a.cur + pm * a.n;
-    const size_t k0 = ch * kFinChunk + (size_t)threadIdx.x * 8;  // 8 consecutive per thread
+    // coalesced: element u * kFinThreads + thread of the chunk, through shared
+    // memory to 8 consecutive ones a thread for the scan and back (a thread's 8
+    // consecutive global words took 47 us for 2^23 positions, now 16)
+    __shared__ uint32_t sv[kFinChunk + kFinChunk / 8];
+    const size_t c0 = ch * kFinChunk;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        const uint32_t k = u * kFinThreads + threadIdx.x;
+        sv[k + k / 8] = c0 + k < a.n ? c[c0 + k] : 0u;
+    }
+    __syncthreads();
     uint32_t v[8], s = 0;
 #pragma unroll
     for (int u = 0; u < 8; u++) {
-        v[u] = k0 + u < a.n ? c[k0 + u] : 0u;
+        v[u] = sv[threadIdx.x * 9 + u];
         s += v[u];
     }
     uint32_t tot;
     uint32_t pre = block_excl_sum(s, red, tot) + a.part[pm * a.chunks + ch];
 #pragma unroll
     for (int u = 0; u < 8; u++) {
-        if (k0 + u < a.n) c[k0 + u] = pre;
+        sv[threadIdx.x * 9 + u] = pre;
         pre += v[u];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        const uint32_t k = u * kFinThreads + threadIdx.x;
+        if (c0 + k < a.n) c[c0 + k] = sv[k + k / 8];
     }
 }
 
