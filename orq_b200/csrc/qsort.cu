@@ -94,6 +94,38 @@ __device__ __forceinline__ void block_scan2(uint32_t s, int32_t m, uint32_t* rs,
     __syncthreads();  // rs / rm are reused by the caller's next scan
 }
 
+// A thread's kQsPer consecutive positions of an int32 / byte array in one
+// access (the arrays start on 16 bytes; positions past n read as `pad`).
+template <typename I>
+__device__ __forceinline__ void qs_load4(const I* x, size_t base, size_t n, I pad, int32_t (&v)[kQsPer]) {
+    if (base + kQsPer <= n) {
+        if constexpr (sizeof(I) == 4) {
+            const int4 q = *reinterpret_cast<const int4*>(x + base);
+            v[0] = q.x;
+            v[1] = q.y;
+            v[2] = q.z;
+            v[3] = q.w;
+        } else {
+            const uint32_t q = *reinterpret_cast<const uint32_t*>(x + base);
+#pragma unroll
+            for (int u = 0; u < kQsPer; u++) v[u] = (q >> (8 * u)) & 255u;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < kQsPer; u++) v[u] = base + u < n ? x[base + u] : pad;
+    }
+}
+template <typename I>
+__device__ __forceinline__ void qs_store4(I* x, size_t base, size_t n, const int32_t (&v)[kQsPer]) {
+    if (base + kQsPer <= n) {
+        *reinterpret_cast<int4*>(x + base) = make_int4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int u = 0; u < kQsPer; u++)
+            if (base + u < n) x[base + u] = (I)v[u];
+    }
+}
+
 // MODE 0: (non-pivots, max pivot) per chunk; MODE 1: zeros per chunk
 template <int MODE>
 __global__ void __launch_bounds__(kQsThreads) k_qs_part(QsRound a) {
@@ -101,18 +133,16 @@ __global__ void __launch_bounds__(kQsThreads) k_qs_part(QsRound a) {
     __shared__ int32_t rm[32];
     const size_t base = (size_t)blockIdx.x * kQsChunk + (size_t)threadIdx.x * kQsPer;
     uint32_t s = 0;
-    int32_t m = -1;
+    int32_t m = -1, p[kQsPer], b[kQsPer];
+    qs_load4(a.piv, base, a.n, 0, p);  // (past n: pivots at 0, which count nothing)
+    if (MODE == 1) qs_load4<uint8_t>(a.cb, base, a.n, 1, b);
 #pragma unroll
     for (int u = 0; u < kQsPer; u++) {
-        const size_t q = base + u;
-        if (q < a.n) {
-            const int32_t p = a.piv[q];
-            if (MODE == 0) {
-                s += p < 0;
-                m = max(m, p);
-            } else {
-                s += p < 0 && a.cb[q] == 0;
-            }
+        if (MODE == 0) {
+            s += p[u] < 0;
+            if (base + u < a.n) m = max(m, p[u]);
+        } else {
+            s += p[u] < 0 && b[u] == 0;
         }
     }
     uint32_t es, ts;
@@ -154,9 +184,9 @@ __global__ void __launch_bounds__(kQsThreads) k_qs_heads(QsRound a) {
     int32_t p[kQsPer];
     uint32_t s = 0;
     int32_t m = -1;
+    qs_load4(a.piv, base, a.n, 0, p);
 #pragma unroll
     for (int u = 0; u < kQsPer; u++) {
-        p[u] = base + u < a.n ? a.piv[base + u] : 0;
         if (base + u < a.n) {
             s += p[u] < 0;
             m = max(m, p[u]);
@@ -166,15 +196,14 @@ __global__ void __launch_bounds__(kQsThreads) k_qs_heads(QsRound a) {
     int32_t em, tm;
     block_scan2(s, m, rs, rm, es, em, ts, tm);
     uint32_t r = a.psum[blockIdx.x] + es;
-    int32_t h = max(a.pmax[blockIdx.x], em);
+    int32_t h = max(a.pmax[blockIdx.x], em), hd[kQsPer];
 #pragma unroll
     for (int u = 0; u < kQsPer; u++) {
-        const size_t q = base + u;
-        if (q >= a.n) break;
-        h = max(h, p[u]);
-        a.head[q] = h;
-        if (p[u] < 0) a.idx[r++] = (uint32_t)q;
+        if (base + u < a.n) h = max(h, p[u]);
+        hd[u] = h;
+        if (base + u < a.n && p[u] < 0) a.idx[r++] = (uint32_t)(base + u);
     }
+    qs_store4(a.head, base, a.n, hd);
 }
 
 // zeros up to and including each position
@@ -182,11 +211,13 @@ __global__ void __launch_bounds__(kQsThreads) k_qs_zeros(QsRound a) {
     __shared__ uint32_t rs[32];
     __shared__ int32_t rm[32];
     const size_t base = (size_t)blockIdx.x * kQsChunk + (size_t)threadIdx.x * kQsPer;
-    uint32_t z[kQsPer], s = 0;
+    uint32_t s = 0;
+    int32_t z[kQsPer], p[kQsPer], b[kQsPer];
+    qs_load4(a.piv, base, a.n, 0, p);
+    qs_load4<uint8_t>(a.cb, base, a.n, 1, b);
 #pragma unroll
     for (int u = 0; u < kQsPer; u++) {
-        const size_t q = base + u;
-        z[u] = q < a.n && a.piv[q] < 0 && a.cb[q] == 0;
+        z[u] = p[u] < 0 && b[u] == 0;
         s += z[u];
     }
     uint32_t es, ts;
@@ -195,11 +226,10 @@ __global__ void __launch_bounds__(kQsThreads) k_qs_zeros(QsRound a) {
     uint32_t g = a.psum[blockIdx.x] + es;
 #pragma unroll
     for (int u = 0; u < kQsPer; u++) {
-        const size_t q = base + u;
-        if (q >= a.n) break;
         g += z[u];
-        a.gz[q] = g;
+        z[u] = (int32_t)g;
     }
+    qs_store4(a.gz, base, a.n, z);
 }
 
 // segment totals at the heads, and each zero's position by rank
