@@ -43,8 +43,9 @@ struct CmpArgs {
     StreamArg pair[3];  // nonces at the start of the compare
     unsigned long long C, Cp;  // nonces per full-size and per packed AND call
     unsigned long long m;      // pairs
-    // quicksort's compare: pair p is (key[idx[p]], key[head[idx[p]]]), and only
-    // the opened gt bit is kept, at cb[idx[p]]
+    // quicksort's compare: with q = idx[p], pair p is (key[ord[q]],
+    // key[ord[head[q]]]), and only the opened gt bit is kept, at cb[q]
+    const uint32_t* ord;
     const uint32_t* idx;
     const int32_t* head;
     uint8_t* cb;
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(kAesThreads, 1) k_cmp(CmpArgs<T> a) {
                 const unsigned long long u = it * 32 + lane, p = u * E;
                 T A[E][3], Sm[E][3], G[E][3];
                 uint32_t sa[3] = {0, 0, 0}, sb[3] = {0, 0, 0};  // sign bits, bit e = pair p + e
-                unsigned long long xi[E];
+                uint32_t xi[E], xr[E], yr[E];
 #pragma unroll
                 for (int j = 0; j < 3; j++) {
                     union {
@@ -274,9 +275,13 @@ __global__ void __launch_bounds__(kAesThreads, 1) k_cmp(CmpArgs<T> a) {
                         for (int e = 0; e < E; e++) {
                             x.t[e] = y.t[e] = 0;
                             if (p + e < a.m) {
-                                if (j == 0) xi[e] = a.idx[p + e];
-                                x.t[e] = a.key[j][xi[e]];
-                                y.t[e] = a.key[j][(unsigned long long)a.head[xi[e]]];
+                                if (j == 0) {
+                                    xi[e] = a.idx[p + e];
+                                    xr[e] = a.ord[xi[e]];
+                                    yr[e] = a.ord[a.head[xi[e]]];
+                                }
+                                x.t[e] = a.key[j][xr[e]];
+                                y.t[e] = a.key[j][yr[e]];
                             }
                         }
                     } else {
@@ -908,12 +913,12 @@ void compare_t(Ctx& c, size_t n, CSh3 x, CSh3 y, Sh3 eq, Sh3 gt) {
     for (int q = 0; q < 3; q++) c.nonce[PAIR0 + q] += (unsigned long long)(L + 1) * a.C + a.Cp;
 }
 
-// quicksort's compare of the rows idx[0..n) with their segments' heads
+// quicksort's compare of the rows at positions idx[0..n) with their segments' heads
 // (quicksort.h:120-150): _compare's calls on the gathered rows, of which only
 // the opened gt bits are written. The gathered copies, the eq and gt shares
 // and the opened column that separate steps pass on are 400 bytes a row.
 template <typename T>
-void qs_compare_t(Ctx& c, size_t n, CSh3 rows, const uint32_t* idx, const int32_t* head, uint8_t* cb) {
+void qs_compare_t(Ctx& c, size_t n, CSh3 rows, const uint32_t* ord, const uint32_t* idx, const int32_t* head, uint8_t* cb) {
     constexpr int W = sizeof(T);
     constexpr int L = cmp_levels<W>();
     CmpArgs<T> a{};
@@ -921,6 +926,7 @@ void qs_compare_t(Ctx& c, size_t n, CSh3 rows, const uint32_t* idx, const int32_
         a.key[j] = (const T*)rows.p[j];
         a.pair[j] = c.stream_arg(PAIR0 + j);
     }
+    a.ord = ord;
     a.idx = idx;
     a.head = head;
     a.cb = cb;
@@ -1221,9 +1227,10 @@ void op_compare(Ctx& c, int w, size_t n, CSh3 x, CSh3 y, Sh3 eq, Sh3 gt) {
     else throw std::invalid_argument("compare supports 4, 8 and 16-byte keys");
 }
 
-void op_qs_compare(Ctx& c, int w, size_t n, CSh3 rows, const uint32_t* idx, const int32_t* head, uint8_t* cb) {
-    if (w == 16) qs_compare_t<unsigned __int128>(c, n, rows, idx, head, cb);
-    else if (w == 8) qs_compare_t<unsigned long long>(c, n, rows, idx, head, cb);
+void op_qs_compare(Ctx& c, int w, size_t n, CSh3 rows, const uint32_t* ord, const uint32_t* idx, const int32_t* head,
+                   uint8_t* cb) {
+    if (w == 16) qs_compare_t<unsigned __int128>(c, n, rows, ord, idx, head, cb);
+    else if (w == 8) qs_compare_t<unsigned long long>(c, n, rows, ord, idx, head, cb);
     else throw std::invalid_argument("quicksort rows are 8 or 16 bytes");
 }
 void op_equal(Ctx& c, int w, size_t n, CSh3 x, CSh3 y, Sh3 eq) {

@@ -17,9 +17,9 @@
 //  * relative t > Z receives W(t): row t when c_t = 1, else W(Z_t) — Lomuto
 //    swaps the row at the front of its "greater" run into position t when the
 //    zero at t arrives, and no later swap reaches a position beyond Z.
-// A round is: a scan for segment heads and the ranks of the non-pivots, a
-// gather of the compared rows, the compare and open, a scan of the zero
-// flags, and one gather that moves every row to its new position.
+// A round is: a scan for segment heads and the ranks of the non-pivots, the
+// compare with the opened bits, a scan of the zero flags, and one gather that
+// moves every row's index to its new position.
 #include <algorithm>
 
 #include "launch.cuh"
@@ -244,10 +244,11 @@ __global__ void k_qs_seg(QsRound a) {
     }
 }
 
-// every row to its position after the round's partitions; new pivots marked
-template <int PW>
-__global__ void k_qs_move(QsRound a, CSh3 P, Sh3 NP) {
-    using V = typename std::conditional<PW == 16, uint4, unsigned long long>::type;
+// every position's row after the round's partitions; new pivots marked. Rows
+// stay where they are until the last round (k_qs_rows): a round moves their
+// 4-byte indices, not 96 bytes of shares read and written (2^22 int64 rows: the
+// rounds 16.0 and 12.5 ms).
+__global__ void k_qs_move(QsRound a, const uint32_t* ord, uint32_t* nord) {
     for (unsigned long long p = gtid(); p < a.n; p += gstride()) {
         const uint32_t h = (uint32_t)a.head[p];
         const uint32_t t = (uint32_t)p - h;
@@ -276,10 +277,24 @@ __global__ void k_qs_move(QsRound a, CSh3 P, Sh3 NP) {
                 if (added) atomicAdd(a.npiv, added);
             }
         }
+        nord[p] = ord[src];
+    }
+}
+
+// the rows in their final order
+template <int PW>
+__global__ void k_qs_rows(uint32_t n, const uint32_t* ord, CSh3 P, Sh3 NP) {
+    using V = typename std::conditional<PW == 16, uint4, unsigned long long>::type;
+    for (unsigned long long p = gtid(); p < n; p += gstride()) {
+        const uint32_t src = ord[p];
 #pragma unroll
         for (int j = 0; j < 3; j++)
             reinterpret_cast<V*>(NP.p[j])[p] = reinterpret_cast<const V*>(P.p[j])[src];
     }
+}
+
+__global__ void k_qs_iota(uint32_t n, uint32_t* ord) {
+    for (unsigned long long p = gtid(); p < n; p += gstride()) ord[p] = (uint32_t)p;
 }
 
 template <int PW>
@@ -287,7 +302,8 @@ void quicksort_rounds(Ctx& c, size_t n, Sh3 P) {
     const uint32_t chunks = (uint32_t)ceil_div(n, (size_t)kQsChunk);
     Scratch pivb(c, n * 4), headb(c, n * 4), idxb(c, n * 4), cbb(c, n), gzb(c, n * 4), zsegb(c, n * 4),
         sendb(c, n * 4), zposb(c, n * 4), psb(c, chunks * 4), pmb(c, chunks * 4), npb(c, 4);
-    Scratch npbuf(c, 3 * n * PW);
+    Scratch npbuf(c, 3 * n * PW), ordb(c, n * 4), ord2b(c, n * 4);
+    uint32_t *ord = ordb.as<uint32_t>(), *nord = ord2b.as<uint32_t>();  // row at each position
     QsRound a;
     a.n = (uint32_t)n;
     a.chunks = chunks;
@@ -309,13 +325,16 @@ void quicksort_rounds(Ctx& c, size_t n, Sh3 P) {
         return s;
     };
     auto cc = [](Sh3 s) { return CSh3{{s.p[0], s.p[1], s.p[2]}}; };
-    Sh3 cur = P, nxt = split(npbuf, n);
+    const Sh3 nxt = split(npbuf, n);
     // pivots: position 0 only
     ORQ_CUDA_CHECK(cudaMemsetAsync(a.piv, 0xff, n * 4, c.stream));
     ORQ_CUDA_CHECK(cudaMemsetAsync(a.piv, 0, 4, c.stream));
     uint32_t num_pivots = 1;
     ORQ_CUDA_CHECK(cudaMemcpyAsync(a.npiv, &num_pivots, 4, cudaMemcpyHostToDevice, c.stream));
     const unsigned gg = plain_grid(c, n);
+    k_qs_iota<<<gg, 256, 0, c.stream>>>((uint32_t)n, ord);
+    ORQ_CUDA_CHECK(cudaGetLastError());
+    c.kernels_launched++;
     for (size_t round = 0; num_pivots < n; round++) {
         if (round > 4 * n + 64) throw std::runtime_error("quicksort did not converge");
         const uint32_t size = (uint32_t)(n - num_pivots);
@@ -328,24 +347,26 @@ void quicksort_rounds(Ctx& c, size_t n, Sh3 P) {
             c.kernels_launched += 3;
         }
         // reduced._compare(pivot): gt = row > pivot, opened
-        op_qs_compare(c, PW, size, cc(cur), a.idx, a.head, a.cb);
+        op_qs_compare(c, PW, size, cc(P), ord, a.idx, a.head, a.cb);
         {
             ProfScope ps(c, "quicksort_round", 0.0);
             k_qs_part<1><<<chunks, kQsThreads, 0, c.stream>>>(a);
             k_qs_top<<<1, kQsThreads, 0, c.stream>>>(a);
             k_qs_zeros<<<chunks, kQsThreads, 0, c.stream>>>(a);
             k_qs_seg<<<gg, 256, 0, c.stream>>>(a);
-            k_qs_move<PW><<<gg, 256, 0, c.stream>>>(a, cc(cur), nxt);
+            k_qs_move<<<gg, 256, 0, c.stream>>>(a, ord, nord);
             ORQ_CUDA_CHECK(cudaGetLastError());
             c.kernels_launched += 5;
         }
-        std::swap(cur, nxt);
+        std::swap(ord, nord);
         ORQ_CUDA_CHECK(cudaMemcpyAsync(&num_pivots, a.npiv, 4, cudaMemcpyDeviceToHost, c.stream));
         ORQ_CUDA_CHECK(cudaStreamSynchronize(c.stream));
     }
-    if (cur.p[0] != P.p[0])
-        for (int j = 0; j < 3; j++)
-            ORQ_CUDA_CHECK(cudaMemcpyAsync(P.p[j], cur.p[j], n * PW, cudaMemcpyDeviceToDevice, c.stream));
+    k_qs_rows<PW><<<gg, 256, 0, c.stream>>>((uint32_t)n, ord, cc(P), nxt);
+    ORQ_CUDA_CHECK(cudaGetLastError());
+    c.kernels_launched++;
+    for (int j = 0; j < 3; j++)
+        ORQ_CUDA_CHECK(cudaMemcpyAsync(P.p[j], nxt.p[j], n * PW, cudaMemcpyDeviceToDevice, c.stream));
     c.check_device_error();
 }
 

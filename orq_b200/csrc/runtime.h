@@ -262,8 +262,9 @@ void op_radix_sort_batch(Ctx& c, int kw, int count, const size_t* n, void* const
 
 // ---- compare circuit and bitonic sort (cmp.cu) ----
 void op_compare(Ctx& c, int w, size_t n, CSh3 x, CSh3 y, Sh3 eq, Sh3 gt);
-// rows idx[k] against rows head[idx[k]], opened gt bits to cb[idx[k]]
-void op_qs_compare(Ctx& c, int w, size_t n, CSh3 rows, const uint32_t* idx, const int32_t* head, uint8_t* cb);
+// the row at position q = idx[k] (rows[ord[q]]) against the one at head[q], opened gt bits to cb[q]
+void op_qs_compare(Ctx& c, int w, size_t n, CSh3 rows, const uint32_t* ord, const uint32_t* idx, const int32_t* head,
+                   uint8_t* cb);
 void op_bitonic_sort(Ctx& c, int w, size_t n, Sh3 key, bool desc);
 void op_equal(Ctx& c, int w, size_t n, CSh3 x, CSh3 y, Sh3 eq);
 void op_not1(Ctx& c, int w, size_t n, CSh3 x, Sh3 y);
