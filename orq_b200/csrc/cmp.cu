@@ -13,6 +13,7 @@
 // in registers.
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -1010,18 +1011,19 @@ void bitonic_t(Ctx& c, int count, const size_t* n, const Sh3* keys, const int* d
     std::vector<uint32_t> toff(items.size() + 1, 0);
     for (size_t i = 0; i < items.size(); i++) toff[i + 1] = toff[i] + (uint32_t)ceil_div(items[i].m, a.np);
     const size_t ib = items.size() * sizeof(BitonicItem), tb = toff.size() * 4;
-    Scratch bar(c, 4), table(c, items.size() > 1 ? ib + tb : 16);
+    std::unique_ptr<Scratch> table;
     if (items.size() > 1) {
+        table.reset(new Scratch(c, ib + tb));
         uint8_t* h = (uint8_t*)c.batch_table(ib + tb);
         std::memcpy(h, items.data(), ib);
         std::memcpy(h + ib, toff.data(), tb);
-        ORQ_CUDA_CHECK(cudaMemcpyAsync(table.p, h, ib + tb, cudaMemcpyHostToDevice, c.stream));
+        ORQ_CUDA_CHECK(cudaMemcpyAsync(table->p, h, ib + tb, cudaMemcpyHostToDevice, c.stream));
         ORQ_CUDA_CHECK(cudaEventRecord(c.batch.read, c.stream));
-        a.items = table.as<BitonicItem>();
-        a.toff = reinterpret_cast<const uint32_t*>(table.as<uint8_t>() + ib);
+        a.items = table->as<BitonicItem>();
+        a.toff = reinterpret_cast<const uint32_t*>(table->as<uint8_t>() + ib);
     }
-    a.bar = bar.as<uint32_t>();
-    ORQ_CUDA_CHECK(cudaMemsetAsync(bar.p, 0, 4, c.stream));
+    a.bar = c.grid_bar();
+    ORQ_CUDA_CHECK(cudaMemsetAsync(a.bar, 0, 4, c.stream));
     constexpr size_t per_warp = (size_t)(L + 3) * 3 * (32 * W / 4) * 4;
     const size_t smem = kAesSmemBytes + bitonic_bufs<W>() * (a.np / 32) * per_warp;
     const auto kern = &k_bitonic<T>;

@@ -1126,7 +1126,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     // not for the generator, 24 (44 permutations of 100003 rows 4.8 and 4.0 ms,
     // of 262143 7.4 and 6.4; of 2^19 rows, M = 2^20, 11.6 and 11.4). W is
     // rounded so that the last wave of lists is full.
-    const uint32_t gen_sms = (uint32_t)std::max(1, c.num_sms - (bitsw <= 19 ? 24 : 3)), gen_warps = gen_sms * (kGenThreads / 32);
+    const uint32_t gen_sms = (uint32_t)std::max(1, c.num_sms - (bitsw <= 19 ? std::min(24, c.num_sms / 6) : 3)), gen_warps = gen_sms * (kGenThreads / 32);
     const double want = std::clamp(per_perm * count / 8.0, 2.0, 64.0);
     const uint32_t waves = std::max(1u, (uint32_t)(want * kListsPerBuf / gen_warps));
     const uint32_t W = std::max(2u, waves * gen_warps / kListsPerBuf);

@@ -394,7 +394,7 @@ void op_radix_bits(Ctx& c, int PW, size_t n, Sh3 P, int bits, bool invert_last) 
     const uint32_t chunk = (uint32_t)(ceil_div(ceil_div(n, sms), 64) * 64);
     const uint32_t grid = (uint32_t)ceil_div(n, chunk);
     const size_t n4 = ceil_div(n, 4) * 4;  // 16-byte aligned share arrays
-    Scratch recs(c, 2 * n * kRec), f1b(c, 3 * n4 * 4), part(c, (size_t)6 * grid * 4), bar(c, 4);
+    Scratch recs(c, 2 * n * kRec), f1b(c, 3 * n4 * 4), part(c, (size_t)6 * grid * 4);
     BitsArgs a;
     for (int j = 0; j < 3; j++) {
         a.P[j] = P.p[j];
@@ -407,7 +407,7 @@ void op_radix_bits(Ctx& c, int PW, size_t n, Sh3 P, int bits, bool invert_last) 
     a.rec[0] = recs.as<uint8_t>();
     a.rec[1] = a.rec[0] + n * kRec;
     a.part = part.as<uint32_t>();
-    a.bar = bar.as<uint32_t>();
+    a.bar = c.grid_bar();
     a.err = c.d_err;
     a.ch4 = chunks_of((unsigned long long)n * 4);
     a.chx = chunks_of((unsigned long long)n * PW);
@@ -420,7 +420,7 @@ void op_radix_bits(Ctx& c, int PW, size_t n, Sh3 P, int bits, bool invert_last) 
         used.push_back(next_perm(c, n));
         for (int g = 0; g < 3; g++) a.inv[3 * b + g] = used.back().inv[g];
     }
-    ORQ_CUDA_CHECK(cudaMemsetAsync(bar.p, 0, 4, c.stream));
+    ORQ_CUDA_CHECK(cudaMemsetAsync(a.bar, 0, 4, c.stream));
     {
         const double el = (double)n * bits;
         ProfScope ps(c, "radix_bits", el * (24.0 + 24.0 + 3 * (4.0 + 6.0 * PW + 24.0)),

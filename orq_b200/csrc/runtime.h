@@ -120,6 +120,7 @@ struct FyRes {
     void* hst = nullptr;  // pinned scan states, [group][batch]
 };
 
+constexpr size_t kErrBytes = 256;  // the error word, and the grid barriers' counter in a line of its own
 struct Ctx {
     int device = 0;
     int nparties = 3;  // 3: replicated 3PC; 2: Beaver 2PC; 4: Fantastic-4PC
@@ -138,6 +139,9 @@ struct Ctx {
     // (they skip the access); checked at the synchronous points.
     int* d_err = nullptr;
     void check_device_error();
+    // arrival counter of the grid barriers (the cooperative kernels of a runtime
+    // follow each other on its stream, so one serves all)
+    uint32_t* grid_bar() const { return reinterpret_cast<uint32_t*>(d_err) + 32; }
     FyRes fy;
     BatchTable batch;
     void* batch_table(size_t bytes);  // the staging, once its last copy is done
