@@ -86,6 +86,8 @@ def _rows3(t):
     pointer and the row stride: indexing a tensor costs more than a small
     call's launch (1000-element AND: 25 us a call with nine row views, 15
     without)."""
+    if t.shape[0] < 3:
+        raise IndexError("a shared vector has three share rows")
     b = t.data_ptr()
     if not b:  # an empty tensor
         return 0, 0, 0
