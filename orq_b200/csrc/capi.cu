@@ -588,6 +588,16 @@ int orqcu_reserve_permutations(orqcu_runtime* rt, size_t n, size_t count) {
     });
 }
 
+int orqcu_runtime_tune_permutations(orqcu_runtime* rt, int buffers, unsigned chunks) {
+    return guard([&] {
+        need_rt(rt);
+        need(buffers >= -1024 && buffers <= 1024, "buffers must lie in [-1024, 1024]");
+        need(chunks <= 1u << 16, "chunks must be at most 65536");
+        rt->ctx.fy_tune.buffers = buffers;
+        rt->ctx.fy_tune.chunks = chunks;
+    });
+}
+
 int orqcu_next_permutation(orqcu_runtime* rt, size_t n, int32_t* const perm_dev[3]) {
     return guard([&] {
         need_rt(rt);

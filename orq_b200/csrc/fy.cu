@@ -574,7 +574,9 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_emit(FyScanArgs a) {
 // against the used counts; from the first permutation of a group whose start
 // was wrong, the rest are run again from the corrected start (each pass
 // fixes at least that one). A permutation needing more than `max_chunks`
-// chunks sets `overflow`, and the general chain redoes everything.
+// chunks sets `overflow`, and the pass is run again with twice as many (the
+// chain below cannot take these: a run of it holds 2048 draws, of which more
+// than kRunUnc are uncertain when M is that small).
 constexpr uint32_t kSmallChunk = 8192;  // draws per chunk
 constexpr int kSmallThreads = 512;
 // above it predictions fail too often (at 2^16 one in 75 permutations) and a
@@ -582,6 +584,7 @@ constexpr int kSmallThreads = 512;
 // rows took 20.2 ms with this path and takes 19.5 with the chain
 constexpr uint32_t kSmallMaxM = 1u << 15;
 constexpr uint32_t kChunksPerBuffer = (1u << 20) / kSmallChunk;  // 128
+constexpr uint32_t kSmallChunkLimit = (1u << 31) / kSmallChunk;   // draws are counted in 32 bits
 constexpr size_t kSmallSmem = (size_t)kAesSmemBytes + kSmallChunk * 4;
 constexpr int kSmallEach = kSmallChunk / kSmallThreads;  // 16: draws a thread decides at most at once
 
@@ -1042,7 +1045,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     if ((1ull << bitsw) <= kSmallMaxM) {
         // every permutation of every group at once from predicted start
         // buffers, corrected pass by pass (k_fy_small)
-        const uint32_t bhat = 1u + (uint32_t)(M * H / (double)(1u << 20));
+        const uint32_t bhat = (uint32_t)std::max(1, 1 + (int)(M * H / (double)(1u << 20)) + c.fy_tune.buffers);
         std::vector<uint32_t> hstart(3 * count), hused(3 * count);
         for (int g = 0; g < 3; g++)
             for (size_t m = 0; m < count; m++) hstart[g * count + m] = (uint32_t)m * bhat;
@@ -1060,13 +1063,12 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         sa.n = (uint32_t)n;
         sa.mask = mask;
         sa.count = (uint32_t)count;
-        sa.max_chunks = (bhat + 6) * kChunksPerBuffer;
+        sa.max_chunks = c.fy_tune.chunks ? c.fy_tune.chunks : (bhat + 6) * kChunksPerBuffer;
         sa.start = d_start.as<uint32_t>();
         sa.used = d_used.as<uint32_t>();
         sa.acc = acc.as<uint32_t>();
         sa.overflow = ovf.as<uint32_t>();
-        bool ok = false;
-        for (int pass = 0; pass < 64; pass++) {
+        for (bool again = true; again;) {
             ORQ_CUDA_CHECK(cudaMemcpyAsync(d_start.p, hstart.data(), hstart.size() * 4, cudaMemcpyHostToDevice, gs));
             {
                 ProfScope ps(c, "fy_small", 0.0, 0.0, gs);
@@ -1078,11 +1080,18 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
             ORQ_CUDA_CHECK(cudaMemcpyAsync(hused.data(), d_used.p, hused.size() * 4, cudaMemcpyDeviceToHost, gs));
             ORQ_CUDA_CHECK(cudaMemcpyAsync(&overflow, ovf.p, 4, cudaMemcpyDeviceToHost, gs));
             ORQ_CUDA_CHECK(cudaStreamSynchronize(gs));
-            if (overflow) break;
+            if (overflow) {
+                // the same pass with room for more draws (some `used` are not set)
+                if (sa.max_chunks > kSmallChunkLimit / 2)
+                    throw std::runtime_error("permutation generation did not converge");
+                sa.max_chunks *= 2;
+                ORQ_CUDA_CHECK(cudaMemsetAsync(ovf.p, 0, 4, gs));
+                continue;
+            }
             // permutations before m0[g] are verified, and so is m0[g]'s start;
             // the first one whose assumed start differs from the true one is
-            // where the next pass begins
-            bool again = false;
+            // where the next pass begins (so every pass verifies at least one)
+            again = false;
             for (int g = 0; g < 3; g++) {
                 uint32_t* st = hstart.data() + g * count;
                 const uint32_t* us = hused.data() + g * count;
@@ -1099,22 +1108,14 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
                     for (size_t k = m; k < count; k++) st[k] = expect + (uint32_t)(k - m) * bhat;
                 }
             }
-            if (!again) {
-                ok = true;
-                break;
-            }
         }
-        if (ok) {
-            for (int g = 0; g < 3; g++)
-                c.nonce[G01 + g] += 4ull * (hstart[g * count + count - 1] + hused[g * count + count - 1]);
-            for (; fin_next < 3 * count; fin_next += fin_p) launch_fin(fin_next, std::min(3 * count, fin_next + fin_p));
-            ORQ_CUDA_CHECK(cudaEventRecord(R.fin_done, fs));
-            ORQ_CUDA_CHECK(cudaStreamWaitEvent(c.stream, R.fin_done, 0));
-            c.check_device_error();
-            return;
-        }
-        // a permutation ran past max_chunks (or the passes did not settle):
-        // the general chain below redoes all of them (no nonce was consumed)
+        for (int g = 0; g < 3; g++)
+            c.nonce[G01 + g] += 4ull * (hstart[g * count + count - 1] + hused[g * count + count - 1]);
+        for (; fin_next < 3 * count; fin_next += fin_p) launch_fin(fin_next, std::min(3 * count, fin_next + fin_p));
+        ORQ_CUDA_CHECK(cudaEventRecord(R.fin_done, fs));
+        ORQ_CUDA_CHECK(cudaStreamWaitEvent(c.stream, R.fin_done, 0));
+        c.check_device_error();
+        return;
     }
 
     // Buffers are generated `W` at a time per group into a ring of kRing * W

@@ -120,6 +120,13 @@ struct FyRes {
     void* hst = nullptr;  // pinned scan states, [group][batch]
 };
 
+// What the permutation generator tries first. The permutations and the nonces
+// they use do not depend on it, only the passes that it takes.
+struct FyTune {
+    int buffers = 0;      // small permutations: added to the predicted getNext buffers of each
+    uint32_t chunks = 0;  // small permutations: chunks of draws a pass has room for (0: by the prediction)
+};
+
 constexpr size_t kErrBytes = 256;  // the error word, and the grid barriers' counter in a line of its own
 struct Ctx {
     int device = 0;
@@ -143,6 +150,7 @@ struct Ctx {
     // follow each other on its stream, so one serves all)
     uint32_t* grid_bar() const { return reinterpret_cast<uint32_t*>(d_err) + 32; }
     FyRes fy;
+    FyTune fy_tune;
     BatchTable batch;
     void* batch_table(size_t bytes);  // the staging, once its last copy is done
     void release_batch();

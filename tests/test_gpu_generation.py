@@ -1,0 +1,41 @@
+"""The permutation generator's corrections: what it does when its first guess
+is wrong. The permutations and the nonces must be those of the C restatement
+whatever was guessed first."""
+import pytest
+
+from replay import same
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def orq(cuda_lib, oracle_lib):
+    import orq_b200
+
+    return orq_b200
+
+
+def check_permutations(orq, rt, n, count, seed):
+    from oracle.oracle import G01, Oracle
+
+    o = Oracle(seed)
+    rt.reserve_permutations(n, count)
+    for m in range(count):
+        got = rt.next_permutation(n).cpu().numpy()
+        for g in range(3):
+            want, _ = o.gen_perm(G01 + g, n)
+            assert same(got[g], want), (m, g)
+    for g in range(3):
+        assert rt.nonce(orq.STREAM_G01 + g) == o.nonce(G01 + g)
+
+
+# wrong predicted starts (the second of 70 permutations on: a pass verifies one
+# more of each group, more passes than 64), and room for too few draws in the
+# first pass, at the smallest sizes, at a chunk's 8192 draws and at the largest
+@pytest.mark.parametrize("n,count,buffers,chunks", [(1, 70, 1, 0), (300, 70, 2, 0), (1000, 3, -1, 0), (32767, 4, 1, 0),
+                                                    (1, 1, 0, 1), (63, 2, 0, 1), (2000, 3, 0, 1), (5000, 2, 1, 1),
+                                                    (32767, 3, 0, 3)])
+def test_small_permutations_from_wrong_first_guesses(orq, n, count, buffers, chunks):
+    rt = orq.Runtime(seed=17)
+    rt.tune_permutations(buffers=buffers, chunks=chunks)
+    check_permutations(orq, rt, n, count, 17)
