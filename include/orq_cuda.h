@@ -172,10 +172,12 @@ int orqcu_prefix_sum_a_noalloc(orqcu_runtime* rt, int width, size_t n, void* con
  * `count` sharded permutations of size n ahead of use. Synchronous. */
 int orqcu_reserve_permutations(orqcu_runtime* rt, size_t n, size_t count);
 /* What the generator of this runtime tries first, for tests of its corrections:
- * `buffers` is added to the getNext buffers a small permutation is predicted
- * to use, `chunks` is how many chunks of 8192 draws a first pass gives each (0:
- * by the prediction). The permutations and the nonces used stay the same. */
-int orqcu_runtime_tune_permutations(orqcu_runtime* rt, int buffers, unsigned chunks);
+ * `width` is the half width of the chain's threshold windows in standard
+ * deviations (6 otherwise), `buffers` is added to the getNext buffers a small
+ * permutation is predicted to use, `chunks` is how many chunks of 8192 draws a
+ * first pass gives each (0: by the prediction). The permutations and the nonces
+ * used stay the same. */
+int orqcu_runtime_tune_permutations(orqcu_runtime* rt, double width, int buffers, unsigned chunks);
 /* Pop the next sharded permutation (PermutationManager::getNext) and copy its
  * three group-local permutations ({0,1},{0,2},{1,2}; gen_perm's output,
  * hm_sharded_permutation_generator.h:70-108) to perm_dev[g]. */

@@ -229,9 +229,10 @@ class Runtime:
         """PermutationManager::reserve (permutation_manager.h:102-181)."""
         _check(self.lib.orqcu_reserve_permutations(self.h, ctypes.c_size_t(n), ctypes.c_size_t(count)))
 
-    def tune_permutations(self, buffers: int = 0, chunks: int = 0):
+    def tune_permutations(self, width: float = 6.0, buffers: int = 0, chunks: int = 0):
         """What the generator tries first (tests of its corrections)."""
-        _check(self.lib.orqcu_runtime_tune_permutations(self.h, buffers, ctypes.c_uint(chunks)))
+        _check(self.lib.orqcu_runtime_tune_permutations(self.h, ctypes.c_double(width), buffers,
+                                                        ctypes.c_uint(chunks)))
 
     def next_permutation(self, n: int):
         """The three group-local permutations of the next sharded permutation."""

@@ -588,11 +588,13 @@ int orqcu_reserve_permutations(orqcu_runtime* rt, size_t n, size_t count) {
     });
 }
 
-int orqcu_runtime_tune_permutations(orqcu_runtime* rt, int buffers, unsigned chunks) {
+int orqcu_runtime_tune_permutations(orqcu_runtime* rt, double width, int buffers, unsigned chunks) {
     return guard([&] {
         need_rt(rt);
+        need(width >= 0.25 && width <= 1000.0, "width must lie in [0.25, 1000]");
         need(buffers >= -1024 && buffers <= 1024, "buffers must lie in [-1024, 1024]");
         need(chunks <= 1u << 16, "chunks must be at most 65536");
+        rt->ctx.fy_tune.width = width;
         rt->ctx.fy_tune.buffers = buffers;
         rt->ctx.fy_tune.chunks = chunks;
     });

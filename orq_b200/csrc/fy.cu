@@ -28,7 +28,6 @@
 //    parallel (the gather index of an application; the permutation itself,
 //    which only inverse applications read, is derived when one asks for it).
 #include <algorithm>
-#include <cstdlib>
 #include <cstring>
 #include <memory>
 
@@ -1304,10 +1303,8 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     };
     // A threshold outside its window (6 deviations: about once in 1e7
     // permutations) shows up as `bad`: nothing has been consumed yet, so the
-    // chain runs again with wider windows. ORQ_FY_WIDTH sets the first width
-    // (tests narrow it).
-    const char* we = std::getenv("ORQ_FY_WIDTH");
-    double width = we ? std::clamp(std::atof(we), 0.25, 6.0) : 6.0;
+    // chain runs again with wider windows.
+    double width = c.fy_tune.width;
     while (!run_chain(width)) {
         width *= 1.5;
         if (width > 20.0) throw std::runtime_error("permutation generation did not converge");

@@ -123,6 +123,7 @@ struct FyRes {
 // What the permutation generator tries first. The permutations and the nonces
 // they use do not depend on it, only the passes that it takes.
 struct FyTune {
+    double width = 6.0;   // chain: half width of the threshold windows in standard deviations
     int buffers = 0;      // small permutations: added to the predicted getNext buffers of each
     uint32_t chunks = 0;  // small permutations: chunks of draws a pass has room for (0: by the prediction)
 };

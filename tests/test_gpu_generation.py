@@ -39,3 +39,25 @@ def test_small_permutations_from_wrong_first_guesses(orq, n, count, buffers, chu
     rt = orq.Runtime(seed=17)
     rt.tune_permutations(buffers=buffers, chunks=chunks)
     check_permutations(orq, rt, n, count, 17)
+
+
+# windows too narrow for the thresholds: every chain starts over with wider ones
+@pytest.mark.parametrize("n,count", [(65536, 4), (131071, 3), (262143, 2), (524288, 2), (1048577, 1)])
+def test_chain_from_windows_too_narrow(orq, n, count):
+    rt = orq.Runtime(seed=5)
+    rt.tune_permutations(width=0.25)
+    check_permutations(orq, rt, n, count, 5)
+
+
+def test_the_environment_does_not_reach_the_generator(orq, monkeypatch):
+    def launches():
+        rt = orq.Runtime(seed=5)
+        rt.reserve_permutations(100003, 2)  # (loads the kernels, fills the pool)
+        rt.reseed(5)
+        k = rt.kernels_launched()
+        rt.reserve_permutations(100003, 2)
+        return rt.kernels_launched() - k
+
+    want = launches()
+    monkeypatch.setenv("ORQ_FY_WIDTH", "none")
+    assert launches() < 1.5 * want  # (a second chain doubles them)
