@@ -194,9 +194,12 @@ struct FyScanArgs {
 // past the place where the permutation ends (x = n - i values remain; they
 // take about M (ln x + 4) draws or fewer with probability 0.98; a step that
 // stops short is continued by the next). Integer arithmetic, so that every
-// kernel of the step finds the same number.
+// kernel of the step finds the same number. `bad` is no part of it: another
+// CTA's classification may set it while this one's warps read the state, and
+// warps with different numbers would take sums of shared memory that the others
+// have not written, and store by them.
 __device__ __forceinline__ uint32_t fy_step_tiles(const FyScanArgs& a, const FyState& s) {
-    if (s.done || s.bad || s.pos >= a.limit) return 0;
+    if (s.done || s.pos >= a.limit) return 0;
     const uint32_t lg = 32 - __clz(a.n - s.i);                                // log2(x) rounded up
     // M in tiles (kRuns * rl * 2048 draws each), times ln x + 4 in 16 fractional bits
     const unsigned long long span =
@@ -367,7 +370,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_fy_resolve(FyScanArgs a) {
     __shared__ uint32_t red[33];
     __shared__ uint32_t s_take, s_end, s_call;
     const FyState s = *a.state;
-    const uint32_t nt = fy_step_tiles(a, s);
+    const uint32_t nt = s.bad ? 0 : fy_step_tiles(a, s);  // (nothing else runs that sets it)
     const uint32_t tid = threadIdx.x;
     if (!nt) {
         if (tid == 0) *a.seg = FySeg{0, s.m};

@@ -61,3 +61,18 @@ def test_the_environment_does_not_reach_the_generator(orq, monkeypatch):
     want = launches()
     monkeypatch.setenv("ORQ_FY_WIDTH", "none")
     assert launches() < 1.5 * want  # (a second chain doubles them)
+
+
+@pytest.mark.parametrize("n,count", [(65536, 3), (300001, 2)])
+def test_chain_after_lists_that_overflow(orq, n, count):
+    """windows so wide that runs of the classification hold more uncertain
+    draws than they keep: whatever becomes of that call, the next ones are right"""
+    rt = orq.Runtime(seed=23)
+    rt.tune_permutations(width=1000.0)
+    try:
+        rt.reserve_permutations(n, 1)
+    except orq.OrqError:
+        pass
+    rt.reseed(23)
+    rt.tune_permutations()
+    check_permutations(orq, rt, n, count, 23)
