@@ -51,6 +51,9 @@ constexpr uint32_t kPieceUnc = 8192;       // uncertain draws k_fy_resolve holds
 constexpr int kGenThreads = 512;
 constexpr int kTabEntries = 520;           // U[256], V[257] of one chunk, padded
 
+constexpr uint32_t kMissed = 1;    // a window missed its threshold
+constexpr uint32_t kOverflow = 2;  // more uncertain draws in a run than it keeps
+
 // Scan state of one group's chain. `pos` counts tiles and `start` buffers from
 // the chain's first buffer.
 struct FyState {
@@ -59,7 +62,7 @@ struct FyState {
     uint32_t m;                // index of the current permutation
     uint32_t i;                // accepted so far
     uint32_t done;             // every permutation is complete
-    uint32_t bad;              // a window missed its threshold or a list overflowed
+    uint32_t bad;              // kMissed, kOverflow
 };
 
 // GCM's counter block is (nonce, 0, BE32(j + 2)): inside a chunk of 65536
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_classify(FyScanArgs a) {
             k += __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
         }
         if (nu > kRunUnc) {
-            if (lane == 0) atomicOr(&a.state->bad, 2u);
+            if (lane == 0) atomicOr(&a.state->bad, kOverflow);
             nu = kRunUnc;
         }
         if (lane == 0) {
@@ -536,7 +539,7 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_emit(FyScanArgs a) {
         const long long T = (long long)a.n - 1 - out;
         // past the permutation's end (T < 0) nothing may be certain
         const bool good = T >= 0 ? (T >= r.lo && T <= r.hi) : r.cnt == r.unc;
-        if (!good && lane == 0) atomicOr(&a.state->bad, 1u);
+        if (!good && lane == 0) atomicOr(&a.state->bad, kMissed);
         const uint32_t* cand = a.cand + ((size_t)t * kRuns + w) * (a.rl * kListDraws);
         for (uint32_t b = 0; b < r.cnt; b += 256) {
             uint32_t v[8];
@@ -1173,7 +1176,8 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     prep_aes_kernel(k_fy_gen);
     FyState* hst = static_cast<FyState*>(R.hst);
 
-    const auto run_chain = [&](double width) -> bool {
+    // runs the chain; what went wrong, if anything (kMissed, kOverflow)
+    const auto run_chain = [&](double width) -> uint32_t {
     FyScanArgs sa[3];
     for (int g = 0; g < 3; g++) {
         FyScanArgs& x = sa[g];
@@ -1224,7 +1228,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         ORQ_CUDA_CHECK(cudaEventRecord(R.st_ev[g][k], ss[g]));
         q.head++;
     };
-    bool bad = false;
+    uint32_t bad = 0;
     // waits for the oldest batch of steps queued for g
     const auto read_back = [&](int g) {
         Group& q = G[g];
@@ -1236,7 +1240,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         q.start = z.start;
         q.m = z.m;
         q.done = z.done != 0;
-        bad = bad || z.bad;
+        bad |= z.bad;
         const size_t mmin = std::min({G[0].m, G[1].m, G[2].m});
         // the accepted offsets of these permutations precede the states read
         if (!bad && mmin < count)
@@ -1299,18 +1303,20 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     ORQ_CUDA_CHECK(cudaMemcpyAsync(hst, state.p, 3 * sizeof(FyState), cudaMemcpyDeviceToHost, gs));
     ORQ_CUDA_CHECK(cudaStreamSynchronize(gs));
     for (int g = 0; g < 3; g++) {
-        bad = bad || hst[g].bad;
+        bad |= hst[g].bad;
         G[g].start = hst[g].start;
     }
-    return !bad;
+    return bad;
     };
     // A threshold outside its window (6 deviations: about once in 1e7
-    // permutations) shows up as `bad`: nothing has been consumed yet, so the
-    // chain runs again with wider windows.
+    // permutations) shows up as kMissed: nothing has been consumed yet, so the
+    // chain runs again with wider windows. Windows so wide that a run's
+    // uncertain draws overflow (a quarter of M, some 80 deviations at M = 2^16)
+    // are narrowed instead.
     double width = c.fy_tune.width;
-    while (!run_chain(width)) {
-        width *= 1.5;
-        if (width > 20.0) throw std::runtime_error("permutation generation did not converge");
+    for (int tries = 1; const uint32_t bad = run_chain(width); tries++) {
+        if (tries == 24) throw std::runtime_error("permutation generation did not converge");
+        width *= bad & kOverflow ? 0.6 : 1.5;
         ORQ_CUDA_CHECK(cudaStreamSynchronize(fs));
         ORQ_CUDA_CHECK(cudaMemsetAsync(state.p, 0, 3 * sizeof(FyState), gs));
         ORQ_CUDA_CHECK(cudaStreamSynchronize(gs));

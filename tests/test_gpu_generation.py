@@ -76,3 +76,11 @@ def test_chain_after_lists_that_overflow(orq, n, count):
     rt.reseed(23)
     rt.tune_permutations()
     check_permutations(orq, rt, n, count, 23)
+
+
+@pytest.mark.parametrize("n,count,width", [(65536, 2, 1000.0), (100003, 3, 60.0), (524287, 1, 400.0)])
+def test_chain_from_windows_too_wide(orq, n, count, width):
+    """lists that overflow are answered with narrower windows"""
+    rt = orq.Runtime(seed=29)
+    rt.tune_permutations(width=width)
+    check_permutations(orq, rt, n, count, 29)
