@@ -21,7 +21,7 @@
 //    A one-CTA scanner that replayed every draw bounded the chain before: the
 //    radix step of 2^22 rows took 418 ms and takes 280 ms, of 2^20 rows 127.6
 //    and 62.8 ms, of 100003 rows 19.0 and 12.5 ms.
-//  * fy_small (M <= 2^15, one buffer per permutation almost always):
+//  * fy_small (M <= 2^15, many of M = 2^16; one buffer per permutation almost always):
 //    every (permutation, group) in its own CTA at once from predicted start
 //    buffers, re-run from the first wrong prediction until all are verified;
 //  * fy_finalize: turns the accepted offsets into the inverse permutation in
@@ -38,7 +38,7 @@ namespace orqcu {
 namespace {
 
 // ---------------------------------------------------------------------------
-// The chain of permutations of one group (M = 2^bit_width(n) >= kChainMinM).
+// The chain of permutations of one group (M = 2^bit_width(n) >= 2^16).
 constexpr uint32_t kBufDraws = 1u << 20;   // draws per getNext buffer
 constexpr uint32_t kListDraws = 2048;      // draws behind one sparse list
 constexpr uint32_t kListCap = 256;
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_emit(FyScanArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Small permutations (M = 2^bit_width(n) <= 2^15). A permutation then takes
+// Small permutations (M = 2^bit_width(n) up to 2^16). A permutation then takes
 // d ≈ M·H_n draws (std ≈ 1.3·M) and 1 + floor(d / 2^20) getNext buffers, a
 // count that is predictable: permutation m of a group is assumed to start at
 // buffer m·b̂ of the chain, and every (permutation, group) pair runs at once,
@@ -584,10 +584,14 @@ __global__ void __launch_bounds__(kRuns * 32, 4) k_fy_emit(FyScanArgs a) {
 // than kRunUnc are uncertain when M is that small).
 constexpr uint32_t kSmallChunk = 8192;  // draws per chunk
 constexpr int kSmallThreads = 512;
-// above it predictions fail too often (at 2^16 one in 75 permutations) and a
-// repeated pass costs a whole permutation on one SM: the group-by of 60000
-// rows took 20.2 ms with this path and takes 19.5 with the chain
-constexpr uint32_t kSmallMaxM = 1u << 15;
+// Up to M = 2^15 always, at 2^16 from 18 permutations on: one permutation then
+// takes its SM 1.2 ms however few there are, and a prediction fails in one of
+// 140 to 270, which costs another pass, where the chain takes 70 to 80 us for
+// each in turn. 33000 rows, mean of 12 seeds, chain and this path: 8
+// permutations 0.92 and 1.32 ms, 20 1.71 and 1.55, 42 3.11 and 1.90, 66 4.57
+// and 2.86; 65535 rows: 1.08 and 1.49, 1.99 and 1.75, 3.62 and 2.72, 5.17 and
+// 4.07. At 2^17 a pass takes twice as long and a prediction fails twice as often.
+inline bool fy_small_path(uint64_t M, size_t count) { return M <= 1u << 15 || (M == 1u << 16 && count >= 18); }
 constexpr uint32_t kChunksPerBuffer = (1u << 20) / kSmallChunk;  // 128
 constexpr uint32_t kSmallChunkLimit = (1u << 31) / kSmallChunk;   // draws are counted in 32 bits
 constexpr size_t kSmallSmem = (size_t)kAesSmemBytes + kSmallChunk * 4;
@@ -1047,7 +1051,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     for (int g = 0; g < 3; g++) ORQ_CUDA_CHECK(cudaStreamWaitEvent(ss[g], ev_start, 0));
     ORQ_CUDA_CHECK(cudaStreamWaitEvent(fs, ev_start, 0));
 
-    if ((1ull << bitsw) <= kSmallMaxM) {
+    if (fy_small_path(1ull << bitsw, count)) {
         // every permutation of every group at once from predicted start
         // buffers, corrected pass by pass (k_fy_small)
         const uint32_t bhat = (uint32_t)std::max(1, 1 + (int)(M * H / (double)(1u << 20)) + c.fy_tune.buffers);

@@ -84,3 +84,14 @@ def test_chain_from_windows_too_wide(orq, n, count, width):
     rt = orq.Runtime(seed=29)
     rt.tune_permutations(width=width)
     check_permutations(orq, rt, n, count, 29)
+
+
+# both sides of the rule that sends permutations of M = 2^16 to the path of the
+# small ones; there, many take one launch a pass and one batch of finalizes
+@pytest.mark.parametrize("n,count", [(32768, 17), (32768, 18), (65535, 18), (50001, 66)])
+def test_many_permutations_of_medium_size(orq, n, count):
+    rt = orq.Runtime(seed=31)
+    check_permutations(orq, rt, n, count, 31)
+    k = rt.kernels_launched()
+    rt.reserve_permutations(n, count)
+    assert count < 18 or rt.kernels_launched() - k < 60
