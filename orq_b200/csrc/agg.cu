@@ -21,16 +21,15 @@ namespace orqcu {
 namespace {
 
 constexpr int kMaxAggKeys = 4;
-// A thread carries the group bits of its unit in four forms (boolean and
-// arithmetic, with and without the table restriction) across the level's
-// calls, so it needs up to 255 registers: 256 threads per CTA, one CTA per SM
-// (the AES tables take 128 KiB of shared memory).
-// Threads per CTA: the compare circuit of min / max needs 200 registers, a
-// level without one fits 128. Smaller CTAs while that spreads a level over
-// more SMs.
-template <bool MINMAX>
-constexpr int agg_threads() { return MINMAX ? 256 : 512; }
+// Threads per CTA, one CTA per SM (the AES tables take 128 KiB of shared
+// memory): the compare circuit of min / max needs 200 registers, a level without
+// one fits 128. Smaller CTAs while that spreads a level over more SMs.
 constexpr int kAggSmall = 256;
+// Kinds of level. BOOLEAN: one of boolean columns without min / max with at most
+// a unit a thread, GENERAL: any other without min / max.
+enum AggKind { AGG_GENERAL, AGG_BOOLEAN, AGG_MINMAX };
+template <AggKind KIND>
+constexpr int agg_threads() { return KIND == AGG_GENERAL ? 512 : kAggSmall; }
 constexpr int kMaxAggSpecs = 8;
 
 struct AggLevelArgs {
@@ -199,10 +198,11 @@ __device__ __forceinline__ void compare_rows(const T (&X)[E][3], const T (&Y)[E]
         for (int p = 0; p < 3; p++) Gt[k][p] = (s1[p] >> (rowbase + k)) & 1;
 }
 
-// MINMAX: whether the level has a min or max aggregation; without one the
-// compare circuit is compiled out (it holds most of the registers)
-template <int W, bool MINMAX>
-__global__ void __launch_bounds__(agg_threads<MINMAX>(), 1) k_agg_level(AggLevelArgs a) {
+// Without a min or max aggregation the compare circuit is compiled out (it holds
+// most of the registers), and in a BOOLEAN level everything arithmetic
+template <int W, AggKind KIND>
+__global__ void __launch_bounds__(agg_threads<KIND>(), 1) k_agg_level(AggLevelArgs a) {
+    constexpr bool MINMAX = KIND == AGG_MINMAX;
     using T = typename std::conditional<W == 4, uint32_t, unsigned long long>::type;
     constexpr int E = 16 / W;               // rows per unit
     constexpr int L = (W == 4) ? 5 : 6;     // bit_same rounds
@@ -220,9 +220,13 @@ __global__ void __launch_bounds__(agg_threads<MINMAX>(), 1) k_agg_level(AggLevel
         // (the stream loop stays rolled: inlined at every call of the level,
         // three AES bodies each overflowed the instruction cache, 19.2 ms for the
         // levels of a join of 2^16 and 2^18 rows, 14.0 now; each pass
-        // appends stream q and moves the others down, so K[.][q] ends up in place)
+        // appends stream q and moves the others down, so K[.][q] ends up in place.
+        // A BOOLEAN level has few calls in its code, most run in a loop, and 8
+        // warps an SM that wait for one block after the other: inlined there, three
+        // keys and a copy of 2^15 rows take 1.36 and 1.17 ms at 4 bytes, 1.54 and
+        // 1.12 at 8)
         auto next_call = [&]() {
-#pragma unroll 1
+#pragma unroll(KIND == AGG_BOOLEAN ? 3 : 1)
             for (int q = 0; q < 3; q++) {
                 const uint4 b = keystream_block_n(S, a.pair[q].rk, a.pair[q].nonce + off, u);
 #pragma unroll
@@ -422,7 +426,7 @@ __global__ void __launch_bounds__(agg_threads<MINMAX>(), 1) k_agg_level(AggLevel
                     for (int p = 0; p < 3; p++)
                         reinterpret_cast<T*>(a.b_dst[s][p])[a.reverse ? hi[k] : lo[k]] = R[k][p];
         }
-        if (a.na == 0) continue;  // uniform across the grid
+        if (KIND == AGG_BOOLEAN || a.na == 0) continue;  // uniform across the grid
         // ---- group bits as arithmetic shares (b2a_bit, replicated_3pc.h:220-251)
         T GA[E][3], JGA[E][3];
 #pragma unroll
@@ -628,10 +632,14 @@ void op_aggregate(Ctx& c, int w, size_t n, int nkeys, const void* const* keys, i
         {
             bool minmax = false;
             for (int s2 = 0; s2 < nb; s2++) minmax = minmax || bs[s2].func == AGG_MIN || bs[s2].func == AGG_MAX;
-            auto kern = w == 4 ? (minmax ? k_agg_level<4, true> : k_agg_level<4, false>)
-                               : (minmax ? k_agg_level<8, true> : k_agg_level<8, false>);
+            const bool small = units <= (unsigned long long)c.num_sms * kAggSmall;
+            // (below 128 units loading the longer code costs more: 64 rows of 4
+            // bytes 0.38 and 0.48 ms)
+            const bool boolean = small && na == 0 && units >= 128;
+            auto kern = w == 4 ? (minmax ? k_agg_level<4, AGG_MINMAX> : boolean ? k_agg_level<4, AGG_BOOLEAN> : k_agg_level<4, AGG_GENERAL>)
+                               : (minmax ? k_agg_level<8, AGG_MINMAX> : boolean ? k_agg_level<8, AGG_BOOLEAN> : k_agg_level<8, AGG_GENERAL>);
             prep_aes_kernel(kern);
-            const int nt = minmax || units <= (unsigned long long)c.num_sms * kAggSmall ? kAggSmall : agg_threads<false>();
+            const int nt = minmax || small ? kAggSmall : agg_threads<AGG_GENERAL>();
             const unsigned grid = (unsigned)std::min<unsigned long long>(ceil_div(units, nt), (unsigned long long)c.num_sms);
             ProfScope ps(c, "agg_level", bytes, 3.0 * calls * units + 3.0 * packed * units);
             kern<<<grid, nt, kAesSmemBytes, c.stream>>>(a);
