@@ -171,6 +171,10 @@ int orqcu_prefix_sum_a_noalloc(orqcu_runtime* rt, int width, size_t n, void* con
 /* PermutationManager::reserve (permutation_manager.h:102-181): generate
  * `count` sharded permutations of size n ahead of use. Synchronous. */
 int orqcu_reserve_permutations(orqcu_runtime* rt, size_t n, size_t count);
+/* Device memory that reserving `count` permutations of size n takes from a
+ * runtime's pool on `sms` SMs: the permutations, and what generating them holds
+ * meanwhile. Needs no device. */
+int orqcu_permutation_bytes(size_t n, size_t count, int sms, size_t* bytes);
 /* What the generator of this runtime tries first, for tests of its corrections:
  * `width` is the half width of the chain's threshold windows in standard
  * deviations (6 otherwise), `buffers` is added to the getNext buffers a small

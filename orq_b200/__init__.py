@@ -78,6 +78,14 @@ def _tdtype(width: int):
     return {1: torch.int8, 2: torch.int16, 4: torch.int32, 8: torch.int64, 16: torch.int64}[width]
 
 
+def permutation_bytes(n: int, count: int, sms: int = 148) -> int:
+    """Device memory that reserving `count` permutations of size n takes from
+    a runtime's pool: the permutations, and what generating them holds."""
+    v = ctypes.c_size_t()
+    _check(load_library().orqcu_permutation_bytes(ctypes.c_size_t(n), ctypes.c_size_t(count), int(sms), ctypes.byref(v)))
+    return v.value
+
+
 _P3 = ctypes.c_void_p * 3
 
 

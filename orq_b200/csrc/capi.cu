@@ -588,6 +588,15 @@ int orqcu_reserve_permutations(orqcu_runtime* rt, size_t n, size_t count) {
     });
 }
 
+int orqcu_permutation_bytes(size_t n, size_t count, int sms, size_t* bytes) {
+    return guard([&] {
+        need(bytes != nullptr, "null output");
+        need(n < (1ull << 31), "permutation size must be < 2^31");
+        need(sms >= 1, "no SMs");
+        *bytes = orqcu::perm_bytes(sms, n, count);
+    });
+}
+
 int orqcu_runtime_tune_permutations(orqcu_runtime* rt, double width, int buffers, unsigned chunks) {
     return guard([&] {
         need_rt(rt);

@@ -950,6 +950,81 @@ void release_fy(Ctx& c) {
     R = FyRes{};
 }
 
+namespace {
+// How `count` permutations of n > 0 rows are generated on num_sms SMs.
+struct FyPlan {
+    int bitsw;               // M = 2^bitsw
+    double M, H, per_perm;   // harmonic number of n, expected getNext buffers
+    bool small;
+    size_t fin_p;            // local permutations finalized at once
+    uint32_t fin_chunks;     // scan chunks of a permutation
+    // the chain
+    uint32_t gen_sms, W, rl, tpb, ring_bufs, ring_tiles, seg_cap;
+};
+FyPlan fy_plan(int num_sms, size_t n, size_t count) {
+    FyPlan p{};
+    while (p.bitsw < 64 && (n >> p.bitsw)) p.bitsw++;
+    p.M = (double)(1ull << p.bitsw);
+    for (size_t k = 1; k <= std::min<size_t>(n, 1 << 16); k++) p.H += 1.0 / k;
+    if (n > (1u << 16)) p.H += std::log((double)n / (1 << 16));
+    p.per_perm = p.M * p.H / (double)(1 << 20) + 1.0;
+    p.small = fy_small_path(1ull << p.bitsw, count);
+    p.fin_p = std::clamp<size_t>(kFinBatch / n, 1, 3 * count);
+    p.fin_chunks = (uint32_t)ceil_div(n, (size_t)kFinChunk);
+    // Buffers are generated `W` at a time per group into a ring of kRing * W
+    // (up to kRing - 1 chunks ahead of the scan: the draws do not depend on
+    // it). W buffers of 2^20 draws keep every SM busy for ~6 us each.
+    constexpr uint32_t kRing = 4;
+    // Three SMs are left to k_fy_resolve, whose registers do not fit beside a
+    // generator CTA's; up to M = 2^19, where the chain waits for its steps and
+    // not for the generator, 24 (44 permutations of 100003 rows 4.8 and 4.0 ms,
+    // of 262143 7.4 and 6.4; of 2^19 rows, M = 2^20, 11.6 and 11.4). W is
+    // rounded so that the last wave of lists is full.
+    p.gen_sms = (uint32_t)std::max(1, num_sms - (p.bitsw <= 19 ? std::min(24, num_sms / 6) : 3));
+    const uint32_t gen_warps = p.gen_sms * (kGenThreads / 32);
+    const double want = std::clamp(p.per_perm * count / 8.0, 2.0, 64.0);
+    const uint32_t waves = std::max(1u, (uint32_t)(want * kListsPerBuf / gen_warps));
+    p.W = std::max(2u, waves * gen_warps / kListsPerBuf);
+    // Runs of 8192 draws, or shorter ones where a permutation has few of them:
+    // a step's latency is then what counts, and more warps share its draws.
+    p.rl = p.M >= (double)(1u << 22) ? 4 : (p.M >= (double)(1u << 20) ? 2 : 1);
+    p.tpb = kListsPerBuf / (kRuns * p.rl);
+    p.ring_bufs = kRing * p.W;
+    p.ring_tiles = p.ring_bufs * p.tpb;
+    p.seg_cap = p.W * p.tpb;
+    return p;
+}
+
+// The buffers of one group's chain.
+enum { RING_RAW, RING_LST, RING_LCNT, RING_TAB, RING_CAND, RING_UNC, RING_RUN, RING_TC, RING_TU, RING_BASE, RING_UOFF, RING_OK, RING_N };
+void ring_bytes(const FyPlan& p, size_t (&b)[RING_N]) {
+    b[RING_RAW] = (size_t)p.ring_bufs * kBufDraws * 4;
+    b[RING_LST] = (size_t)p.ring_bufs * kListsPerBuf * kListCap * 4;
+    b[RING_LCNT] = (size_t)p.ring_bufs * kListsPerBuf * 4;
+    b[RING_TAB] = (size_t)p.ring_bufs * 4 * kTabEntries * sizeof(uint4);
+    b[RING_CAND] = (size_t)p.W * kBufDraws * 4;
+    b[RING_UNC] = (size_t)p.seg_cap * kTileUnc * sizeof(uint2);
+    b[RING_RUN] = (size_t)p.seg_cap * kRuns * sizeof(FyRun);
+    b[RING_TC] = b[RING_TU] = b[RING_BASE] = b[RING_UOFF] = (size_t)p.seg_cap * 4;
+    b[RING_OK] = (size_t)p.seg_cap * (kPieceUnc / 8);  // (a piece of k_fy_resolve takes at least one tile)
+}
+}  // namespace
+
+size_t perm_bytes(int num_sms, size_t n, size_t count) {
+    if (!count) return 0;
+    size_t t = count * pool_block(3 * std::max<size_t>(n, 1) * 4);
+    if (!n) return t;
+    const FyPlan p = fy_plan(num_sms, n, count);
+    const size_t el = p.fin_p * n;
+    t += pool_block(3 * count * n * 4) + 4 * pool_block(el * 4) + pool_block(p.fin_p * p.fin_chunks * 4) +
+         pool_block(3 * count * sizeof(void*));
+    if (p.small) return t + 2 * pool_block(3 * count * 4) + pool_block(4);
+    size_t b[RING_N];
+    ring_bytes(p, b);
+    for (size_t x : b) t += 3 * pool_block(x);
+    return t + pool_block(3 * sizeof(FyState)) + pool_block(3 * sizeof(FySeg));
+}
+
 void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>& out) {
     out.clear();
     if (count == 0) return;
@@ -965,16 +1040,9 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         for (int g = 0; g < 3; g++) c.nonce[G01 + g] += 4ull * count;
         return;
     }
-    int bitsw = 0;
-    while (bitsw < 64 && (n >> bitsw)) bitsw++;
-    const uint32_t mask = (uint32_t)((1ull << bitsw) - 1);
-
-    // window of buffers generated per pipeline step
-    const double M = (double)(1ull << bitsw);
-    double H = 0;
-    for (size_t k = 1; k <= std::min<size_t>(n, 1 << 16); k++) H += 1.0 / k;
-    if (n > (1u << 16)) H += std::log((double)n / (1 << 16));
-    const double per_perm = M * H / (double)(1 << 20) + 1.0;  // expected buffers
+    const FyPlan plan = fy_plan(c.num_sms, n, count);
+    const double M = plan.M, H = plan.H, per_perm = plan.per_perm;
+    const uint32_t mask = (uint32_t)((1ull << plan.bitsw) - 1);
     Scratch acc(c, (size_t)3 * count * n * 4);
     // generator and scans run on private non-blocking streams so they overlap
     // whatever the caller's stream is (the legacy default stream included)
@@ -993,9 +1061,8 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     // SMs idle while the scanners work through dense windows). acc is laid out
     // [permutation][group], so consecutive local permutations are one
     // contiguous batch; the scratch holds one batch.
-    const size_t fin_p = std::clamp<size_t>(kFinBatch / n, 1, 3 * count);
-    const size_t fin_el = fin_p * n;
-    const uint32_t fin_chunks = (uint32_t)ceil_div(n, (size_t)kFinChunk);
+    const size_t fin_p = plan.fin_p, fin_el = fin_p * n;
+    const uint32_t fin_chunks = plan.fin_chunks;
     Scratch f_cur(c, fin_el * 4), f_part(c, fin_p * fin_chunks * 4), f_bucket(c, fin_el * 4),
         f_par(c, fin_el * 4), f_A(c, fin_el * 4), f_ptrs(c, 3 * count * sizeof(void*));
     {
@@ -1051,7 +1118,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
     for (int g = 0; g < 3; g++) ORQ_CUDA_CHECK(cudaStreamWaitEvent(ss[g], ev_start, 0));
     ORQ_CUDA_CHECK(cudaStreamWaitEvent(fs, ev_start, 0));
 
-    if (fy_small_path(1ull << bitsw, count)) {
+    if (plan.small) {
         // every permutation of every group at once from predicted start
         // buffers, corrected pass by pass (k_fy_small)
         const uint32_t bhat = (uint32_t)std::max(1, 1 + (int)(M * H / (double)(1u << 20)) + c.fy_tune.buffers);
@@ -1127,26 +1194,10 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         return;
     }
 
-    // Buffers are generated `W` at a time per group into a ring of kRing * W
-    // (up to kRing - 1 chunks ahead of the scan: the draws do not depend on
-    // it). W buffers of 2^20 draws keep every SM busy for ~6 us each.
-    constexpr uint32_t kRing = 4;
-    // Three SMs are left to k_fy_resolve, whose registers do not fit beside a
-    // generator CTA's; up to M = 2^19, where the chain waits for its steps and
-    // not for the generator, 24 (44 permutations of 100003 rows 4.8 and 4.0 ms,
-    // of 262143 7.4 and 6.4; of 2^19 rows, M = 2^20, 11.6 and 11.4). W is
-    // rounded so that the last wave of lists is full.
-    const uint32_t gen_sms = (uint32_t)std::max(1, c.num_sms - (bitsw <= 19 ? std::min(24, c.num_sms / 6) : 3)), gen_warps = gen_sms * (kGenThreads / 32);
-    const double want = std::clamp(per_perm * count / 8.0, 2.0, 64.0);
-    const uint32_t waves = std::max(1u, (uint32_t)(want * kListsPerBuf / gen_warps));
-    const uint32_t W = std::max(2u, waves * gen_warps / kListsPerBuf);
-    // Runs of 8192 draws, or shorter ones where a permutation has few of them:
-    // a step's latency is then what counts, and more warps share its draws.
-    const uint32_t rl = M >= (double)(1u << 22) ? 4 : (M >= (double)(1u << 20) ? 2 : 1);
-    const uint32_t tpb = kListsPerBuf / (kRuns * rl);
-    const uint32_t ring_bufs = kRing * W, ring_tiles = ring_bufs * tpb, seg_cap = W * tpb;
+    const uint32_t W = plan.W, rl = plan.rl, tpb = plan.tpb, gen_sms = plan.gen_sms;
+    const uint32_t ring_bufs = plan.ring_bufs, ring_tiles = plan.ring_tiles, seg_cap = plan.seg_cap;
     struct Group {
-        std::unique_ptr<Scratch> raw, lst, lcnt, tab, cand, unc, run, tc, tu, base, uoff, ok;
+        std::unique_ptr<Scratch> buf[RING_N];
         unsigned long long gen = 0;   // buffers generated (or queued)
         unsigned long long pos = 0;   // tiles known to be scanned
         unsigned long long start = 0;
@@ -1154,21 +1205,10 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         bool done = false;
         unsigned head = 0, tail = 0;  // step batches queued / read back
     } G[3];
-    for (auto& q : G) {
-        q.raw.reset(new Scratch(c, (size_t)ring_bufs * kBufDraws * 4));
-        q.lst.reset(new Scratch(c, (size_t)ring_bufs * kListsPerBuf * kListCap * 4));
-        q.lcnt.reset(new Scratch(c, (size_t)ring_bufs * kListsPerBuf * 4));
-        q.tab.reset(new Scratch(c, (size_t)ring_bufs * 4 * kTabEntries * sizeof(uint4)));
-        q.cand.reset(new Scratch(c, (size_t)W * kBufDraws * 4));
-        q.unc.reset(new Scratch(c, (size_t)seg_cap * kTileUnc * sizeof(uint2)));
-        q.run.reset(new Scratch(c, (size_t)seg_cap * kRuns * sizeof(FyRun)));
-        q.tc.reset(new Scratch(c, (size_t)seg_cap * 4));
-        q.tu.reset(new Scratch(c, (size_t)seg_cap * 4));
-        q.base.reset(new Scratch(c, (size_t)seg_cap * 4));
-        q.uoff.reset(new Scratch(c, (size_t)seg_cap * 4));
-        // a piece of k_fy_resolve takes at least one tile
-        q.ok.reset(new Scratch(c, (size_t)seg_cap * (kPieceUnc / 8)));
-    }
+    size_t rb_bytes[RING_N];
+    ring_bytes(plan, rb_bytes);
+    for (auto& q : G)
+        for (int k = 0; k < RING_N; k++) q.buf[k].reset(new Scratch(c, rb_bytes[k]));
     Scratch state(c, 3 * sizeof(FyState)), seg(c, 3 * sizeof(FySeg));
     ORQ_CUDA_CHECK(cudaMemsetAsync(state.p, 0, 3 * sizeof(FyState), c.stream));
     // the side streams start after these allocations and the memset, and are
@@ -1188,7 +1228,7 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         x.n = (uint32_t)n;
         x.count = (uint32_t)count;
         x.g = (uint32_t)g;
-        x.mbits = (uint32_t)bitsw;
+        x.mbits = (uint32_t)plan.bitsw;
         x.th = (uint32_t)(n >> 4);
         x.rl = rl;
         x.tpb = tpb;
@@ -1197,18 +1237,18 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
         x.limit = 0;
         x.rate = std::log1p(-1.0 / M);
         x.width = width;
-        x.raw = G[g].raw->as<uint32_t>();
-        x.lst = G[g].lst->as<uint32_t>();
-        x.lcnt = G[g].lcnt->as<uint32_t>();
+        x.raw = G[g].buf[RING_RAW]->as<uint32_t>();
+        x.lst = G[g].buf[RING_LST]->as<uint32_t>();
+        x.lcnt = G[g].buf[RING_LCNT]->as<uint32_t>();
         x.state = state.as<FyState>() + g;
-        x.cand = G[g].cand->as<uint32_t>();
-        x.unc = G[g].unc->as<uint2>();
-        x.run = G[g].run->as<FyRun>();
-        x.tc = G[g].tc->as<uint32_t>();
-        x.tu = G[g].tu->as<uint32_t>();
-        x.base = G[g].base->as<uint32_t>();
-        x.uoff = G[g].uoff->as<uint32_t>();
-        x.ok = G[g].ok->as<uint32_t>();
+        x.cand = G[g].buf[RING_CAND]->as<uint32_t>();
+        x.unc = G[g].buf[RING_UNC]->as<uint2>();
+        x.run = G[g].buf[RING_RUN]->as<FyRun>();
+        x.tc = G[g].buf[RING_TC]->as<uint32_t>();
+        x.tu = G[g].buf[RING_TU]->as<uint32_t>();
+        x.base = G[g].buf[RING_BASE]->as<uint32_t>();
+        x.uoff = G[g].buf[RING_UOFF]->as<uint32_t>();
+        x.ok = G[g].buf[RING_OK]->as<uint32_t>();
         x.seg = seg.as<FySeg>() + g;
         x.acc = acc.as<uint32_t>();
     }
@@ -1278,16 +1318,16 @@ void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>&
             continue;
         }
         const size_t rb = b % ring_bufs;
-        uint4* tab = G[g].tab->as<uint4>() + rb * 4 * kTabEntries;
+        uint4* tab = G[g].buf[RING_TAB]->as<uint4>() + rb * 4 * kTabEntries;
         FyGenArgs ga;
         ga.st = c.stream_arg(G01 + g, 4ull * b);
         ga.tab = tab;
         ga.mask = mask;
         ga.th = (uint32_t)(n >> 4);
         ga.lists = take * kListsPerBuf;
-        ga.raw = G[g].raw->as<uint32_t>() + rb * kBufDraws;
-        ga.lst = G[g].lst->as<uint32_t>() + rb * kListsPerBuf * kListCap;
-        ga.lcnt = G[g].lcnt->as<uint32_t>() + rb * kListsPerBuf;
+        ga.raw = G[g].buf[RING_RAW]->as<uint32_t>() + rb * kBufDraws;
+        ga.lst = G[g].buf[RING_LST]->as<uint32_t>() + rb * kListsPerBuf * kListCap;
+        ga.lcnt = G[g].buf[RING_LCNT]->as<uint32_t>() + rb * kListsPerBuf;
         ga.state = state.as<FyState>() + g;
         {
             ProfScope ps(c, "fy_gen", 0.0, (double)take * kBufDraws / 4, gs);

@@ -193,7 +193,7 @@ void upload_aes_tables(int device) {
 // allocator on the runtime's stream and trim() returns cached blocks the same
 // way, so neither ever synchronises the device (runtimes on different streams
 // allocate and release independently).
-static size_t bucket(size_t bytes) {
+size_t pool_block(size_t bytes) {
     if (bytes < 256) return 256;
     if (bytes <= (1u << 20)) return (bytes + 255) & ~size_t(255);
     size_t p = size_t(1) << 20;
@@ -203,7 +203,7 @@ static size_t bucket(size_t bytes) {
 }
 
 void* Pool::get(size_t bytes, cudaStream_t stream) {
-    const size_t b = bucket(bytes);
+    const size_t b = pool_block(bytes);
     {
         std::lock_guard<std::mutex> lk(mu_);
         // the smallest cached block of at least b bytes, if it wastes at most half of b

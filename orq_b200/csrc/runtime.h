@@ -69,6 +69,8 @@ class Pool {
     uint64_t clock_ = 0;
     void forget(std::multimap<size_t, void*>::iterator it);
 };
+// bytes of the block that a request for `bytes` takes
+size_t pool_block(size_t bytes);
 // the device's default memory pool keeps freed memory mapped (once per device)
 void keep_pool_memory(int device);
 // returns the device pool's unused memory to the system
@@ -248,6 +250,8 @@ void op_reshare(Ctx& c, bool arith, int w, size_t n, int group, Sh3 s);
 // ---- permutations (fy.cu, perm.cu) ----
 void release_fy(Ctx& c);
 void gen_sharded_perms(Ctx& c, size_t n, size_t count, std::vector<ShardedPerm>& out);
+// device memory of the permutations and of their generation, in the pool's blocks
+size_t perm_bytes(int num_sms, size_t n, size_t count);
 void reserve_perms(Ctx& c, size_t n, size_t count);
 ShardedPerm next_perm(Ctx& c, size_t n);
 void ensure_perm(Ctx& c, ShardedPerm& sp);

@@ -33,15 +33,31 @@ import time
 
 import numpy as np
 
-from . import ASC, Runtime, SortingProtocol, _torch, aggregators, quicksort, radix_sort
+from . import ASC, Runtime, SortingProtocol, _torch, aggregators, permutation_bytes, quicksort, radix_sort
 from .table import EncodedTable
 
 KINDS = ("sort", "groupby", "join")
-# device bytes per row (rows = all input rows of the request), measured
-# upper bounds of the pool's peak use: the sharded permutations reserved by
-# 64-bit radix sorts dominate (66 permutations x 3 groups x 8 bytes per row)
-_BYTES_PER_ROW = {"sort": 2200, "groupby": 2600, "join": 2600}
+# Permutations that the sorts of a request of int64 columns reserve, by protocol:
+# a sort's 3 or 64 bits + 2; table_sort's of (valid, key) with two payloads; a
+# join's of (valid, key, table id) and the sort on valid that trims it.
+_PERMUTATIONS = {"sort": {"quick": (3,), "radix": (66,)},
+                 "groupby": {"quick": (12,), "radix": (75,)},
+                 "join": {"quick": (18, 7), "radix": (81, 7)}}
+# the rest per row (rows = all input rows of the request): the runtime's pool
+# takes up to 210, 380 and 400 bytes, torch's allocator up to 80, 420 and 670
+_BYTES_PER_ROW = {"sort": 350, "groupby": 900, "join": 1100}
 _FIXED_BYTES = 64 << 20
+
+
+def estimate_bytes(kind, n, protocol="quick", sms=148):
+    """Upper bound of the device memory that a request holds while it runs.
+    Generating the permutations dominates and does not grow with the rows alone
+    (a ring of draws that depends on their number and size), so it is asked of
+    the library; both sorts of a join count, since their rings seldom fit each
+    other's blocks."""
+    rows = 5 * n if kind == "join" else n
+    return (_FIXED_BYTES + _BYTES_PER_ROW[kind] * rows
+            + sum(permutation_bytes(rows, c, sms) for c in _PERMUTATIONS[kind][protocol]))
 
 
 def _splitmix(seed, n):
@@ -74,7 +90,7 @@ class Request:
             q = (1 + _splitmix(seed + 1, 4 * n) % np.uint64(50)).astype(np.int64)
             self.inputs = (pk, v, fk, q)
             self.rows = 5 * n
-        self.est_bytes = _FIXED_BYTES + _BYTES_PER_ROW[kind] * self.rows
+        self.est_bytes = None  # set by the server that runs it
         self.result = None
         self.t_admit = self.t_done = None
         self.slot = None
@@ -200,6 +216,7 @@ class Server:
         sms = torch.cuda.get_device_properties(device).multi_processor_count
         limit = sms // slots if (share_sms and slots > 1) else 0
         self.slots = [_Slot(i, device, limit) for i in range(slots)]
+        self.sms = limit or sms
 
     def close(self):
         for s in self.slots:
@@ -210,6 +227,8 @@ class Server:
         start); returns summary statistics. Requests keep their results."""
         torch = _torch()
         reqs = sorted(requests, key=lambda r: r.arrival)
+        for r in reqs:
+            r.est_bytes = estimate_bytes(r.kind, r.n, self.protocol, self.sms)
         lock = threading.Condition()
         queue = collections.deque()
         state = {"reserved": 0, "done": 0, "error": None}
