@@ -66,7 +66,13 @@ int orqcu_runtime_destroy(orqcu_runtime* rt);
 /* Run subsequent work on an existing cudaStream_t; NULL selects the CUDA
  * default stream (as in the CUDA runtime API). */
 int orqcu_runtime_set_stream(orqcu_runtime* rt, void* cuda_stream);
+/* Wait for the runtime's stream. An error that a kernel has flagged since the
+ * last check (an index out of range in corrupted shares, a grid barrier that was
+ * given up) is returned here, or by a call that synchronises before. */
 int orqcu_synchronize(orqcu_runtime* rt);
+/* Text of such an error's bits into buf, at most len bytes with the final 0.
+ * Needs no device. */
+int orqcu_device_error_text(int bits, char* buf, size_t len);
 /* Nonce counter of a PRG stream (AESPRGAlgorithm::nonce, prg_algorithm.h:208). */
 int orqcu_get_nonce(orqcu_runtime* rt, int stream, uint64_t* nonce);
 /* Number of kernels this runtime has launched. */
@@ -233,8 +239,10 @@ int orqcu_equal_b(orqcu_runtime* rt, int width, size_t n, const void* const x[3]
  * becomes !(s & 1), the logical NOT of a B-shared bit. Local. */
 int orqcu_not_b_1(orqcu_runtime* rt, int width, size_t n, const void* const x[3], void* const y[3]);
 /* bitonic_sort (sorting.h:266-353) of one B-shared key column in place, in the
- * signed order; n a power of two, width 4 or 8. One launch per network stage
- * (compare + two multiplexes, operators/common.h:20-28). */
+ * signed order; n a power of two, width 4 or 8 (per stage a compare and two
+ * multiplexes, operators/common.h:20-28). One cooperative launch, not waited
+ * for: a grid barrier that had to be given up is reported by the next call that
+ * synchronises (orqcu_synchronize at the latest). */
 int orqcu_bitonic_sort(orqcu_runtime* rt, int width, size_t n, void* const key[3],
                        int descending);
 /* bitonic_sort (sorting.h:266-353) over nkeys B-shared key columns (keys[3*k+p],

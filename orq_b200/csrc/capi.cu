@@ -339,6 +339,16 @@ int orqcu_runtime_set_stream(orqcu_runtime* rt, void* s) {
     });
 }
 
+int orqcu_device_error_text(int bits, char* buf, size_t len) {
+    return guard([&] {
+        need(buf != nullptr && len > 0, "null output");
+        const std::string t = orqcu::device_error_text(bits);
+        const size_t k = std::min(len - 1, t.size());
+        std::memcpy(buf, t.data(), k);
+        buf[k] = 0;
+    });
+}
+
 int orqcu_synchronize(orqcu_runtime* rt) {
     return guard([&] {
         need_rt_any(rt);

@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(kBitThreads, 1) k_bitonic(BitonicArgs a) {
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
                 } while (v < target && ++spins < (1u << 24));
                 if (v < target) {
-                    atomicOr(a.err, 64);
+                    atomicOr(a.err, kErrBarrier);
                     s_dead = 1;
                 }
             }

@@ -263,7 +263,7 @@ __global__ void k_qs_move(QsRound a, const uint32_t* ord, uint32_t* nord) {
                 while (a.cb[h + f] == 0) {
                     const uint32_t r = a.gz[h + f] - a.gz[h];
                     if (r >= f) {  // a zero with only zeros before it: cannot sit past Z
-                        atomicOr(a.err, 64);
+                        atomicOr(a.err, kErrPartition);
                         break;
                     }
                     f = r;

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_radix_bits(BitsArgs a) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
         } while (v < target && ++spins < (1u << 24));
         if (v < target) {
-            atomicOr(a.err, 64);
+            atomicOr(a.err, kErrBarrier);
             s_dead = 1;
         }
     };

@@ -339,6 +339,14 @@ void Ctx::release_batch() {
     batch = BatchTable{};
 }
 
+std::string device_error_text(int bits) {
+    std::string t;
+    if (bits & kErrBarrier) t = "a grid barrier was given up: the results of the call that waited are incomplete";
+    if (bits & kErrPartition) t += std::string(t.empty() ? "" : "; ") + "corrupted partition in a quicksort";
+    if (bits & ~(kErrBarrier | kErrPartition)) t += std::string(t.empty() ? "" : "; ") + "out-of-range index in a permutation";
+    return t + " (code " + std::to_string(bits) + ")";
+}
+
 void Ctx::check_device_error() {
     if (!d_err) return;
     int h = 0;
@@ -346,7 +354,7 @@ void Ctx::check_device_error() {
     ORQ_CUDA_CHECK(cudaStreamSynchronize(stream));
     if (h) {
         ORQ_CUDA_CHECK(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
-        throw std::runtime_error("out-of-range index in a permutation (code " + std::to_string(h) + ")");
+        throw std::runtime_error(device_error_text(h));
     }
 }
 

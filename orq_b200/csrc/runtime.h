@@ -130,6 +130,11 @@ struct FyTune {
     uint32_t chunks = 0;  // small permutations: chunks of draws a pass has room for (0: by the prediction)
 };
 
+// Bits of the error word; the others are indices out of range.
+constexpr int kErrPartition = 64;  // quicksort's partition is not one
+constexpr int kErrBarrier = 256;   // a grid barrier was given up
+std::string device_error_text(int bits);
+
 constexpr size_t kErrBytes = 256;  // the error word, and the grid barriers' counter in a line of its own
 struct Ctx {
     int device = 0;
