@@ -162,16 +162,10 @@ int orqcu_prefix_sum_a(orqcu_runtime* rt, int width, size_t n, void* const share
  * call: a host program that has already reserved the GPU's memory for its own
  * pool, or a service loop that cannot afford cudaMalloc's device-wide
  * synchronisation while other work runs. It has no counterpart in the
- * reference. Its scratch (the tile sums) is a fixed 384 KiB array in the
- * library, held on every GPU that loads it until the process exits, so n is
- * limited to 2^26 elements (larger n returns ORQCU_EINVAL and touches nothing).
- * The first call on a device looks up the array's device address, so make
- * that first call before any stream capture; the address is looked up again
- * after the last runtime on the device has been destroyed (a cudaDeviceReset
- * while a runtime of the device is alive is not supported). All calls share
- * the array: calls
- * that overlap on the GPU (on any streams) race and must be serialised. No
- * cudaMalloc, cudaFree or other allocating routine is called. */
+ * reference. Its scratch (the tile sums) is 384 KiB that the runtime took when
+ * it was created, so n is limited to 2^26 elements (larger n returns
+ * ORQCU_EINVAL and touches nothing). Calls on different runtimes may overlap on
+ * the GPU. No cudaMalloc, cudaFree or other allocating routine is called. */
 int orqcu_prefix_sum_a_noalloc(orqcu_runtime* rt, int width, size_t n, void* const shares[3]);
 
 /* PermutationManager::reserve (permutation_manager.h:102-181): generate

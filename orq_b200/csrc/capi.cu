@@ -74,7 +74,7 @@ static void create_runtime(uint64_t seed, int device, int nparties, orqcu_runtim
     ORQ_CUDA_CHECK(cudaDeviceGetAttribute(&rt->ctx.num_sms, cudaDevAttrMultiProcessorCount, device));
     ORQ_CUDA_CHECK(cudaStreamCreateWithFlags(&rt->ctx.stream, cudaStreamNonBlocking));
     rt->ctx.owns_stream = true;
-    ORQ_CUDA_CHECK(cudaMalloc(&rt->ctx.d_err, orqcu::kErrBytes));
+    ORQ_CUDA_CHECK(cudaMalloc(&rt->ctx.d_err, orqcu::kErrBytes + orqcu::kScanBytes));
     ORQ_CUDA_CHECK(cudaMemset(rt->ctx.d_err, 0, orqcu::kErrBytes));
     if (party >= 0) {
         // one party: its keys arrive through orqcu_party_set_key

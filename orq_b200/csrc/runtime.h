@@ -136,6 +136,8 @@ constexpr int kErrBarrier = 256;   // a grid barrier was given up
 std::string device_error_text(int bits);
 
 constexpr size_t kErrBytes = 256;  // the error word, and the grid barriers' counter in a line of its own
+constexpr size_t kNoAllocMaxElems = size_t(1) << 26;
+constexpr size_t kScanBytes = 384 << 10;  // tile sums of a prefix sum without allocation, behind them
 struct Ctx {
     int device = 0;
     int nparties = 3;  // 3: replicated 3PC; 2: Beaver 2PC; 4: Fantastic-4PC
@@ -157,6 +159,7 @@ struct Ctx {
     // arrival counter of the grid barriers (the cooperative kernels of a runtime
     // follow each other on its stream, so one serves all)
     uint32_t* grid_bar() const { return reinterpret_cast<uint32_t*>(d_err) + 32; }
+    void* scan_scratch() const { return reinterpret_cast<uint8_t*>(d_err) + kErrBytes; }
     FyRes fy;
     FyTune fy_tune;
     BatchTable batch;
@@ -219,8 +222,8 @@ void op_np_open(Ctx& c, bool arith, int w, size_t n, const void* const* s, void*
 void op_np_local(Ctx& c, int op, int w, size_t n, const void* const* x, const void* const* y, void* const* z);
 void op_np_mult(Ctx& c, int mode, int w, size_t n, const void* const* x, const void* const* y, void* const* z);
 void upload_aes_tables(int device);
-// Per-device set-up (the AES tables, the address of the no-alloc scratch
-// array) is done once per device and remembered with the device's epoch. The
+// Per-device set-up (the AES tables) is done once per device and remembered with
+// the device's epoch. The
 // epoch advances when the last live runtime on the device is destroyed, so a
 // cudaDeviceReset between runtimes (which drops the context's memory and can
 // move its module globals) makes the next runtime redo the set-up. A reset

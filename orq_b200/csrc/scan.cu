@@ -6,7 +6,6 @@
 // S[0], S[1], S[2]. Reduce-then-scan over 4096-element tiles: per-tile sums,
 // a scan of the tile sums per share, then each tile rescanned with its offset.
 #include <memory>
-#include <mutex>
 
 #include "launch.cuh"
 
@@ -143,45 +142,19 @@ void op_prefix_sum_into(Ctx& c, int w, size_t n, Sh3 s, void* tsum) {
 // host program that reserved the GPU's memory up front for its own pool (so a
 // cudaMalloc would fail or break its budget), or a service loop that must not
 // pay cudaMalloc's implicit device-wide synchronisation while other requests
-// are running. For them the tile sums live in this fixed array instead of the
-// runtime's pool. It holds 3 x 16384 tile sums of 8 bytes (384 KiB per device,
-// kept until the process exits), which limits a call to 2^26 elements. Every
-// call reuses the same array, so two such calls must not run at the same time
-// on the GPU (different streams included): their tile sums would mix. Each
-// call writes every tile sum it reads, so nothing needs clearing between calls.
-constexpr size_t kNoAllocMaxElems = size_t(1) << 26;
-constexpr size_t kNoAllocTiles = kNoAllocMaxElems / kTile;
-static __device__ __align__(256) unsigned long long g_noalloc_tsum[3 * kNoAllocTiles];
-
-// Device address of g_noalloc_tsum on `device`, looked up once per device with
-// that device current (host code may not pass the symbol itself to a kernel).
-// The address is remembered with the device's epoch: once the last runtime on
-// the device is destroyed (after which the context may have been reset and
-// the array moved) the next call looks it up again.
-static void* noalloc_scratch(int device) {
-    static std::mutex mu;
-    static void* ptrs[kMaxDevices] = {};
-    static unsigned long long epoch[kMaxDevices] = {};
-    if (device < 0 || device >= kMaxDevices) throw std::invalid_argument("device ordinal out of range");
-    std::lock_guard<std::mutex> lk(mu);
-    const unsigned long long ep = device_epoch(device);
-    if (ptrs[device] && epoch[device] == ep) return ptrs[device];
-    int cur = -1;
-    ORQ_CUDA_CHECK(cudaGetDevice(&cur));
-    if (cur != device) throw std::runtime_error("the runtime's device is not the current device");
-    void* p = nullptr;
-    ORQ_CUDA_CHECK(cudaGetSymbolAddress(&p, g_noalloc_tsum));
-    ptrs[device] = p;
-    epoch[device] = ep;
-    return p;
-}
+// are running. For them the tile sums live in memory that every runtime takes
+// when it is created (kScanBytes: 3 x 16384 tile sums of 8 bytes), which limits
+// a call to 2^26 elements. A runtime's calls follow each other on its stream,
+// and those of two runtimes may run at the same time. Each call writes every
+// tile sum it reads, so nothing needs clearing between calls.
+static_assert(kScanBytes == 3 * (kNoAllocMaxElems / kTile) * 8, "tile sums of the largest call");
 
 void op_prefix_sum_noalloc(Ctx& c, int w, size_t n, Sh3 s) {
     if (w != 4 && w != 8) throw std::invalid_argument("prefix sum supports 4 and 8-byte shares");
     if (n > kNoAllocMaxElems)
         throw std::invalid_argument("orqcu_prefix_sum_a_noalloc handles at most 2^26 elements per call");
     if (n == 0) return;
-    void* ts = noalloc_scratch(c.device);
+    void* ts = c.scan_scratch();
     const uint32_t tiles = prefix_sum_tiles(n);
     if (w == 4) run_scan<uint32_t>(c, n, s, reinterpret_cast<uint32_t*>(ts), tiles, false);
     else run_scan<unsigned long long>(c, n, s, reinterpret_cast<unsigned long long*>(ts), tiles, false);
