@@ -443,8 +443,10 @@ class PrimsWorkload:
         from oracle import run_ref
 
         n = max(1024, min(sample, 1 << 22))
+        driver = ref_driver()
         t0 = time.time()
-        _, out = run_ref.run("prims_time", n, self.seed, shim_seed=7, bits=32, threads=threads, timeout=1800)
+        _, out = run_ref.run("prims_time", n, self.seed, shim_seed=7, bits=32, threads=threads, timeout=1800,
+                             driver=driver)
         prims = None
         for line in out.splitlines():
             if line.startswith('{"prims"'):
@@ -921,21 +923,48 @@ def roofline(prof, steps, n):
     return out
 
 
+class ReferenceUnavailable(Exception):
+    """The reference's driver is not on this host (it is built where an ORQ
+    source tree is present)."""
+
+
+def ref_driver(quick_tables=False):
+    from oracle import run_ref
+
+    driver = run_ref.DRIVER_QS if quick_tables else run_ref.DRIVER
+    if not os.path.exists(driver):
+        raise ReferenceUnavailable(f"{os.path.relpath(driver, ROOT)} is not built: it needs an ORQ source tree")
+    return driver
+
+
 def run_ref_seconds(op, n, seed, bits, threads, timeout=1800, quick_tables=False):
     """ORQ's own CPU code for one op (oracle/_ref/ref_driver, three party
     processes; with quick_tables the build whose EncodedTable sorts default to
     quicksort); returns the seconds it reports for the timed region."""
     from oracle import run_ref
 
+    driver = ref_driver(quick_tables)
     t0 = time.time()
-    _, out = run_ref.run(op, n, seed, shim_seed=7, bits=bits, threads=threads, timeout=timeout,
-                         driver=run_ref.DRIVER_QS if quick_tables else None)
+    _, out = run_ref.run(op, n, seed, shim_seed=7, bits=bits, threads=threads, timeout=timeout, driver=driver)
     wall = time.time() - t0
     sec = None
     for line in out.splitlines():
         if line.startswith("{"):
             sec = json.loads(line)["seconds"]
     return sec if sec else wall
+
+
+def cpu_baseline(wl, args):
+    """The CPU reference on a bounded sample, or why there is none."""
+    try:
+        v, _, sample = wl.cpu_reference(args.cpu_sample, 1)
+    except ReferenceUnavailable as e:
+        return {"unavailable": str(e)}
+    out = {"value": v, "unit": "rows/s", "cores": 3, "kind": "reference", "sample": sample, "cpu": cpu_model(),
+           "threads_per_party": 1}
+    if getattr(wl, "ref_prims", None):
+        out["seconds_per_primitive"] = wl.ref_prims
+    return out
 
 
 def splitmix(seed, n):
@@ -995,7 +1024,12 @@ def main():
         # over its workers, which does not always pay
         calib_sample = max(args.cpu_sample // 16, min(args.cpu_sample, 1 << 10))
         cands = sorted({1, max(1, nproc // 3)})
-        calib = {t: wl.cpu_reference(calib_sample, t)[0] for t in cands} if len(cands) > 1 else {1: None}
+        try:
+            ref_driver()
+            calib = {t: wl.cpu_reference(calib_sample, t)[0] for t in cands} if len(cands) > 1 else {1: None}
+        except ReferenceUnavailable as e:
+            print(json.dumps({"impl": "reference", "unavailable": str(e)}))
+            return
         threads = max(calib, key=lambda t: calib[t] or 0.0)
         # warm-up runs are whole fresh party processes: a small sample suffices
         warm_sample = min(args.cpu_sample, max(calib_sample // 4, 1 << 10))
@@ -1119,11 +1153,7 @@ def main():
     if e2e:
         line["e2e"] = e2e
     if not args.no_cpu_baseline and world == 1:
-        v, _, sample = wl.cpu_reference(args.cpu_sample, 1)
-        line["cpu_baseline"] = {"value": v, "unit": "rows/s", "cores": 3, "kind": "reference",
-                                "sample": sample, "cpu": cpu_model(), "threads_per_party": 1}
-        if getattr(wl, "ref_prims", None):
-            line["cpu_baseline"]["seconds_per_primitive"] = wl.ref_prims
+        line["cpu_baseline"] = cpu_baseline(wl, args)
     print(json.dumps(line))
 
 
