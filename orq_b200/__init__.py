@@ -280,19 +280,22 @@ class SharedVector:
                                  ctypes.c_void_p(out.data_ptr())))
         return out
 
-    def _bin(self, other, fn, cls):
-        if other.size() != self.size() or other.width != self.width:
+    def _like(self, other):
+        """(size, width), which `other` must have too."""
+        n, w = self.size(), self.width
+        if other.size() != n or other.width != w:
             raise ValueError("size/width mismatch")
-        z = self.rt._alloc(self.size(), self.width)
-        _check(fn(self.rt.h, self.width, ctypes.c_size_t(self.size()), _p3(self.shares),
-                  _p3(other.shares), _p3(z)))
+        return n, w
+
+    def _bin(self, other, fn, cls):
+        n, w = self._like(other)
+        z = self.rt._alloc(n, w)
+        _check(fn(self.rt.h, w, ctypes.c_size_t(n), _p3(self.shares), _p3(other.shares), _p3(z)))
         return cls(self.rt, z)
 
     def _ibin(self, other, fn):
-        if other.size() != self.size() or other.width != self.width:
-            raise ValueError("size/width mismatch")
-        _check(fn(self.rt.h, self.width, ctypes.c_size_t(self.size()), _p3(self.shares),
-                  _p3(other.shares), _p3(self.shares)))
+        n, w = self._like(other)
+        _check(fn(self.rt.h, w, ctypes.c_size_t(n), _p3(self.shares), _p3(other.shares), _p3(self.shares)))
         return self
 
     def clone(self):
@@ -335,18 +338,16 @@ class BSharedVector(SharedVector):
         return ~((~self) & (~o))
 
     def __invert__(self):
-        z = self.rt._alloc(self.size(), self.width)
-        _check(self.rt.lib.orqcu_not_b(self.rt.h, self.width, ctypes.c_size_t(self.size()),
-                                       _p3(self.shares), _p3(z)))
+        n, w = self.size(), self.width
+        z = self.rt._alloc(n, w)
+        _check(self.rt.lib.orqcu_not_b(self.rt.h, w, ctypes.c_size_t(n), _p3(self.shares), _p3(z)))
         return BSharedVector(self.rt, z)
 
     def extend_lsb(self, inp: "BSharedVector"):
         """BSharedVector::extend_lsb (b_shared_vector.h:145-147): every element
         of self becomes all ones where inp's LSB is set (local)."""
-        if inp.size() != self.size() or inp.width != self.width:
-            raise ValueError("size/width mismatch")
-        _check(self.rt.lib.orqcu_extend_lsb(self.rt.h, self.width, ctypes.c_size_t(self.size()),
-                                            _p3(inp.shares), _p3(self.shares)))
+        n, w = self._like(inp)
+        _check(self.rt.lib.orqcu_extend_lsb(self.rt.h, w, ctypes.c_size_t(n), _p3(inp.shares), _p3(self.shares)))
         return self
 
     def mask(self, m: int):
@@ -357,20 +358,19 @@ class BSharedVector(SharedVector):
 
     def b2a_bit(self) -> "ASharedVector":
         """b2a_bit (b_shared_vector.h:279-284, replicated_3pc.h:220-251)."""
-        z = self.rt._alloc(self.size(), self.width)
-        _check(self.rt.lib.orqcu_b2a_bit(self.rt.h, self.width, ctypes.c_size_t(self.size()),
-                                         _p3(self.shares), _p3(z)))
+        n, w = self.size(), self.width
+        z = self.rt._alloc(n, w)
+        _check(self.rt.lib.orqcu_b2a_bit(self.rt.h, w, ctypes.c_size_t(n), _p3(self.shares), _p3(z)))
         return ASharedVector(self.rt, z)
 
     def _compare(self, other: "BSharedVector"):
         """BSharedVector::_compare (circuits.h:231-295): (eq, gt) as B-shared
         bits, self vs other in the signed order."""
-        if other.size() != self.size() or other.width != self.width:
-            raise ValueError("size/width mismatch")
-        eq = self.rt._alloc(self.size(), self.width)
-        gt = self.rt._alloc(self.size(), self.width)
-        _check(self.rt.lib.orqcu_compare_b(self.rt.h, self.width, ctypes.c_size_t(self.size()),
-                                           _p3(self.shares), _p3(other.shares), _p3(eq), _p3(gt)))
+        n, w = self._like(other)
+        eq = self.rt._alloc(n, w)
+        gt = self.rt._alloc(n, w)
+        _check(self.rt.lib.orqcu_compare_b(self.rt.h, w, ctypes.c_size_t(n), _p3(self.shares), _p3(other.shares),
+                                           _p3(eq), _p3(gt)))
         return BSharedVector(self.rt, eq), BSharedVector(self.rt, gt)
 
     def __gt__(self, other: "BSharedVector") -> "BSharedVector":
@@ -383,18 +383,16 @@ class BSharedVector(SharedVector):
 
     def __eq__(self, other: "BSharedVector") -> "BSharedVector":
         """operator== (b_shared_vector.h:493-504): bit_same, then mask(1)."""
-        if other.size() != self.size() or other.width != self.width:
-            raise ValueError("size/width mismatch")
-        eq = self.rt._alloc(self.size(), self.width)
-        _check(self.rt.lib.orqcu_equal_b(self.rt.h, self.width, ctypes.c_size_t(self.size()),
-                                         _p3(self.shares), _p3(other.shares), _p3(eq)))
+        n, w = self._like(other)
+        eq = self.rt._alloc(n, w)
+        _check(self.rt.lib.orqcu_equal_b(self.rt.h, w, ctypes.c_size_t(n), _p3(self.shares), _p3(other.shares), _p3(eq)))
         return BSharedVector(self.rt, eq)
 
     def lnot(self) -> "BSharedVector":
         """operator! (not_b_1, replicated_3pc.h:207): logical NOT of a bit."""
-        y = self.rt._alloc(self.size(), self.width)
-        _check(self.rt.lib.orqcu_not_b_1(self.rt.h, self.width, ctypes.c_size_t(self.size()),
-                                         _p3(self.shares), _p3(y)))
+        n, w = self.size(), self.width
+        y = self.rt._alloc(n, w)
+        _check(self.rt.lib.orqcu_not_b_1(self.rt.h, w, ctypes.c_size_t(n), _p3(self.shares), _p3(y)))
         return BSharedVector(self.rt, y)
 
     def __ne__(self, other: "BSharedVector") -> "BSharedVector":
@@ -419,9 +417,9 @@ class ASharedVector(SharedVector):
     def a2b(self) -> "BSharedVector":
         """ASharedVector::a2b (a_shared_vector.h:138-144): full-width
         arithmetic -> boolean conversion (redistribution + ripple-carry adder)."""
-        z = self.rt._alloc(self.size(), self.width)
-        _check(self.rt.lib.orqcu_a2b(self.rt.h, self.width, ctypes.c_size_t(self.size()), _p3(self.shares),
-                                     _p3(z)))
+        n, w = self.size(), self.width
+        z = self.rt._alloc(n, w)
+        _check(self.rt.lib.orqcu_a2b(self.rt.h, w, ctypes.c_size_t(n), _p3(self.shares), _p3(z)))
         return BSharedVector(self.rt, z)
 
     def __mul__(self, o):

@@ -29,3 +29,24 @@ def test_fewer_than_three_share_rows_are_refused(shape):
 def test_share_rows_are_the_tensors_rows(make):
     t = make()
     assert orq_b200._rows3(t) == tuple(t[j].data_ptr() for j in range(3))
+
+
+@pytest.mark.parametrize("other", [torch.zeros((3, 4), dtype=torch.int64), torch.zeros((3, 5), dtype=torch.int32),
+                                   torch.zeros((3, 5, 2), dtype=torch.int64)])
+def test_vectors_of_another_size_or_width_are_refused(other):
+    """before anything is allocated or launched (there is no runtime here)"""
+    A, B = orq_b200.ASharedVector, orq_b200.BSharedVector
+    t = torch.zeros((3, 5), dtype=torch.int64)
+    x, y, xa, ya = B(Lib(), t), B(Lib(), other), A(Lib(), t), A(Lib(), other)
+    calls = [lambda: x & y, lambda: x.__iand__(y), lambda: x == y, lambda: x > y, lambda: x + y,
+             lambda: x.extend_lsb(y), lambda: xa * ya, lambda: xa.__iadd__(ya)]
+    for call in calls:
+        with pytest.raises(ValueError):
+            call()
+
+
+class Lib:
+    """a runtime whose library has entry points that nothing may call"""
+
+    def __getattr__(self, name):
+        return self if name == "lib" else None
