@@ -45,12 +45,11 @@ WORKLOAD = ("3PC oblivious shuffle-based radix sort, 2^22 rows, uint64 key unifo
 # last) = 228 LDS per block at one warp-wide LDS per clock per SM.
 AES_LDS_PER_BLOCK = 228
 DEFAULT_N = 1 << 22
-# DRAM traffic of the dominant k_apply instance (padded 16-byte key + int32
-# permutation, one group): dram__bytes_read.sum + dram__bytes_write.sum of one
-# ncu capture of that kernel at 2^21 rows, scaled per row to the benchmarked
-# size. A constant taken from that capture, not measured by this run (a bench
-# run is never under ncu).
-APPLY_TRAFFIC_BYTES_PER_ROW = 690.5e6 / (1 << 21)
+# DRAM traffic of the bit loop (k_radix_bits<16>, all 40 bits in one launch):
+# dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture at 2^20 rows,
+# scaled per row to the benchmarked size. A constant taken from that capture,
+# not measured by this run (a bench run is never under ncu).
+BITS_TRAFFIC_BYTES_PER_ROW = 18207.7e6 / (1 << 20)
 
 
 def cpu_model():
@@ -562,8 +561,8 @@ class JoinWorkload:
 def run_batch(args, rank, world, local_rank):
     """Config 4: 512 independent sorts (256 bitonic with sizes padded to 2^k,
     256 radix), lengths log-uniform over 2^10..2^20, int32 keys uniform over
-    32 bits. Batched path: one bitonic_sort_batch (persistent work-list kernel
-    per network round, autotuned CTA size, CUDA graph) then one
+    32 bits. Batched path: one bitonic_sort_batch (one cooperative launch for
+    all of them) then one
     radix_sort_batch (the radix items back to back, one synchronisation);
     plain path: 512 per-call operators in the same order (bitonic items, then
     radix items), which yields the same shares. Timed with CUDA events on the
@@ -892,10 +891,10 @@ def roofline(prof, steps, n):
         ach = (v["bytes"] / v["launches"]) / (per_launch_ms / 1e3) / 1e9
         out["roofline"] = {"bound": "hbm", "kernel": name, "achieved": round(ach, 1), "peak": hbm,
                            "unit": "GB/s", "frac": round(ach / hbm, 4),
-                           "traffic": (round(APPLY_TRAFFIC_BYTES_PER_ROW * n)
-                                       if name == "apply_group" and n else None),
+                           "traffic": (round(BITS_TRAFFIC_BYTES_PER_ROW * n)
+                                       if name == "radix_bits" and n else None),
                            "traffic_note": ("fixed constant, not measured by this run: bytes per launch of the "
-                                            "key-apply instance from one ncu capture at 2^21 rows, scaled by rows"),
+                                            "40-bit loop from one ncu capture at 2^20 rows, scaled by rows"),
                            "peak_source": src, "launches_per_step": v["launches"] / steps,
                            "avg_launch_ms": round(per_launch_ms, 4)}
     aes = {k: v for k, v in prof.items() if v["aes_blocks"] > 0}
@@ -1081,7 +1080,7 @@ def main():
                     "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic",
                     "config": {"workload": f"ragged batch: {res['items']} independent 3PC sorts (half bitonic "
                                            "padded to 2^k, half radix), lengths log-uniform 2^10..2^20, int32 "
-                                           "keys uniform; batched bitonic work-list kernels + CUDA graph",
+                                           "keys uniform; bitonic items in one cooperative launch",
                                "rows_per_gpu": res["rows"], "padded_rows": res["padded_rows"],
                                "parallelism": f"replicas x{world}", "l2": "inputs larger than L2"},
                     "correct": res["ok"], "gpu_launches": res["launches_per_step"] * args.steps,
@@ -1146,7 +1145,7 @@ def main():
         "scaling": "weak", "vs_baseline": None, "dtype": "int64", "data": "synthetic", "config": config,
         "correct": ok, "gpu_launches": launches, "clocks": clk,
     }
-    line.update(roofline(prof, args.steps, wl.units if wl.name == "radix" else None))
+    line.update(roofline(prof, args.steps, wl.units if wl.name == "radix" and args.bits == 40 else None))
     if wl.name == "prims":
         line["dtype"] = "int32"
     line.update(getattr(wl, "extra", {}))

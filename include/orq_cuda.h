@@ -338,10 +338,9 @@ int orqcu_bitonic_sort_batch(orqcu_runtime* rt, int width, int count, const size
                              void* const* keys, const int* descending, int use_graph);
 
 /* Re-key the runtime as orqcu_runtime_create(seed) would (fresh keys, nonces
- * at zero, reserved permutations dropped) while keeping its stream, its
- * cached device memory. A serving
- * slot runs each request on its own seed this way, so a request's shares do
- * not depend on what ran before it. No reference counterpart (one
+ * at zero, reserved permutations dropped) while keeping its stream and its
+ * cached device memory. A serving slot runs each request on its own seed this
+ * way, so a request's shares do not depend on what ran before it. No reference counterpart (one
  * orq_init per process there). */
 int orqcu_runtime_reseed(orqcu_runtime* rt, uint64_t seed);
 /* Return the runtime's cached (unused) device memory to the device's memory

@@ -654,8 +654,8 @@ def bitonic_sort_batch(vectors, order=ASC, use_graph: bool = True):
 def radix_sort_batch(vectors, order=ASC, bits=None):
     """Radix sorts of many independent B-shared key columns (same width), in
     place; returns their sorting permutations. Shares equal those of calling
-    radix_sort on each column in list order; item i's bit passes overlap item
-    i+1's permutation generation. `order` and `bits` are one value or a list."""
+    radix_sort on each column in list order; the items run back to back.
+    `order` and `bits` are one value or a list."""
     if not vectors:
         return []
     rt, w = vectors[0].rt, vectors[0].width

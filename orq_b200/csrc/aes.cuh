@@ -142,7 +142,8 @@ __device__ __forceinline__ uint4 keystream_block(const AesSmem& S, const StreamA
     return make_uint4(s0, s1, s2, s3);
 }
 
-// The first two rounds of a chunk's blocks without their constant parts. GCM's
+// The first two rounds of a chunk's blocks without their constant parts (counter
+// mode caching: Bernstein and Schwabe, New AES software speed records, 2008). GCM's
 // counter block is (nonce, 0, BE32(j + 2)): in round 1 counter byte 15 reaches
 // column 0, byte 14 column 1 and byte 13 (1 for the chunk's last two blocks,
 // else 0) column 2, so round 2 is the XOR of two table words a column and a

@@ -1214,7 +1214,7 @@ void op_bitonic_sort_rows(Ctx& c, int w, size_t n, int nkeys, const Sh3* keys, c
         throw std::invalid_argument("bitonic sort takes at most 40 key and data columns");
     if (w != 4 && w != 8) throw std::invalid_argument("bitonic sort supports int32 and int64 keys");
     if (n < 2) return;
-    if (nkeys == 1 && na == 0 && nb == 0) {  // one fused launch per stage
+    if (nkeys == 1 && na == 0 && nb == 0) {  // one launch for the whole sort
         op_bitonic_sort(c, w, n, keys[0], desc[0] != 0);
         return;
     }

@@ -27,6 +27,7 @@ struct RcaArgs {
     int carry_in;          // subtraction: the carry starts as all ones (inplace_invert)
 };
 
+// The masked-swap transpose of a bit matrix (Warren, Hacker's Delight, 7-3) on
 // 16 x 32 bits: reg k holds 16 bits of elements k (low half) and k + 16 (high
 // half); afterwards reg b holds bit b of elements 0..31. Its own inverse.
 __device__ __forceinline__ void transpose16(uint32_t (&x)[16]) {
@@ -53,7 +54,9 @@ __device__ __forceinline__ void transpose16(uint32_t (&x)[16]) {
 // through shared memory so that global accesses are coalesced at any
 // alignment. Bound by the T-table lookups; int32, 2^24 elements: 1.64 ms when a
 // ballot packed every bit, 0.63 ms
-// now (1024 elements 29.6 and 30.0 us a call, 10000 35.4 and 29.1).
+// now (1024 elements 29.6 and 30.0 us a call, 10000 35.4 and 29.1). The 255
+// registers that 8 warps leave do not quite hold a slice: 164 bytes a thread are
+// spilled for int32, 112 for int64.
 constexpr int kRcaThreads = 256;
 constexpr int kRcaRow = 36;  // words of a staged row (32, padded for 16-byte reads)
 constexpr int kRcaStage = 32 * kRcaRow, kRcaKs = 16 * 3 * 32;  // words per warp

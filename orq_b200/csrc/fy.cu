@@ -18,9 +18,10 @@
 //  * k_fy_resolve (one CTA per group) walks only the uncertain draws in order,
 //    and k_fy_emit writes the accepted offsets at their exact ranks and checks
 //    the windows against the exact thresholds;
-//    A one-CTA scanner that replayed every draw bounded the chain before: the
-//    radix step of 2^22 rows took 418 ms and takes 280 ms, of 2^20 rows 127.6
-//    and 62.8 ms, of 100003 rows 19.0 and 12.5 ms.
+//    a one-CTA scanner that replayed every draw bounded the chain before (the
+//    same radix steps with it and without: 2^22 rows 418 and 280 ms, 2^20 rows
+//    127.6 and 62.8, 100003 rows 19.0 and 12.5; the faster bit loop and the rest
+//    have since made 214, 53 and 6.6 of these);
 //  * fy_small (M <= 2^15, many of M = 2^16; one buffer per permutation almost always):
 //    every (permutation, group) in its own CTA at once from predicted start
 //    buffers, re-run from the first wrong prediction until all are verified;

@@ -178,13 +178,13 @@ void op_radix_sort(Ctx& c, int kw, size_t n, Sh3 key, int bits, bool desc, Sh3 p
 
 // ---------------------------------------------------------------------------
 // Batched radix sorts: `count` items in list order, the shares of `count`
-// plain calls. Items run back to back on the runtime's stream with no host
-// synchronisation between them (a plain call ends with one). Overlapping item
-// k's bit passes with item k+1's Fisher-Yates chain is allowed by the PRG
-// order (the chain only needs nonces the host knows once item k's chain has
-// ended) and was measured: on a second stream, with or without a static SM
-// split, it made the ragged batch slower (both halves want every SM for AES,
-// and the data side's CTAs delay the scanner launches the chain waits on).
+// plain calls. Items run back to back on the runtime's stream; the host waits
+// for their permutations, and once at the end. Overlapping item k's bit
+// passes with item k+1's permutations is allowed by the PRG order (they only
+// need nonces the host knows once item k's are generated). With the one-CTA
+// scanner of an earlier chain it made the ragged batch slower, on a second
+// stream with or without a static SM split (both halves want every SM for AES);
+// it has not been measured with the present generator.
 void op_radix_sort_batch(Ctx& c, int kw, int count, const size_t* n, void* const* keys, const int* bits,
                          const int* desc, void* const* perms_out) {
     if (count <= 0) return;
