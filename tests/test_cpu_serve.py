@@ -4,6 +4,8 @@ import pytest
 import orq_b200
 from orq_b200 import serve
 
+pytestmark = pytest.mark.usefixtures("cuda_lib")  # (built)
+
 
 # the arithmetic of the generator's buffers: permutations and accepted offsets,
 # and from 2^16 rows on (few: 2^15) three rings of four times the buffers, of 4
